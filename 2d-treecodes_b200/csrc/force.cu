@@ -93,12 +93,6 @@ __device__ __forceinline__ int classify(const TNode &nd, const Brick &b, double 
 
 constexpr int TR_WARPS = 4;
 constexpr int TR_STACK = 2048;
-// A brick's evaluation is split into tasks of at most P2P_SEG near-field sources (task 0 also
-// does the far field), so that the few bricks on a dense region do not serialise the kernel.
-constexpr int P2P_SEG = 2048;
-// Runs of blocks whose outputs are copied to the host while the next run is evaluated.
-constexpr int FORCE_CHUNKS = 4;
-
 // MODE 1: write the lists at the scanned offsets (CSR); MODE 2: count them and write each
 // warp's entries into its own scratch region (ScratchLayout), recording where each brick's run
 // starts, so that a copy into CSR order replaces a second walk.  A region that fills up sets
@@ -110,7 +104,7 @@ __global__ __launch_bounds__(TR_WARPS * 32) void k_force_lists(
     const double *__restrict__ hs, double theta, const TNode *__restrict__ tnode, int nnodes,
     int *__restrict__ counts, const int *__restrict__ offs, int *__restrict__ lists,
     int *__restrict__ scratch, ScratchLayout sl, int *__restrict__ sstart, int *meta,
-    unsigned *err, unsigned long long *stats, int stack_cap) {
+    unsigned *err, unsigned long long *stats, int stack_cap, int seg) {
     constexpr bool FILL = MODE == 1;
     __shared__ int stack_all[TR_WARPS][TR_STACK];
     const int lane = lane_id(), warp = threadIdx.x >> 5;
@@ -196,8 +190,8 @@ __global__ __launch_bounds__(TR_WARPS * 32) void k_force_lists(
                 counts[brick] = n[0];
                 counts[nbricks + brick] = n[1];
                 counts[2 * nbricks + brick] = n[2];
-                // evaluation tasks: the brick's P2P sources in segments of at most P2P_SEG
-                counts[3 * nbricks + brick] = max(1, (total + P2P_SEG - 1) / P2P_SEG);
+                // near-field tasks: the brick's P2P sources in runs of `seg`
+                counts[3 * nbricks + brick] = max(1, (total + seg - 1) / seg);
                 if (MODE == 2)
                     for (int k = 0; k < 3; ++k)
                         sstart[k * nbricks + brick] = sl.koff[k] + wglob * sl.cap[k] + cur[k];
@@ -638,7 +632,7 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
     const double *__restrict__ ys, const double *__restrict__ vs, const int *__restrict__ offs,
     const int *__restrict__ lists, double *__restrict__ xout, double *__restrict__ yout,
     double *__restrict__ partial, int brick_lo, int brick_hi, int *task_ctr,
-    const int *__restrict__ task_brick) {
+    const int *__restrict__ task_brick, int seg) {
     const BlockLayout L = LBS ? BlockLayout{LBS, LBS - 3} : L_arg;
     __shared__ NearShared<MIXED> shared[EV_WARPS];
     const int lane = lane_id(), warp = threadIdx.x >> 5;
@@ -646,9 +640,9 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
     const int tx = lane & 7, ty = lane >> 3;   // targets (tx, ty) and (tx, ty + 4)
     const double eps = 10 * DBL_EPSILON;
 
-    // Tasks: brick b owns tasks [toff[b], toff[b+1]) (relative to toff[0]); task p covers
-    // sources [p * P2P_SEG, (p + 1) * P2P_SEG) of the brick's P2P sequence.  This launch
-    // evaluates the tasks of bricks [brick_lo, brick_hi).
+    // Tasks: brick b owns tasks [toff[b], toff[b+1]) (relative to toff[0]); task p covers the
+    // tiles that start in sources [p * seg, (p + 1) * seg) of the brick's P2P sequence.  This
+    // launch evaluates the tasks of bricks [brick_lo, brick_hi).
     const int *toff = offs + 3 * nbricks;
     const int tbase = toff[0];
     const int task_lo = toff[brick_lo] - tbase, task_hi = toff[brick_hi] - tbase;
@@ -667,19 +661,28 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
         const Brick b = brick_geometry(x0s[blk], y0s[blk], h, bx, by);
         double ax0 = 0, ay0 = 0, ax1 = 0, ay1 = 0;
 
-        // Tiles of up to EV_CHUNK consecutive sources walk the listed leaves in order.
-        int it = beg, s_next = 0, e_next = 0;
+        // Tiles of up to EV_CHUNK consecutive sources of one leaf and one segment walk the
+        // listed leaves in order; positions count the brick's near-field sources.
+        int it = beg, pos = 0, s_next = 0, e_next = 0;
         auto take = [&]() { return range[lists[it++]]; };
-        int skip = part * P2P_SEG, budget = P2P_SEG;
+        const int lo = part * seg, hi = lo + seg;
+        const int seg0 = lo - (lo & (P2P_SEG - 1)), pos_seg = seg0 + P2P_SEG;
+        // the first tile that starts at or after lo
         while (it < end) {
             const int2 rg = take();
             const int cnt = rg.y - rg.x;
-            if (skip < cnt) {
-                s_next = rg.x + skip;
-                e_next = rg.y;
-                break;
+            if (pos + cnt > lo) {
+                const int first = max(0, seg0 - pos);   // the leaf's first tile of the segment
+                const int skip = first + (max(0, lo - pos - first) + EV_CHUNK - 1) / EV_CHUNK *
+                                             EV_CHUNK;
+                if (skip < cnt) {
+                    s_next = rg.x + skip;
+                    e_next = rg.y;
+                    pos += skip;
+                    break;
+                }
             }
-            skip -= cnt;
+            pos += cnt;
         }
         auto next_tile = [&](int &t0, int &tn) {
             while (s_next >= e_next && it < end) {
@@ -688,10 +691,10 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
                 e_next = rg.y;
             }
             t0 = s_next;
-            tn = min(min(EV_CHUNK, e_next - s_next), budget);
+            tn = pos < hi ? min(min(EV_CHUNK, e_next - s_next), pos_seg - pos) : 0;
             if (tn < 0) tn = 0;
             s_next += tn;
-            budget -= tn;
+            pos += tn;
         };
         int t0, tn;
         next_tile(t0, tn);
@@ -935,6 +938,7 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
     // them instead, and the regions are sized up for the next solve.  The runs live in the
     // sort's record buffer when they fit in it, else in a block held only for the build.
     const int nwarps = trgrid * TR_WARPS;
+    const int seg = near_segment(nbricks);
     ScratchLayout sl;
     ListScratch ls;   // released (when transient) after the copy, in stream order
     int *sstart, *meta;
@@ -955,7 +959,7 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
         TC_CUDA_TRY(cudaMemsetAsync(meta, 0, sizeof(int) * 4, c.stream));
         k_force_lists<2><<<trgrid, TR_WARPS * 32, 0, c.stream>>>(
             nbricks, L, x0s, y0s, hs, theta, tnode, c.nnodes, counts, nullptr, nullptr,
-            static_cast<int *>(ls.p), sl, sstart, meta, err, stats, stack_cap);
+            static_cast<int *>(ls.p), sl, sstart, meta, err, stats, stack_cap, seg);
         TC_KERNEL_CHECK();
         if ((rc = exclusive_scan(c, counts, offs, 4 * nbricks))) return rc;
         for (int k = 0; k < 4; ++k)
@@ -994,7 +998,7 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
         } else {
             k_force_lists<1><<<trgrid, TR_WARPS * 32, 0, c.stream>>>(
                 nbricks, L, x0s, y0s, hs, theta, tnode, c.nnodes, nullptr, offs, lists, nullptr,
-                sl, nullptr, nullptr, err, nullptr, stack_cap);
+                sl, nullptr, nullptr, err, nullptr, stack_cap, seg);
         }
         TC_KERNEL_CHECK();
         TC_CUDA_TRY(cudaEventRecord(c.ev_join, c.stream));
@@ -1033,7 +1037,7 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
         near<<<neargrid, EV_WARPS * 32, 0, c.stream>>>(
             nbricks, L, x0s, y0s, hs, slot_ptr<int2>(c, S_RANGE), slot_ptr<double>(c, S_XS),
             slot_ptr<double>(c, S_YS), slot_ptr<double>(c, S_VS), offs, lists, xout, yout,
-            partial, 0, nbricks, brick_ctr, task_brick);
+            partial, 0, nbricks, brick_ctr, task_brick, seg);
         TC_KERNEL_CHECK();
         if (ntasks > nbricks) {
             k_force_gather_parts<<<(int)std::min<long long>((nbricks + 7) / 8,

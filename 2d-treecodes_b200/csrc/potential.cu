@@ -20,9 +20,29 @@
 namespace tc {
 
 constexpr int PT_WARPS = 4;
-// A group's evaluation is split into tasks of at most PT_SEG near-field sources (task 0 also
-// does the far field), so that groups inside dense clusters do not serialise the kernel.
+// A group's near field is cut into segments of PT_SEG sources, so that groups inside dense
+// clusters do not serialise the kernel.  The segments also fix the grid of source tiles (a
+// segment's tiles start at its own start, at a leaf's start, or 32 sources after another), and
+// with it how the mixed form's FP32 sums are grouped.
 constexpr int PT_SEG = 4096;
+// With few groups a segment is cut further, at tile starts, into tasks of `seg` sources (a
+// divisor of PT_SEG), and the far field becomes a task of its own.
+constexpr int PT_MIN_SEG = 64;
+constexpr int PT_FULL_GROUPS = 16384;
+
+// Near-field sources per evaluation task.  The kernel holds about 2400 resident warps; with whole
+// segments, fewer than ~16K groups leave most of them idle or waiting for the longest task.
+// FP64, sources = targets, theta 0.5, the evaluation kernel with whole segments and with this
+// rule: 4096 (128 groups, seg 64) 152 -> 23 us, 65,536 (2048 groups, seg 512) 307 -> 208 us;
+// at 131,072 groups the tasks balance without cutting.  The mixed form keeps whole segments: its
+// compensated FP32 sum runs over a segment, and cutting it moves results by 1e-9.
+static int task_segment(int ngroups, bool mixed) {
+    int seg = PT_SEG;
+    while (!mixed && seg > PT_MIN_SEG &&
+           (long long)ngroups * PT_SEG < (long long)PT_FULL_GROUPS * seg)
+        seg >>= 1;
+    return seg;
+}
 
 // Lists of one group of 32 targets.  The warp pops up to 32 stack entries (node, target mask)
 // at a time, one per lane, so the latency of the node reads is shared by a whole batch.  A lane
@@ -52,7 +72,7 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
     const int *__restrict__ tperm, double theta, const TNode *__restrict__ tnode, int nnodes,
     int *__restrict__ counts, const int *__restrict__ offs, int2 *__restrict__ lists,
     int2 *__restrict__ scratch, ScratchLayout sl, int *__restrict__ sstart, int *meta,
-    unsigned *err, unsigned long long *stats) {
+    unsigned *err, unsigned long long *stats, int seg) {
     constexpr bool FILL = MODE == 1;
     const int wglob = blockIdx.x * PT_WARPS + (threadIdx.x >> 5);
     int cur[2] = {0, 0};   // MODE 2: entries this warp has written, per kind
@@ -200,8 +220,10 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
         if (!FILL && lane == 0) {
             counts[g] = n0;
             counts[ngroups + g] = n1;
-            // evaluation tasks: the group's near-field sources in segments of at most PT_SEG
-            counts[2 * ngroups + g] = max(1, (gsrc + PT_SEG - 1) / PT_SEG);
+            // evaluation tasks: the group's near-field sources in runs of `seg`; below PT_SEG
+            // the far field is a task of its own
+            counts[2 * ngroups + g] =
+                max(1, (gsrc + seg - 1) / seg + (seg < PT_SEG && n0 > 0 ? 1 : 0));
             if (MODE == 2) {
                 sstart[g] = sl.koff[0] + wglob * sl.cap[0] + cur[0];
                 sstart[ngroups + g] = sl.koff[1] + wglob * sl.cap[1] + cur[1];
@@ -271,8 +293,10 @@ __device__ __forceinline__ void split2(double v, float &hi, float &lo) {
     lo = (float)(v - (double)hi);
 }
 
-// Tasks: group g owns tasks [toff[g], toff[g+1]); task 0 evaluates the far field and the first
-// PT_SEG near-field sources of the group, task p > 0 the p-th segment.
+// Tasks: group g owns tasks [toff[g], toff[g+1]).  seg == PT_SEG: task 0 evaluates the far field
+// and the first segment of the group's near field, task p > 0 the p-th segment.  seg < PT_SEG:
+// the far field is task 0 (where the group has one), and the p-th near-field task takes the tiles
+// that start in sources [p seg, (p + 1) seg) of the group's near field.
 // MIXED = false: FP64 throughout (log of FP64).  MIXED = true: the series of E2P and the P2P
 // logs in FP32 (offsets from the group's first target split hi + lo, lg2.approx, compensated
 // sums); the monopole term m log|z| of E2P stays FP64.
@@ -285,7 +309,7 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval(
     const double *__restrict__ ys, const double *__restrict__ vs,
     const int *__restrict__ offs, const int2 *__restrict__ lists, double *__restrict__ out,
     double *__restrict__ partial, int *task_ctr, const int *__restrict__ task_group,
-    const float2 *__restrict__ sexp, const float *__restrict__ sscale) {
+    const float2 *__restrict__ sexp, const float *__restrict__ sscale, int seg) {
     __shared__ cplx s_coef[PE_WARPS][P];
     // mixed E2P coefficients in pairs (D_2j.re, D_2j+1.re, D_2j.im, D_2j+1.im): the even and
     // the odd series run side by side in f32x2 lanes
@@ -315,6 +339,8 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval(
         const int g = task_group[task];
         const int part = task - (toff[g] - tbase);
         const int nparts = toff[g + 1] - toff[g];
+        // the near-field task of this part; -1: the far field alone
+        const int npart = seg < PT_SEG && offs[g + 1] > offs[g] ? part - 1 : part;
         const int t = g * 32 + lane;
         const bool valid = t < m;
         int j = 0;
@@ -411,26 +437,37 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval(
             if (MIXED) far += (double)sh + (double)sl;
         }
 
-        // P2P (potential-kernels.m4:19-57): 0.5 sum v log(r2 + eps), sources
-        // [part * PT_SEG, (part + 1) * PT_SEG) of the group's listed leaves.  Tiles of up to
-        // PE_CHUNK consecutive sources of one leaf; the next tile is loaded into registers while
-        // the current one is evaluated.
-        {
+        // P2P (potential-kernels.m4:19-57): 0.5 sum v log(r2 + eps) over the tiles of the
+        // group's listed leaves that start in sources [npart * seg, (npart + 1) * seg).  Tiles
+        // of up to PE_CHUNK consecutive sources of one leaf and one segment; the next tile is
+        // loaded into registers while the current one is evaluated.
+        if (npart >= 0) {
             const int b1 = offs[ngroups + g], e1 = offs[ngroups + g + 1];
-            int it = b1, skip = part * PT_SEG, budget = PT_SEG;
+            // positions count the group's near-field sources; the segment ends at pos_seg
+            const int lo = npart * seg;
+            const int seg0 = lo - (lo & (PT_SEG - 1)), pos_seg = seg0 + PT_SEG;
+            const int hi = lo + seg;
+            int it = b1, pos = 0;
             int s_next = 0, e_next = 0;
             unsigned mask_next = 0;
+            // the first tile that starts at or after lo
             while (it < e1) {
                 const int2 ent = lists[it++];
                 const int2 rg = range[ent.x];
                 const int cnt = rg.y - rg.x;
-                if (skip < cnt) {
-                    s_next = rg.x + skip;
-                    e_next = rg.y;
-                    mask_next = (unsigned)ent.y;
-                    break;
+                if (pos + cnt > lo) {
+                    const int first = max(0, seg0 - pos);   // the leaf's first tile of the segment
+                    const int skip = first + (max(0, lo - pos - first) + PE_CHUNK - 1) / PE_CHUNK *
+                                                 PE_CHUNK;
+                    if (skip < cnt) {
+                        s_next = rg.x + skip;
+                        e_next = rg.y;
+                        mask_next = (unsigned)ent.y;
+                        pos += skip;
+                        break;
+                    }
                 }
-                skip -= cnt;
+                pos += cnt;
             }
             auto next_tile = [&](int &t0, int &tn, unsigned &msk) {
                 while (s_next >= e_next && it < e1) {
@@ -441,11 +478,11 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval(
                     mask_next = (unsigned)ent.y;
                 }
                 t0 = s_next;
-                tn = min(min(PE_CHUNK, e_next - s_next), budget);
+                tn = pos < hi ? min(min(PE_CHUNK, e_next - s_next), pos_seg - pos) : 0;
                 if (tn < 0) tn = 0;
                 msk = mask_next;
                 s_next += tn;
-                budget -= tn;
+                pos += tn;
             };
             int t0, tn;
             unsigned msk;
@@ -662,6 +699,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
     // instead, and the regions are sized up for the next solve.  The runs live in the sort's
     // record buffer when they fit in it, else in a block held only for the build.
     const int nwarps = grid * PT_WARPS;
+    const int seg = task_segment(ngroups, c.precision == 1);
     ScratchLayout sl;
     ListScratch ls;   // released (when transient) after the copy, in stream order
     int *sstart, *meta;
@@ -681,7 +719,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
         TC_CUDA_TRY(cudaMemsetAsync(meta, 0, sizeof(int) * 4, c.stream));
         k_potential_lists<2><<<grid, PT_WARPS * 32, 0, c.stream>>>(
             ngroups, m, xt, yt, vo, theta, tnode, c.nnodes, counts, nullptr, nullptr,
-            static_cast<int2 *>(ls.p), sl, sstart, meta, err, stats);
+            static_cast<int2 *>(ls.p), sl, sstart, meta, err, stats, seg);
         TC_KERNEL_CHECK();
         if ((rc = exclusive_scan(c, counts, offs, 3 * ngroups))) return rc;
         for (int k = 0; k < 3; ++k)
@@ -721,7 +759,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
                                         c.stream));
             k_potential_lists<1><<<grid, PT_WARPS * 32, 0, c.stream>>>(
                 ngroups, m, xt, yt, vo, theta, tnode, c.nnodes, nullptr, offs, lists, nullptr,
-                sl, nullptr, nullptr, err, stats);
+                sl, nullptr, nullptr, err, stats, seg);
         }
         TC_KERNEL_CHECK();
         TC_CUDA_TRY(cudaEventRecord(c.ev_join, c.stream));
@@ -764,7 +802,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
         eval<<<egrid, PE_WARPS * 32, 0, c.stream>>>(
             ngroups, m, xt, yt, vo, tnode, slot_ptr<double>(c, S_MASS), slot_ptr<double>(c, S_EXPS),
             slot_ptr<int2>(c, S_RANGE), slot_ptr<double>(c, S_XS), slot_ptr<double>(c, S_YS),
-            slot_ptr<double>(c, S_VS), offs, lists, out, partial, task_ctr, task_group, sexp, sscale);
+            slot_ptr<double>(c, S_VS), offs, lists, out, partial, task_ctr, task_group, sexp, sscale, seg);
         TC_KERNEL_CHECK();
         return TC_OK;
     });

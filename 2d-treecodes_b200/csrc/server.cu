@@ -135,11 +135,18 @@ size_t footprint_estimate(int kind, long long n, long long ntargets, long long n
     if (force) {
         const long long m = nblocks * tc::BLOCKSIZE * tc::BLOCKSIZE;
         b += (size_t)m * 16 + (size_t)m * 64;   // outputs + per-brick lists and partial sums
+        // with few bricks the near field runs in more tasks, 1 KB of partial sums each (about
+        // 1024 sources per brick)
+        const long long bricks = m / (tc::TILE * tc::TILE);
+        b += (size_t)bricks * (1024 / tc::near_segment((int)std::min<long long>(bricks, 1 << 24))) *
+             1024;
     } else {
         // staged targets, output, target sort, partials and the per-group lists, whose far
         // part grows as 1/theta^2 (about 14 entries per target at theta = 0.3); the list
         // build's scratch, held only while the lists are built, is not charged
         b += (size_t)ntargets * 210;
+        // FP64: with few target groups the near field runs in more tasks, 256 B each
+        if (!precision) b += (size_t)std::min(ntargets, 1ll << 19) * 256;
     }
     return b + (4u << 20);
 }

@@ -39,6 +39,30 @@ struct Frame {
     double scale;             // (1 / ext) * 2^LMAX, the factor the compiled reference uses
 };
 
+// A brick's near field is cut into segments of P2P_SEG sources, so that the few bricks on a dense
+// region do not serialise the kernel.  The segments also fix the grid of source tiles (a
+// segment's tiles start at its own start, at a leaf's start, or 32 sources after another), and
+// with it how the mixed form's FP32 sums are grouped.
+constexpr int P2P_SEG = 2048;
+// With few bricks a segment is cut further, at tile starts, into tasks of `seg` sources (a
+// divisor of P2P_SEG).
+constexpr int P2P_MIN_SEG = 64;
+constexpr int P2P_FULL_BRICKS = 32768;
+
+// Near-field sources per task.  The kernel holds about 4700 resident warps; with whole segments
+// fewer than ~32K bricks leave warps idle or waiting for the longest task.  The kernel alone,
+// whole segments and this rule: 16 bricks (seg 64), mixed, 72 -> 35 us; 5476 bricks (seg 256),
+// mixed, 126 -> 81 us; 16,384 bricks (seg 1024), FP64, 596 -> 555 us.
+constexpr int near_segment(int nbricks) {
+    int seg = P2P_SEG;
+    while (seg > P2P_MIN_SEG && (long long)nbricks * P2P_SEG < (long long)P2P_FULL_BRICKS * seg)
+        seg >>= 1;
+    return seg;
+}
+
+// Runs of blocks whose outputs are copied to the host while the next run is evaluated.
+constexpr int FORCE_CHUNKS = 4;
+
 constexpr unsigned FULL_MASK = 0xffffffffu;
 
 // Reads without progress after which a device wait on another CTA's published state gives up
