@@ -293,30 +293,24 @@ __device__ __forceinline__ void split2(double v, float &hi, float &lo) {
     lo = (float)(v - (double)hi);
 }
 
-// Tasks: group g owns tasks [toff[g], toff[g+1]).  seg == PT_SEG: task 0 evaluates the far field
-// and the first segment of the group's near field, task p > 0 the p-th segment.  seg < PT_SEG:
-// the far field is task 0 (where the group has one), and the p-th near-field task takes the tiles
-// that start in sources [p seg, (p + 1) seg) of the group's near field.
-// MIXED = false: FP64 throughout (log of FP64).  MIXED = true: the series of E2P and the P2P
-// logs in FP32 (offsets from the group's first target split hi + lo, lg2.approx, compensated
-// sums); the monopole term m log|z| of E2P stays FP64.
-template <int P, bool MIXED>
-__global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval(
+// Tasks: group g owns tasks [toff[g], toff[g+1]); task 0 evaluates the far field and the first
+// PT_SEG near-field sources of the group, task p > 0 the p-th segment.
+// The mixed form: the series of E2P and the P2P logs in FP32 (offsets from the group's first
+// target split hi + lo, lg2.approx, compensated sums); the monopole term m log|z| of E2P stays
+// FP64.
+template <int P>
+__global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval_mixed(
     int ngroups, int m, const double *__restrict__ xt, const double *__restrict__ yt,
     const int *__restrict__ tperm, const TNode *__restrict__ tnode,
-    const double *__restrict__ mass, const double *__restrict__ exps,
-    const int2 *__restrict__ range, const double *__restrict__ xs,
+    const double *__restrict__ mass, const int2 *__restrict__ range, const double *__restrict__ xs,
     const double *__restrict__ ys, const double *__restrict__ vs,
     const int *__restrict__ offs, const int2 *__restrict__ lists, double *__restrict__ out,
     double *__restrict__ partial, int *task_ctr, const int *__restrict__ task_group,
-    const float2 *__restrict__ sexp, const float *__restrict__ sscale, int seg) {
-    __shared__ cplx s_coef[PE_WARPS][P];
-    // mixed E2P coefficients in pairs (D_2j.re, D_2j+1.re, D_2j.im, D_2j+1.im): the even and
+    const float2 *__restrict__ sexp, const float *__restrict__ sscale) {
+    // E2P coefficients in pairs (D_2j.re, D_2j+1.re, D_2j.im, D_2j+1.im): the even and
     // the odd series run side by side in f32x2 lanes
     __shared__ float4 s_coef32[PE_WARPS][P / 2];
-    __shared__ double2 s_xy[PE_WARPS][PE_CHUNK];
-    __shared__ double s_v[PE_WARPS][PE_CHUNK];
-    // mixed form: the tile as negated float offsets (hi + lo) from the group's reference point,
+    // the tile as negated float offsets (hi + lo) from the group's reference point,
     // two sources per entry for paired-FP32 (f32x2) arithmetic: (-x hi, -x hi', -x lo, -x lo'),
     // the same for y, and (v, v')
     __shared__ float4 s_nx[PE_WARPS][PE_CHUNK / 2];
@@ -326,6 +320,296 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval(
     __shared__ double s_neg_log_c[LOG_NTAB];       // log_pos's table
     load_log_table(s_neg_log_c);
     const int lane = lane_id(), warp = threadIdx.x >> 5;
+    const double eps = 10 * DBL_EPSILON;
+    const int *toff = offs + 2 * ngroups;
+    const int tbase = toff[0];
+    const int ntasks = toff[ngroups] - tbase;
+
+    for (;;) {
+        int task = 0;
+        if (lane == 0) task = atomicAdd(task_ctr, 1);
+        task = __shfl_sync(FULL_MASK, task, 0);
+        if (task >= ntasks) break;
+        const int g = task_group[task];
+        const int part = task - (toff[g] - tbase);
+        const int nparts = toff[g + 1] - toff[g];
+        const int t = g * 32 + lane;
+        const bool valid = t < m;
+        int j = 0;
+        double x = 0, y = 0;
+        if (valid) {
+            j = tperm[t];
+            x = xt[j];
+            y = yt[j];
+        }
+        // reference point of the mixed form's offsets: the group's first target
+        const double xref = __shfl_sync(FULL_MASK, x, 0), yref = __shfl_sync(FULL_MASK, y, 0);
+        double far = 0, near = 0;
+
+        // E2P (potential-kernels.m4:59-89): m log(r2)/2 + Re sum_{j=1..p} a_{j-1} z^-j.  The next
+        // entry's cell record and coefficients are loaded while the current one is evaluated.
+        if (part == 0) {
+            const int b0 = offs[g], e0 = offs[g + 1];
+            float sh = 0, sl = 0;
+            int2 ent_n = make_int2(0, 0);
+            TNode nd_n = {};
+            double m_n = 0;
+            float R_n = 1.f;
+            float2 c32_n = make_float2(0.f, 0.f);
+            auto fetch = [&](int at) {
+                ent_n = lists[at];
+                nd_n = tnode[ent_n.x];
+                m_n = mass[ent_n.x];
+                R_n = sscale[ent_n.x];
+                if (lane < P) c32_n = sexp[(size_t)ent_n.x * P + lane];
+            };
+            if (b0 < e0) fetch(b0);
+            for (int it = b0; it < e0; ++it) {
+                const int2 ent = ent_n;
+                const TNode nd = nd_n;
+                const double mm = m_n;
+                const float R = R_n;
+                __syncwarp();
+                if (lane < P) {
+                    float *cp = reinterpret_cast<float *>(s_coef32[warp]);
+                    cp[4 * (lane >> 1) + (lane & 1)] = c32_n.x;
+                    cp[4 * (lane >> 1) + 2 + (lane & 1)] = c32_n.y;
+                }
+                __syncwarp();
+                if (it + 1 < e0) fetch(it + 1);
+                if ((ent.y >> lane) & 1) {
+                    const double rz = x - nd.xcom, iz = y - nd.ycom;
+                    const double r2 = rz * rz + iz * iz;
+                    // series: Re(u' Q(u')), u' = R / z, Q(u') = sum_j D_j u'^j
+                    const float zr = (float)rz, zi = (float)iz;
+                    const float inv = rcp_approx(zr * zr + zi * zi);
+                    const float ur = R * zr * inv, ui = -R * zi * inv;
+                    // Q(u') = E(w) + u' O(w), w = u'^2, E and O the even and odd parts
+                    // of the series, evaluated together by Horner in f32x2 lanes
+                    const float wr = fmaf(ur, ur, -ui * ui), wi = 2.f * ur * ui;
+                    const float2 wr2 = make_float2(wr, wr), wi2 = make_float2(wi, wi);
+                    const float2 nwi2 = make_float2(-wi, -wi);
+                    const float4 cl = s_coef32[warp][P / 2 - 1];
+                    float2 qr2 = make_float2(cl.x, cl.y), qi2 = make_float2(cl.z, cl.w);
+#pragma unroll
+                    for (int j = P / 2 - 2; j >= 0; --j) {
+                        const float4 d = s_coef32[warp][j];
+                        const float2 tr = __ffma2_rn(qi2, nwi2, make_float2(d.x, d.y));
+                        const float2 ti = __ffma2_rn(qi2, wr2, make_float2(d.z, d.w));
+                        const float2 nqr = __ffma2_rn(qr2, wr2, tr);
+                        qi2 = __ffma2_rn(qr2, wi2, ti);
+                        qr2 = nqr;
+                    }
+                    const float2 q = make_float2(
+                        qr2.x + fmaf(ur, qr2.y, -ui * qi2.y),
+                        qi2.x + fmaf(ur, qi2.y, ui * qr2.y));
+                    two_sum_add(sh, sl, ur * q.x - ui * q.y);
+                    far += mm * log_pos(r2, s_neg_log_c) * 0.5;
+                }
+            }
+            far += (double)sh + (double)sl;
+        }
+
+        // P2P (potential-kernels.m4:19-57): 0.5 sum v log(r2 + eps), sources
+        // [part * PT_SEG, (part + 1) * PT_SEG) of the group's listed leaves.  Tiles of up to
+        // PE_CHUNK consecutive sources of one leaf; the next tile is loaded into registers while
+        // the current one is evaluated.
+        {
+            const int b1 = offs[ngroups + g], e1 = offs[ngroups + g + 1];
+            int it = b1, skip = part * PT_SEG, budget = PT_SEG;
+            int s_next = 0, e_next = 0;
+            unsigned mask_next = 0;
+            while (it < e1) {
+                const int2 ent = lists[it++];
+                const int2 rg = range[ent.x];
+                const int cnt = rg.y - rg.x;
+                if (skip < cnt) {
+                    s_next = rg.x + skip;
+                    e_next = rg.y;
+                    mask_next = (unsigned)ent.y;
+                    break;
+                }
+                skip -= cnt;
+            }
+            auto next_tile = [&](int &t0, int &tn, unsigned &msk) {
+                while (s_next >= e_next && it < e1) {
+                    const int2 ent = lists[it++];
+                    const int2 rg = range[ent.x];
+                    s_next = rg.x;
+                    e_next = rg.y;
+                    mask_next = (unsigned)ent.y;
+                }
+                t0 = s_next;
+                tn = min(min(PE_CHUNK, e_next - s_next), budget);
+                if (tn < 0) tn = 0;
+                msk = mask_next;
+                s_next += tn;
+                budget -= tn;
+            };
+            int t0, tn;
+            unsigned msk;
+            next_tile(t0, tn, msk);
+            double px = 0, py = 0, pv = 0;
+            if (lane < tn) {
+                px = xs[t0 + lane];
+                py = ys[t0 + lane];
+                pv = vs[t0 + lane];
+            }
+            float nh = 0, nl = 0, txh = 0, txl = 0, tyh = 0, tyl = 0;
+            split2(x - xref, txh, txl);
+            split2(y - yref, tyh, tyl);
+            const float ln2 = 0.6931471805599453f, epsf = (float)eps;
+            while (tn > 0) {
+                const int cnt = tn;
+                const unsigned cmask = msk;   // this tile's targets (msk moves on to the next tile)
+                const bool mine = (cmask >> lane) & 1;
+                __syncwarp();
+                {
+                    // source `lane` to entry lane / 2, half lane % 2; lanes past the tile add a
+                    // zero-valued source at the reference point (finite, contributes 0)
+                    float a = 0.f, b2 = 0.f, c2 = 0.f, d2 = 0.f, vv = 0.f;
+                    if (lane < cnt) {
+                        split2(px - xref, a, b2);
+                        split2(py - yref, c2, d2);
+                        vv = (float)pv;
+                    }
+                    float *nx = reinterpret_cast<float *>(s_nx[warp]);
+                    float *ny = reinterpret_cast<float *>(s_ny[warp]);
+                    const int e = 4 * (lane >> 1) + (lane & 1);
+                    nx[e] = -a;
+                    nx[e + 2] = -b2;
+                    ny[e] = -c2;
+                    ny[e + 2] = -d2;
+                    reinterpret_cast<float *>(s_v2[warp])[lane] = vv;
+                }
+                __syncwarp();
+                next_tile(t0, tn, msk);
+                if (lane < tn) {
+                    px = xs[t0 + lane];
+                    py = ys[t0 + lane];
+                    pv = vs[t0 + lane];
+                }
+                // A tile needed by few targets of the group (k <= 8) is spread over the lanes:
+                // lane l takes target q = l % k of the mask and sources l / k, l / k + r, ...
+                // (r = 32 / k), and each target adds its r lane partials in lane order.  Denser
+                // tiles keep one target per lane.
+                const int k = __popc(cmask);
+                if (k > 8) {
+                    if (mine) {
+                        // two sources per step in f32x2 lanes; even and odd sources are
+                        // summed apart and added at the end of the tile
+                        const float2 txh2 = make_float2(txh, txh), txl2 = make_float2(txl, txl);
+                        const float2 tyh2 = make_float2(tyh, tyh), tyl2 = make_float2(tyl, tyl);
+                        const float2 eps2 = make_float2(epsf, epsf);
+                        float2 acc = make_float2(0.f, 0.f);
+                        const int npairs = (cnt + 1) >> 1;
+#pragma unroll 4
+                        for (int q = 0; q < npairs; ++q) {
+                            const float4 nx = s_nx[warp][q], ny = s_ny[warp][q];
+                            const float2 dx = __fadd2_rn(__fadd2_rn(txh2, make_float2(nx.x, nx.y)),
+                                                         __fadd2_rn(txl2, make_float2(nx.z, nx.w)));
+                            const float2 dy = __fadd2_rn(__fadd2_rn(tyh2, make_float2(ny.x, ny.y)),
+                                                         __fadd2_rn(tyl2, make_float2(ny.z, ny.w)));
+                            const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, eps2));
+                            acc = __ffma2_rn(make_float2(lg2_approx(r2.x), lg2_approx(r2.y)),
+                                             s_v2[warp][q], acc);
+                        }
+                        two_sum_add(nh, nl, (acc.x + acc.y) * ln2);
+                    }
+                } else if (k > 0) {
+                    const int r = 32 / k;
+                    const int qt = lane % k;
+                    const int tl = (int)__fns(cmask, 0, qt + 1);   // lane of this lane's target
+                    double part = 0;
+                    {
+                        const float qxh = __shfl_sync(FULL_MASK, txh, tl);
+                        const float qxl = __shfl_sync(FULL_MASK, txl, tl);
+                        const float qyh = __shfl_sync(FULL_MASK, tyh, tl);
+                        const float qyl = __shfl_sync(FULL_MASK, tyl, tl);
+                        float acc = 0;
+                        const float *nx = reinterpret_cast<const float *>(s_nx[warp]);
+                        const float *ny = reinterpret_cast<const float *>(s_ny[warp]);
+                        const float *sv = reinterpret_cast<const float *>(s_v2[warp]);
+                        if (lane < r * k)
+                            for (int q = lane / k; q < cnt; q += r) {
+                                const int e = 4 * (q >> 1) + (q & 1);
+                                const float dx = (qxh + nx[e]) + (qxl + nx[e + 2]);
+                                const float dy = (qyh + ny[e]) + (qyl + ny[e + 2]);
+                                acc = fmaf(lg2_approx(fmaf(dx, dx, fmaf(dy, dy, epsf))), sv[q], acc);
+                            }
+                        part = (double)acc;
+                    }
+                    s_part[warp][lane] = part;
+                    __syncwarp();
+                    if (mine) {
+                        const int q = __popc(cmask & ((1u << lane) - 1u));
+                        double sum = 0;
+                        for (int i = 0; i < r; ++i) sum += s_part[warp][q + i * k];
+                        two_sum_add(nh, nl, (float)sum * ln2);
+                    }
+                    __syncwarp();
+                }
+            }
+            near = (double)nh + (double)nl;
+        }
+        const double res = 0.5 * near + far;
+        if (nparts == 1) {
+            if (valid) out[j] = res;
+        } else {
+            partial[(size_t)task * 32 + lane] = res;
+        }
+        __syncwarp();
+    }
+}
+
+// The FP64 form.  Bound by the FP64 pipe (12 operations per P2P pair, 16 lanes of it per scheduler
+// and cycle, so 24 cycles per 32 pairs) with the issue slots and the shared-memory port close
+// behind.  Blocks of 8 warps share one set of table copies (64 KB); three blocks, 24 warps, fit
+// on an SM.
+// Tasks: group g owns tasks [toff[g], toff[g+1]).  seg == PT_SEG: task 0 evaluates the far field
+// and the first segment of the group's near field, task p > 0 the p-th segment.  seg < PT_SEG:
+// the far field is task 0 (where the group has one), and the p-th near-field task takes the tiles
+// that start in sources [p seg, (p + 1) seg) of the group's near field.
+constexpr int PD_WARPS = 8;
+constexpr int PD_MIN_BLOCKS = 3;
+
+// Per-warp staging: a cell's coefficients, or a tile's sources (never both at once); the lane
+// partials of a sparse tile.
+template <int P>
+struct EvalShared {
+    union {
+        cplx coef[P];
+        struct {
+            double2 xy[PE_CHUNK];
+            double v[PE_CHUNK];
+        } src;
+    };
+    double part[32];
+    int lane_of[32];   // sparse tiles: the lane of the q-th target of the mask
+};
+
+template <int P>
+constexpr size_t eval_smem() {
+    return sizeof(double2) * NLOG_NTAB * NLOG_COPIES + sizeof(EvalShared<P>) * PD_WARPS;
+}
+
+template <int P>
+__global__ __launch_bounds__(PD_WARPS * 32, PD_MIN_BLOCKS) void k_potential_eval(
+    int ngroups, int m, const double *__restrict__ xt, const double *__restrict__ yt,
+    const int *__restrict__ tperm, const TNode *__restrict__ tnode,
+    const double *__restrict__ mass, const double *__restrict__ exps,
+    const int2 *__restrict__ range, const double *__restrict__ xs,
+    const double *__restrict__ ys, const double *__restrict__ vs,
+    const int *__restrict__ offs, const int2 *__restrict__ lists, double *__restrict__ out,
+    double *__restrict__ partial, int *task_ctr, const int *__restrict__ task_group, int seg) {
+    extern __shared__ __align__(16) unsigned char eval_dyn[];
+    double2 *s_tab = reinterpret_cast<double2 *>(eval_dyn);
+    load_near_log_table(s_tab);
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    const unsigned tab = shared_address(s_tab);
+    const int copy = (lane & (NLOG_COPIES - 1)) * (int)sizeof(double2);
+    EvalShared<P> &sh =
+        reinterpret_cast<EvalShared<P> *>(s_tab + NLOG_NTAB * NLOG_COPIES)[warp];
     const double eps = 10 * DBL_EPSILON;
     const int *toff = offs + 2 * ngroups;
     const int tbase = toff[0];
@@ -350,28 +634,20 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval(
             x = xt[j];
             y = yt[j];
         }
-        // reference point of the mixed form's offsets: the group's first target
-        const double xref = __shfl_sync(FULL_MASK, x, 0), yref = __shfl_sync(FULL_MASK, y, 0);
         double far = 0, near = 0;
 
         // E2P (potential-kernels.m4:59-89): m log(r2)/2 + Re sum_{j=1..p} a_{j-1} z^-j.  The next
         // entry's cell record and coefficients are loaded while the current one is evaluated.
         if (part == 0) {
             const int b0 = offs[g], e0 = offs[g + 1];
-            float sh = 0, sl = 0;
             int2 ent_n = make_int2(0, 0);
             TNode nd_n = {};
             double m_n = 0, cr_n = 0, ci_n = 0;
-            float R_n = 1.f;
-            float2 c32_n = make_float2(0.f, 0.f);
             auto fetch = [&](int at) {
                 ent_n = lists[at];
                 nd_n = tnode[ent_n.x];
                 m_n = mass[ent_n.x];
-                if (MIXED) {
-                    R_n = sscale[ent_n.x];
-                    if (lane < P) c32_n = sexp[(size_t)ent_n.x * P + lane];
-                } else if (lane < P) {
+                if (lane < P) {
                     const double *ex = exps + (size_t)ent_n.x * 2 * P;
                     cr_n = ex[lane];
                     ci_n = ex[P + lane];
@@ -382,59 +658,22 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval(
                 const int2 ent = ent_n;
                 const TNode nd = nd_n;
                 const double mm = m_n;
-                const float R = R_n;
                 __syncwarp();
-                if (lane < P) {
-                    if (MIXED) {
-                        float *cp = reinterpret_cast<float *>(s_coef32[warp]);
-                        cp[4 * (lane >> 1) + (lane & 1)] = c32_n.x;
-                        cp[4 * (lane >> 1) + 2 + (lane & 1)] = c32_n.y;
-                    }
-                    else s_coef[warp][lane] = {cr_n, ci_n};
-                }
+                if (lane < P) sh.coef[lane] = {cr_n, ci_n};
                 __syncwarp();
                 if (it + 1 < e0) fetch(it + 1);
                 if ((ent.y >> lane) & 1) {
                     const double rz = x - nd.xcom, iz = y - nd.ycom;
                     const double r2 = rz * rz + iz * iz;
-                    if (MIXED) {
-                        // series: Re(u' Q(u')), u' = R / z, Q(u') = sum_j D_j u'^j
-                        const float zr = (float)rz, zi = (float)iz;
-                        const float inv = rcp_approx(zr * zr + zi * zi);
-                        const float ur = R * zr * inv, ui = -R * zi * inv;
-                        // Q(u') = E(w) + u' O(w), w = u'^2, E and O the even and odd parts
-                        // of the series, evaluated together by Horner in f32x2 lanes
-                        const float wr = fmaf(ur, ur, -ui * ui), wi = 2.f * ur * ui;
-                        const float2 wr2 = make_float2(wr, wr), wi2 = make_float2(wi, wi);
-                        const float2 nwi2 = make_float2(-wi, -wi);
-                        const float4 cl = s_coef32[warp][P / 2 - 1];
-                        float2 qr2 = make_float2(cl.x, cl.y), qi2 = make_float2(cl.z, cl.w);
+                    // (the bound keeps the reciprocal's Newton steps finite when r2 overflows)
+                    const double inv = rcp_nr(fmin(r2, 1e300));
+                    const cplx u = {rz * inv, -iz * inv};
+                    cplx q = sh.coef[P - 1];
 #pragma unroll
-                        for (int j = P / 2 - 2; j >= 0; --j) {
-                            const float4 d = s_coef32[warp][j];
-                            const float2 tr = __ffma2_rn(qi2, nwi2, make_float2(d.x, d.y));
-                            const float2 ti = __ffma2_rn(qi2, wr2, make_float2(d.z, d.w));
-                            const float2 nqr = __ffma2_rn(qr2, wr2, tr);
-                            qi2 = __ffma2_rn(qr2, wi2, ti);
-                            qr2 = nqr;
-                        }
-                        const float2 q = make_float2(
-                            qr2.x + fmaf(ur, qr2.y, -ui * qi2.y),
-                            qi2.x + fmaf(ur, qi2.y, ui * qr2.y));
-                        two_sum_add(sh, sl, ur * q.x - ui * q.y);
-                        far += mm * log_pos(r2, s_neg_log_c) * 0.5;
-                    } else {
-                        const double inv = 1.0 / r2;
-                        const cplx u = {rz * inv, -iz * inv};
-                        cplx q = s_coef[warp][P - 1];
-#pragma unroll
-                        for (int k = P - 2; k >= 0; --k) q = cfma(q, u, s_coef[warp][k]);
-                        far += mm * log_pos(r2, s_neg_log_c) * 0.5 +
-                               (u.re * q.re - u.im * q.im);
-                    }
+                    for (int k = P - 2; k >= 0; --k) q = cfma(q, u, sh.coef[k]);
+                    far += mm * log_near(r2, tab, copy) * 0.5 + (u.re * q.re - u.im * q.im);
                 }
             }
-            if (MIXED) far += (double)sh + (double)sl;
         }
 
         // P2P (potential-kernels.m4:19-57): 0.5 sum v log(r2 + eps) over the tiles of the
@@ -493,38 +732,19 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval(
                 py = ys[t0 + lane];
                 pv = vs[t0 + lane];
             }
-            float nh = 0, nl = 0, txh = 0, txl = 0, tyh = 0, tyl = 0;
-            if (MIXED) {
-                split2(x - xref, txh, txl);
-                split2(y - yref, tyh, tyl);
-            }
-            const float ln2 = 0.6931471805599453f, epsf = (float)eps;
+            // a sparse leaf's spreading (below): its mask, 32 / k, lane / k and the lane's target
+            unsigned spread = 0;
+            int sr = 0, sq = 0;
+            double qx = 0, qy = 0;
             while (tn > 0) {
                 const int cnt = tn;
                 const unsigned cmask = msk;   // this tile's targets (msk moves on to the next tile)
                 const bool mine = (cmask >> lane) & 1;
                 __syncwarp();
-                if (MIXED) {
-                    // source `lane` to entry lane / 2, half lane % 2; lanes past the tile add a
-                    // zero-valued source at the reference point (finite, contributes 0)
-                    float a = 0.f, b2 = 0.f, c2 = 0.f, d2 = 0.f, vv = 0.f;
-                    if (lane < cnt) {
-                        split2(px - xref, a, b2);
-                        split2(py - yref, c2, d2);
-                        vv = (float)pv;
-                    }
-                    float *nx = reinterpret_cast<float *>(s_nx[warp]);
-                    float *ny = reinterpret_cast<float *>(s_ny[warp]);
-                    const int e = 4 * (lane >> 1) + (lane & 1);
-                    nx[e] = -a;
-                    nx[e + 2] = -b2;
-                    ny[e] = -c2;
-                    ny[e + 2] = -d2;
-                    reinterpret_cast<float *>(s_v2[warp])[lane] = vv;
-                } else if (lane < cnt) {
-                    s_xy[warp][lane] = make_double2(px, py);
-                    s_v[warp][lane] = pv;
-                }
+                // (lanes past the tile: a zero value at the origin, for the two-source steps)
+                const bool live = lane < cnt;
+                sh.src.xy[lane] = make_double2(live ? px : 0.0, live ? py : 0.0);
+                sh.src.v[lane] = live ? pv : 0.0;
                 __syncwarp();
                 next_tile(t0, tn, msk);
                 if (lane < tn) {
@@ -532,90 +752,58 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval(
                     py = ys[t0 + lane];
                     pv = vs[t0 + lane];
                 }
-                // A tile needed by few targets of the group (k <= 16; k <= 8 in the mixed form,
-                // whose per-pair cost is lower) is spread over the lanes:
+                // A tile needed by few targets of the group (k <= 16) is spread over the lanes:
                 // lane l takes target q = l % k of the mask and sources l / k, l / k + r, ...
                 // (r = 32 / k), and each target adds its r lane partials in lane order.  Denser
-                // tiles keep one target per lane.
+                // tiles keep one target per lane, two sources per step.
                 const int k = __popc(cmask);
-                if (k > (MIXED ? 8 : 16)) {
+                if (k > 16) {
                     if (mine) {
-                        if (MIXED) {
-                            // two sources per step in f32x2 lanes; even and odd sources are
-                            // summed apart and added at the end of the tile
-                            const float2 txh2 = make_float2(txh, txh), txl2 = make_float2(txl, txl);
-                            const float2 tyh2 = make_float2(tyh, tyh), tyl2 = make_float2(tyl, tyl);
-                            const float2 eps2 = make_float2(epsf, epsf);
-                            float2 acc = make_float2(0.f, 0.f);
-                            const int npairs = (cnt + 1) >> 1;
-#pragma unroll 4
-                            for (int q = 0; q < npairs; ++q) {
-                                const float4 nx = s_nx[warp][q], ny = s_ny[warp][q];
-                                const float2 dx = __fadd2_rn(__fadd2_rn(txh2, make_float2(nx.x, nx.y)),
-                                                             __fadd2_rn(txl2, make_float2(nx.z, nx.w)));
-                                const float2 dy = __fadd2_rn(__fadd2_rn(tyh2, make_float2(ny.x, ny.y)),
-                                                             __fadd2_rn(tyl2, make_float2(ny.z, ny.w)));
-                                const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, eps2));
-                                acc = __ffma2_rn(make_float2(lg2_approx(r2.x), lg2_approx(r2.y)),
-                                                 s_v2[warp][q], acc);
-                            }
-                            two_sum_add(nh, nl, (acc.x + acc.y) * ln2);
-                        } else {
-#pragma unroll 4
-                            for (int q = 0; q < cnt; ++q) {
-                                const double2 sp = s_xy[warp][q];
-                                const double xr = x - sp.x, yr = y - sp.y;
-                                near += log_pos(fma(xr, xr, fma(yr, yr, eps)), s_neg_log_c) *
-                                        s_v[warp][q];
-                            }
+                        const double2 *v2 = reinterpret_cast<const double2 *>(sh.src.v);
+                        double n0 = 0, n1 = 0;
+#pragma unroll 2
+                        for (int q = 0; q < cnt; q += 2) {
+                            const double2 sp = sh.src.xy[q], sq = sh.src.xy[q + 1];
+                            const double2 v = v2[q >> 1];
+                            const double xr = x - sp.x, yr = y - sp.y;
+                            const double xq = x - sq.x, yq = y - sq.y;
+                            n0 = fma(log_near(fma(xr, xr, fma(yr, yr, eps)), tab, copy), v.x, n0);
+                            n1 = fma(log_near(fma(xq, xq, fma(yq, yq, eps)), tab, copy), v.y, n1);
                         }
+                        near += n0 + n1;
                     }
                 } else if (k > 0) {
-                    const int r = 32 / k;
-                    const int qt = lane % k;
-                    const int tl = (int)__fns(cmask, 0, qt + 1);   // lane of this lane's target
-                    double part = 0;
-                    if (MIXED) {
-                        const float qxh = __shfl_sync(FULL_MASK, txh, tl);
-                        const float qxl = __shfl_sync(FULL_MASK, txl, tl);
-                        const float qyh = __shfl_sync(FULL_MASK, tyh, tl);
-                        const float qyl = __shfl_sync(FULL_MASK, tyl, tl);
-                        float acc = 0;
-                        const float *nx = reinterpret_cast<const float *>(s_nx[warp]);
-                        const float *ny = reinterpret_cast<const float *>(s_ny[warp]);
-                        const float *sv = reinterpret_cast<const float *>(s_v2[warp]);
-                        if (lane < r * k)
-                            for (int q = lane / k; q < cnt; q += r) {
-                                const int e = 4 * (q >> 1) + (q & 1);
-                                const float dx = (qxh + nx[e]) + (qxl + nx[e + 2]);
-                                const float dy = (qyh + ny[e]) + (qyl + ny[e + 2]);
-                                acc = fmaf(lg2_approx(fmaf(dx, dx, fmaf(dy, dy, epsf))), sv[q], acc);
-                            }
-                        part = (double)acc;
-                    } else {
-                        const double qx = __shfl_sync(FULL_MASK, x, tl);
-                        const double qy = __shfl_sync(FULL_MASK, y, tl);
-                        if (lane < r * k)
-                            for (int q = lane / k; q < cnt; q += r) {
-                                const double2 sp = s_xy[warp][q];
-                                const double xr = qx - sp.x, yr = qy - sp.y;
-                                part += log_pos(fma(xr, xr, fma(yr, yr, eps)), s_neg_log_c) *
-                                        s_v[warp][q];
-                            }
+                    if (cmask != spread) {   // once per leaf: its tiles share the mask
+                        spread = cmask;
+                        __syncwarp();
+                        if (mine) sh.lane_of[__popc(cmask & ((1u << lane) - 1u))] = lane;
+                        __syncwarp();
+                        sr = 32 / k;
+                        sq = lane / k;
+                        const int tl = sh.lane_of[lane - sq * k];   // lane of this lane's target
+                        qx = __shfl_sync(FULL_MASK, x, tl);
+                        qy = __shfl_sync(FULL_MASK, y, tl);
                     }
-                    s_part[warp][lane] = part;
+                    const int r = sr;
+                    double sum = 0;
+                    if (lane < r * k)
+                        for (int q = sq; q < cnt; q += r) {
+                            const double2 sp = sh.src.xy[q];
+                            const double xr = qx - sp.x, yr = qy - sp.y;
+                            sum = fma(log_near(fma(xr, xr, fma(yr, yr, eps)), tab, copy),
+                                      sh.src.v[q], sum);
+                        }
+                    sh.part[lane] = sum;
                     __syncwarp();
                     if (mine) {
                         const int q = __popc(cmask & ((1u << lane) - 1u));
-                        double sum = 0;
-                        for (int i = 0; i < r; ++i) sum += s_part[warp][q + i * k];
-                        if (MIXED) two_sum_add(nh, nl, (float)sum * ln2);
-                        else near += sum;
+                        double tot = 0;
+                        for (int i = 0; i < r; ++i) tot += sh.part[q + i * k];
+                        near += tot;
                     }
                     __syncwarp();
                 }
             }
-            if (MIXED) near = (double)nh + (double)nl;
         }
         const double res = 0.5 * near + far;
         if (nparts == 1) {
@@ -793,16 +981,31 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
                    c.stream>>>(c.nnodes, tnode, slot_ptr<double>(c, S_EXPS), sexp, sscale);
             TC_KERNEL_CHECK();
         }
-        auto eval = mixed ? k_potential_eval<P, true> : k_potential_eval<P, false>;
-        const int occ = mixed ? blocks_per_sm<k_potential_eval<P, true>>(PE_WARPS * 32, 0)
-                              : blocks_per_sm<k_potential_eval<P, false>>(PE_WARPS * 32, 0);
-        const int egrid = (int)std::min<long long>((ntasks + PE_WARPS - 1) / PE_WARPS,
-                                                   (long long)sm_count_p() * occ);
-        phase_mark(c, 6);
-        eval<<<egrid, PE_WARPS * 32, 0, c.stream>>>(
-            ngroups, m, xt, yt, vo, tnode, slot_ptr<double>(c, S_MASS), slot_ptr<double>(c, S_EXPS),
-            slot_ptr<int2>(c, S_RANGE), slot_ptr<double>(c, S_XS), slot_ptr<double>(c, S_YS),
-            slot_ptr<double>(c, S_VS), offs, lists, out, partial, task_ctr, task_group, sexp, sscale, seg);
+        if (mixed) {
+            const int occ = blocks_per_sm<k_potential_eval_mixed<P>>(PE_WARPS * 32, 0);
+            const int egrid = (int)std::min<long long>((ntasks + PE_WARPS - 1) / PE_WARPS,
+                                                       (long long)sm_count_p() * occ);
+            phase_mark(c, 6);
+            k_potential_eval_mixed<P><<<egrid, PE_WARPS * 32, 0, c.stream>>>(
+                ngroups, m, xt, yt, vo, tnode, slot_ptr<double>(c, S_MASS),
+                slot_ptr<int2>(c, S_RANGE), slot_ptr<double>(c, S_XS), slot_ptr<double>(c, S_YS),
+                slot_ptr<double>(c, S_VS), offs, lists, out, partial, task_ctr, task_group, sexp,
+                sscale);
+        } else {
+            static const cudaError_t attr_rc =
+                cudaFuncSetAttribute(k_potential_eval<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)eval_smem<P>());
+            TC_CUDA_TRY(attr_rc);
+            const int occ = blocks_per_sm<k_potential_eval<P>>(PD_WARPS * 32, eval_smem<P>());
+            const int egrid = (int)std::min<long long>((ntasks + PD_WARPS - 1) / PD_WARPS,
+                                                       (long long)sm_count_p() * occ);
+            phase_mark(c, 6);
+            k_potential_eval<P><<<egrid, PD_WARPS * 32, eval_smem<P>(), c.stream>>>(
+                ngroups, m, xt, yt, vo, tnode, slot_ptr<double>(c, S_MASS),
+                slot_ptr<double>(c, S_EXPS), slot_ptr<int2>(c, S_RANGE), slot_ptr<double>(c, S_XS),
+                slot_ptr<double>(c, S_YS), slot_ptr<double>(c, S_VS), offs, lists, out, partial,
+                task_ctr, task_group, seg);
+        }
         TC_KERNEL_CHECK();
         return TC_OK;
     });
@@ -821,8 +1024,8 @@ void kernels_potential(KernelList &v) {
                        (const void *)k_potential_lists_copy, (const void *)k_task_map_groups,
                        (const void *)k_potential_gather_parts});
 #define TC_POTENTIAL_KERNELS(P)                                                                  \
-    v.insert(v.end(), {(const void *)k_potential_eval<P, true>,                                 \
-                       (const void *)k_potential_eval<P, false>, (const void *)k_scale_coeffs_pot<P>});
+    v.insert(v.end(), {(const void *)k_potential_eval_mixed<P>, (const void *)k_potential_eval<P>, \
+                       (const void *)k_scale_coeffs_pot<P>});
     TC_FOR_EACH_ORDER(TC_POTENTIAL_KERNELS)
 #undef TC_POTENTIAL_KERNELS
 }

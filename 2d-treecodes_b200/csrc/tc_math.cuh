@@ -3,6 +3,7 @@
 
 #include "tc_common.cuh"
 #include "tc_log_table.cuh"
+#include "tc_near_log_table.cuh"
 
 namespace tc {
 
@@ -62,6 +63,51 @@ __device__ __forceinline__ double log_pos(double x, const double *__restrict__ n
 // Copies log_pos's table into the block's shared memory; every thread of the block calls it.
 __device__ __forceinline__ void load_log_table(double *s_neg_log_c) {
     for (int i = threadIdx.x; i < LOG_NTAB; i += blockDim.x) s_neg_log_c[i] = LOG_NEG_LOG_C[i];
+    __syncthreads();
+}
+
+// The logarithm of the FP64 potential evaluation: as log_pos, with the reduction's reciprocal c
+// read from the table beside -log c instead of formed by the approximate-reciprocal unit, and
+// the polynomial nested onto the table value: 7 FP64 operations, one conversion, 6 integer ones
+// and one 16-byte shared load, against log_pos's 8, one, 9, a reciprocal and an 8-byte load.  (An
+// FP64 instruction takes two issue slots, so both kinds count.)  The table stands in shared
+// memory NLOG_COPIES times, copy k of entry i at 8 i + k, and a lane reads copy lane % 8: the eight
+// lanes that a 16-byte shared load serves at once then never meet in a bank.
+// fit_near_log_table.py beside this file writes the table; any positive normal x; within 2 ulp
+// of the exact logarithm (tests/test_near_log_table.py).
+constexpr int NLOG_COPIES = 8;
+
+// `tab`: the table's 32-bit shared-memory address; `copy`: the lane's copy, 16 (lane % 8).
+__device__ __forceinline__ unsigned shared_address(const void *p) {
+    return (unsigned)__cvta_generic_to_shared(p);
+}
+
+// (in the constant bank: as literals they were moved into uniform registers again for every source)
+static __constant__ double c_nlog[5] = {NLOG_Q0, NLOG_Q1, NLOG_Q2, NLOG_Q3, 0x1.62e42fefa39efp-1};
+
+__device__ __forceinline__ double log_near(double x, unsigned tab, int copy) {
+    const int ix = __double2hiint(x) - NLOG_BASE;
+    const int e = ix >> 20;
+    // entry (ix >> (20 - NLOG_BITS)) mod NLOG_NTAB, NLOG_COPIES * 16 bytes each
+    constexpr int SHIFT = 20 - NLOG_BITS - 7;
+    static_assert(NLOG_COPIES * sizeof(double2) == 128, "entry stride 2^7 bytes");
+    const int off = ((ix >> SHIFT) & ((NLOG_NTAB - 1) << 7)) | copy;
+    double c, t0;   // (not volatile: the table does not change while it is read)
+    asm("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(c), "=d"(t0) : "r"(tab + off));
+    // r = m c - 1 = x (c 2^-e) - 1: c's exponent takes the scaling (c is in [0.7, 1.42))
+    c = __hiloint2double(__double2hiint(c) - (ix & (int)0xfff00000), __double2loint(c));
+    const double r = fma(x, c, -1.0);
+    double t = fma(c_nlog[3], r, c_nlog[2]);
+    t = fma(t, r, c_nlog[1]);
+    t = fma(t, r, c_nlog[0]);
+    t = fma(t, r, 1.0);
+    return fma((double)e, c_nlog[4], fma(t, r, t0));
+}
+
+// Fills the block's copies of log_near's table; every thread of the block calls it.
+__device__ __forceinline__ void load_near_log_table(double2 *s_tab) {
+    for (int i = threadIdx.x; i < NLOG_NTAB * NLOG_COPIES; i += blockDim.x)
+        s_tab[i] = NLOG_TAB[i / NLOG_COPIES];
     __syncthreads();
 }
 
