@@ -200,27 +200,15 @@ __global__ __launch_bounds__(RANK_THREADS) void k_rank_count(const unsigned shor
 __global__ __launch_bounds__(1024) void k_rank_scan(int *__restrict__ blk, int nblk,
                                                     int *__restrict__ totals) {
     pdl_begin();
-    __shared__ int s_part[1024];
     const int l = blockIdx.x;
     int *row = blk + (size_t)l * nblk;
     const int per = (nblk + 1023) / 1024;
     const int b0 = threadIdx.x * per;
-    int s = 0;
+    int s = 0, total;
     for (int i = 0; i < per; ++i)
         if (b0 + i < nblk) s += row[b0 + i];
-    s_part[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int t = 0; t < 1024; ++t) {
-            const int v = s_part[t];
-            s_part[t] = run;
-            run += v;
-        }
-        totals[l] = run;
-    }
-    __syncthreads();
-    int run = s_part[threadIdx.x];
+    int run = block_exclusive_scan(s, &total);
+    if (threadIdx.x == 0) totals[l] = total;
     for (int i = 0; i < per; ++i)
         if (b0 + i < nblk) {
             const int v = row[b0 + i];
@@ -270,13 +258,65 @@ __global__ __launch_bounds__(RANK_THREADS) void k_rank_apply(const unsigned shor
     }
 }
 
+// The three rank kernels in one block, for short lists: 1024 entries at a time, the levels' running
+// counts kept in shared memory.  A chunk takes about 1.5 us, the three launches about 7.
+constexpr int RANK_SMALL = 4096;   // list capacity up to which this kernel runs
 
-__global__ void k_tree_root(int n, int leafcap, TNode *tnode, int2 *range, int4 *cell) {
+__global__ __launch_bounds__(RANK_THREADS) void k_rank_small(const unsigned short *__restrict__ lmask,
+                                                             const int *__restrict__ d_nlist,
+                                                             int *__restrict__ rank,
+                                                             int *__restrict__ inv, int stride,
+                                                             int *__restrict__ totals) {
     pdl_begin();
+    __shared__ int s_w[LMAX][RANK_THREADS / 32 + 1];
+    __shared__ int s_run[LMAX];
+    const int nlist = min(*d_nlist, stride);
+    const int w = threadIdx.x >> 5;
+    const unsigned lt = lanemask_lt();
+    if (threadIdx.x < LMAX) s_run[threadIdx.x] = 0;
+    for (int base = 0; base < nlist; base += RANK_THREADS) {
+        const int j = base + threadIdx.x;
+        const unsigned m = j < nlist ? lmask[j] : 0u;
+        unsigned bal[LMAX];
+#pragma unroll
+        for (int l = 0; l < LMAX; ++l) {
+            bal[l] = __ballot_sync(FULL_MASK, (m >> l) & 1u);
+            if (lane_id() == 0) s_w[l][w] = __popc(bal[l]);
+        }
+        __syncthreads();
+        // warp l scans level l's warp counts
+        if (w < LMAX) {
+            const int v = s_w[w][lane_id()];
+            int inc = v;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(FULL_MASK, inc, o);
+                if (lane_id() >= o) inc += t;
+            }
+            const int run = s_run[w];
+            __syncwarp();
+            s_w[w][lane_id()] = run + inc - v;
+            if (lane_id() == 31) s_run[w] = run + inc;
+        }
+        __syncthreads();
+        if (j < nlist)
+#pragma unroll
+            for (int l = 0; l < LMAX; ++l) {
+                const int r = s_w[l][w] + __popc(bal[l] & lt);
+                rank[(size_t)l * stride + j] = r;
+                if ((m >> l) & 1u) inv[(size_t)l * stride + r] = j;
+            }
+        __syncthreads();
+    }
+    __syncthreads();
+    if (threadIdx.x < LMAX) totals[threadIdx.x] = s_run[threadIdx.x];
+}
+
+// The root of a tree without inner cells.
+__global__ void k_tree_root(int n, TNode *tnode, int2 *range, int4 *cell) {
     range[0] = make_int2(0, n);
     cell[0] = make_int4(0, 0, 0, -1);
     tnode[0].count = n;
-    if (n <= leafcap) tnode[0].child = -1;
+    tnode[0].child = -1;
 }
 
 // Four threads per inner cell: the r-th inner cell of level l is started by list entry
@@ -331,6 +371,11 @@ __global__ void k_tree_children(const int *__restrict__ keys, int n, int leafcap
             continue;
         }
         if (q == 0) tnode[id].child = base;
+        if (l == 0 && q == 0) {   // the root's record (k_tree_root, when nothing is split)
+            range[0] = make_int2(0, n);
+            cell[0] = make_int4(0, 0, 0, -1);
+            tnode[0].count = n;
+        }
         const int cshift = shift - 2;
         // the end of child q: the first key of child q + 1, or past the cell for q = 3
         int end_q;
@@ -393,15 +438,22 @@ int build_topology(Context &c, int leafcap) {
     // a test stall leaves the list offsets wrong: report it before anything reads them
     if (c.test_stall == TC_STALL_TREE && (rc = check_device_errors(c, "tree build"))) return rc;
     // the rank kernels follow k_tree_list directly (launch_pdl)
-    TC_CUDA_TRY(launch_pdl(ovl, k_rank_count, nblk, RANK_THREADS, 0, c.stream,
-                           (const unsigned short *)lmask, (const int *)d_nlist, blkc, nblk));
-    TC_KERNEL_CHECK();
-    TC_CUDA_TRY(launch_pdl(ovl, k_rank_scan, LMAX, 1024, 0, c.stream, blkc, nblk, totals));
-    TC_KERNEL_CHECK();
-    TC_CUDA_TRY(launch_pdl(ovl, k_rank_apply, nblk, RANK_THREADS, 0, c.stream,
-                           (const unsigned short *)lmask, (const int *)d_nlist, (const int *)blkc,
-                           nblk, rank, rinv, cap));
-    TC_KERNEL_CHECK();
+    if (cap <= RANK_SMALL) {
+        TC_CUDA_TRY(launch_pdl(ovl, k_rank_small, 1, RANK_THREADS, 0, c.stream,
+                               (const unsigned short *)lmask, (const int *)d_nlist, rank, rinv, cap,
+                               totals));
+        TC_KERNEL_CHECK();
+    } else {
+        TC_CUDA_TRY(launch_pdl(ovl, k_rank_count, nblk, RANK_THREADS, 0, c.stream,
+                               (const unsigned short *)lmask, (const int *)d_nlist, blkc, nblk));
+        TC_KERNEL_CHECK();
+        TC_CUDA_TRY(launch_pdl(ovl, k_rank_scan, LMAX, 1024, 0, c.stream, blkc, nblk, totals));
+        TC_KERNEL_CHECK();
+        TC_CUDA_TRY(launch_pdl(ovl, k_rank_apply, nblk, RANK_THREADS, 0, c.stream,
+                               (const unsigned short *)lmask, (const int *)d_nlist, (const int *)blkc,
+                               nblk, rank, rinv, cap));
+        TC_KERNEL_CHECK();
+    }
     // the level totals and the list length, in one read-back
     TC_CUDA_TRY(cudaMemcpyAsync(c.h_pinned, totals, sizeof(int) * (LMAX + 1),
                                 cudaMemcpyDeviceToHost, c.stream));
@@ -442,22 +494,20 @@ int build_topology(Context &c, int leafcap) {
     if ((rc = ensure(c, S_TNODE, nnodes, &tnode)) || (rc = ensure(c, S_RANGE, nnodes, &range)) ||
         (rc = ensure(c, S_CELL, nnodes, &cell)))
         return rc;
-    k_tree_root<<<1, 1, 0, c.stream>>>(n, leafcap, tnode, range, cell);
+    if (ninner == 0)
+        k_tree_root<<<1, 1, 0, c.stream>>>(n, tnode, range, cell);
+    else
+        k_tree_children<<<grid_for_tree(4 * (int)ninner, 128), 128, 0, c.stream>>>(
+            keys, n, leafcap, lpos, lmask, rank, rinv, cap, (int)ninner, lo, c.nnodes, tnode, range,
+            cell, err);
     TC_KERNEL_CHECK();
-    if (ninner > 0) {
-        TC_CUDA_TRY(launch_pdl(ovl, k_tree_children, grid_for_tree(4 * (int)ninner, 128), 128, 0,
-                               c.stream, keys, n, leafcap, (const int *)lpos,
-                               (const unsigned short *)lmask, (const int *)rank,
-                               (const int *)rinv, cap, (int)ninner, lo, c.nnodes, tnode, range,
-                               cell, slot_ptr<unsigned>(c, S_ERR)));
-        TC_KERNEL_CHECK();
-    }
     return TC_OK;
 }
 
 void kernels_tree(KernelList &v) {
     v.insert(v.end(), {(const void *)k_tree_list, (const void *)k_rank_count,
                        (const void *)k_rank_scan, (const void *)k_rank_apply,
+                       (const void *)k_rank_small,
                        (const void *)k_tree_root, (const void *)k_tree_children});
 }
 

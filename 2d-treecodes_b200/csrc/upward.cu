@@ -48,7 +48,10 @@ __device__ const BinomTable g_binom_up = make_binom_table();   // per-lane indic
 
 constexpr int UP_WARPS = 4;          // warps per block of the leaf and per-level merge kernels
 constexpr int UP_TOP_WARPS = 16;     // warps of the single-block launch over the top levels
-constexpr int UP_TOP_MAX_NODES = 64;     // a level this small joins the single-block launch
+// A level this small joins the single-block launch.  One SM reads the children of 64 nodes no
+// faster than a launch over several takes (a launch follows in ~2.5 us): 64 -> 16 took ~8 us off
+// the upward phase of solves of 64K to 1M sources, and nothing off the smallest.
+constexpr int UP_TOP_MAX_NODES = 16;
 constexpr int UP_WIDE_MIN_NODES = 2048;  // a level with this many inner nodes: k_upward_wide
 
 
@@ -674,7 +677,10 @@ static LevelOffsets level_offsets(const Context &c) {
     return offs;
 }
 
-constexpr int MOM_TOP_MAX = 1024;   // levels with at most this many inner nodes: one block
+// Levels with at most this many inner nodes: one block.  With 1024 the single SM's share of the
+// L2 bandwidth bound it (28 words a node: 43 us on the 16M sheet); at 64 the wide levels get
+// launches of their own: the upward phase of a 300K-source solve 127 -> 102 us.
+constexpr int MOM_TOP_MAX = 64;
 
 int upward_moments(Context &c) {
     const bool ovl = c.launch_overlap;   // launch_pdl chains (tc_set_launch_overlap)
