@@ -125,18 +125,16 @@ cudaError_t wait_event(Context &c, cudaEvent_t e) {
     return poll_and_sleep([e] { return cudaEventQuery(e); });
 }
 
-// Reads back the device error word and the work counters (one sync).  The counters land in
-// h_pinned[16 ...] as unsigned long long.
+// Reads back the device error word and the work counters behind it (one copy, one sync).
+constexpr int PINNED_ERR = 64;   // their place in h_pinned, in words
 int check_device_errors(Context &c, const char *where) {
-    unsigned *err = slot_ptr<unsigned>(c, S_ERR);
-    TC_CUDA_TRY(cudaMemcpyAsync(c.h_pinned + 8, err, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                                c.stream));
-    TC_CUDA_TRY(cudaMemcpyAsync(c.h_pinned + 16, c.buf[S_STATS].p,
-                                sizeof(unsigned long long) * STAT_SLOTS, cudaMemcpyDeviceToHost,
+    const size_t bytes = reinterpret_cast<char *>(c.ctrl.stats + STAT_SLOTS) -
+                         reinterpret_cast<char *>(c.ctrl.err);
+    TC_CUDA_TRY(cudaMemcpyAsync(c.h_pinned + PINNED_ERR, c.ctrl.err, bytes, cudaMemcpyDeviceToHost,
                                 c.stream));
     TC_CUDA_TRY(wait_stream(c, c.stream));
     c.counts.launches = g_launches;
-    const unsigned e = c.h_pinned[8];
+    const unsigned e = c.h_pinned[PINNED_ERR];
     if (e & DEVERR_SPIN_LIMIT) {
         set_error(TC_ERR_TIMEOUT, "%s: a bounded device wait gave up (flags 0x%x)", where, e);
         return TC_ERR_TIMEOUT;
@@ -154,7 +152,8 @@ int check_device_errors(Context &c, const char *where) {
 }
 
 static unsigned long long stat_counter(Context &c, int slot) {
-    return reinterpret_cast<unsigned long long *>(c.h_pinned + 16)[slot];
+    const size_t words = reinterpret_cast<unsigned *>(c.ctrl.stats) - c.ctrl.err;
+    return reinterpret_cast<unsigned long long *>(c.h_pinned + PINNED_ERR + words)[slot];
 }
 
 int device_sm_count() {
@@ -298,13 +297,6 @@ static int context_init(Context &c, int device, cudaStream_t stream) {
         return TC_ERR_ALLOC;
     }
     for (auto &ev : c.ev) TC_CUDA_TRY(cudaEventCreate(&ev));
-    unsigned *err;
-    unsigned long long *stats;
-    int rc;
-    if ((rc = ensure(c, S_ERR, 64, &err))) return rc;
-    if ((rc = ensure(c, S_STATS, STAT_SLOTS, &stats))) return rc;
-    TC_CUDA_TRY(cudaMemsetAsync(err, 0, 64 * sizeof(unsigned), c.stream));
-    TC_CUDA_TRY(cudaMemsetAsync(stats, 0, STAT_SLOTS * sizeof(unsigned long long), c.stream));
     context_counted(device, +1);
     c.live = true;
     return TC_OK;
@@ -361,13 +353,12 @@ static void finish_timing(Context &c) {
 // traversals read.  The expansions follow separately (upward_expansions), so that they can be
 // formed while the interaction lists are built.
 static int build_tree_moments(Context &c, int kind, const double *x, const double *y,
-                              const double *v, int n, cudaEvent_t values_ready = nullptr) {
+                              const double *v, int n, int m = 0,
+                              cudaEvent_t values_ready = nullptr) {
     int rc;
     g_launches = 0;
     c.near_marked = false;
-    TC_CUDA_TRY(cudaMemsetAsync(slot_ptr<unsigned>(c, S_ERR), 0, sizeof(unsigned), c.stream));
-    TC_CUDA_TRY(cudaMemsetAsync(c.buf[S_STATS].p, 0, STAT_SLOTS * sizeof(unsigned long long),
-                                c.stream));
+    if ((rc = ctrl_prepare(c, n, m))) return rc;
     if ((rc = sort_sources(c, x, y, v, n, values_ready))) return rc;
     phase_mark(c, 1);
     if ((rc = build_topology(c, kind ? LEAF_FORCE : LEAF_POTENTIAL))) return rc;
@@ -410,7 +401,7 @@ static int potential_device(Context &c, double theta, const double *xs, const do
     }
     int rc;
     phase_mark(c, 0);
-    if ((rc = build_tree_moments(c, 0, xs, ys, vs, n, values_ready))) return rc;
+    if ((rc = build_tree_moments(c, 0, xs, ys, vs, n, m, values_ready))) return rc;
     if ((rc = potential(c, theta, xt, yt, m, out, expansions_then_mark))) return rc;
     phase_mark(c, 5);
     if ((rc = check_device_errors(c, "treecode_potential"))) return rc;
@@ -444,7 +435,7 @@ static int force_device(Context &c, double theta, const double *xs, const double
     }
     int rc;
     phase_mark(c, 0);
-    if ((rc = build_tree_moments(c, 1, xs, ys, vs, n, values_ready))) return rc;
+    if ((rc = build_tree_moments(c, 1, xs, ys, vs, n, 0, values_ready))) return rc;
     if ((rc = force_mrag(c, theta, x0s, y0s, hs, nb, xo, yo, expansions_then_mark, host_x,
                          host_y)))
         return rc;
@@ -754,7 +745,6 @@ TC_API int tc_context_trim(tc_context *ctx) {
     TC_CUDA_TRY(cudaStreamSynchronize(c.stream));
     TC_CUDA_TRY(cudaStreamSynchronize(c.aux));
     for (int s = 0; s < S_NUM_SLOTS; ++s) {
-        if (s == S_ERR || s == S_STATS) continue;   // created with the context, tiny
         DevBuf &b = c.buf[s];
         if (b.p) cudaFreeAsync(b.p, c.stream);   // no device-wide synchronisation
         b.p = nullptr;

@@ -212,22 +212,28 @@ __global__ __launch_bounds__(TR_WARPS * 32) void k_force_lists(
     }
 }
 
-// The lists in CSR order from the scratch runs of k_force_lists<2>: warp per brick.
+// The lists in CSR order from the scratch runs of k_force_lists<2>, and the task -> brick map:
+// warp per brick.
 __global__ __launch_bounds__(256) void k_force_lists_copy(int nbricks,
                                                           const int *__restrict__ counts,
                                                           const int *__restrict__ offs,
                                                           const int *__restrict__ sstart,
                                                           const int *__restrict__ scratch,
-                                                          int *__restrict__ lists) {
+                                                          int *__restrict__ lists,
+                                                          int *__restrict__ task_brick) {
     const int lane = lane_id();
+    const int *toff = offs + 3 * nbricks;
+    const int tbase = toff[0];
     for (int brick = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; brick < nbricks;
-         brick += (gridDim.x * blockDim.x) >> 5)
+         brick += (gridDim.x * blockDim.x) >> 5) {
         for (int k = 0; k < 3; ++k) {
             const int n = counts[k * nbricks + brick];
             const int *src = scratch + sstart[k * nbricks + brick];
             int *dst = lists + offs[k * nbricks + brick];
             for (int i = lane; i < n; i += 32) dst[i] = src[i];
         }
+        for (int t = toff[brick] + lane; t < toff[brick + 1]; t += 32) task_brick[t - tbase] = brick;
+    }
 }
 
 // ------------------------------------------------------------------------------ evaluation
@@ -847,7 +853,7 @@ __global__ __launch_bounds__(256) void k_add_far(double *__restrict__ xout,
     }
 }
 
-// task -> brick map of the evaluation tasks
+// task -> brick map of the evaluation tasks (when a second walk wrote the lists)
 __global__ void k_task_map(int nbricks, const int *__restrict__ offs, int *__restrict__ task_brick) {
     const int *toff = offs + 3 * nbricks;
     const int tbase = toff[0];
@@ -930,7 +936,7 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
         (rc = ensure(c, S_FOFF, (size_t)4 * nbricks + 1, &offs)))
         return rc;
     const TNode *tnode = slot_ptr<TNode>(c, S_TNODE);
-    unsigned *err = slot_ptr<unsigned>(c, S_ERR);
+    unsigned *err = c.ctrl.err;
     const int trgrid = (int)std::min<long long>((nbricks + TR_WARPS - 1) / TR_WARPS,
                                                 (long long)sm_count() * 16);
     // One walk counts the lists and writes them into per-warp scratch runs; after the scan a
@@ -941,32 +947,27 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
     const int seg = near_segment(nbricks);
     ScratchLayout sl;
     ListScratch ls;   // released (when transient) after the copy, in stream order
-    int *sstart, *meta;
+    int *sstart, *meta = c.ctrl.meta;
     {
         AuxScope on_aux(c);
         if ((rc = list_scratch(c, 3, nwarps, nbricks, sizeof(int), sl, ls)) ||
-            (rc = ensure(c, S_LSTART, (size_t)3 * nbricks, &sstart)) ||
-            (rc = ensure(c, S_LMETA, 4, &meta)))
+            (rc = ensure(c, S_LSTART, (size_t)3 * nbricks, &sstart)))
             return rc;
     }
-    unsigned long long *stats = slot_ptr<unsigned long long>(c, S_STATS);
+    unsigned long long *stats = c.ctrl.stats;
     // traversal stack entries per warp: all of them, or fewer as a context's test setting
     const int stack_cap = c.stack_limit > 0 ? std::min(c.stack_limit, TR_STACK) : TR_STACK;
     TC_CUDA_TRY(cudaEventRecord(c.ev_fork, c.stream));
     {
         AuxScope on_aux(c);
         TC_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.ev_fork, 0));
-        TC_CUDA_TRY(cudaMemsetAsync(meta, 0, sizeof(int) * 4, c.stream));
         k_force_lists<2><<<trgrid, TR_WARPS * 32, 0, c.stream>>>(
             nbricks, L, x0s, y0s, hs, theta, tnode, c.nnodes, counts, nullptr, nullptr,
             static_cast<int *>(ls.p), sl, sstart, meta, err, stats, stack_cap, seg);
         TC_KERNEL_CHECK();
-        if ((rc = exclusive_scan(c, counts, offs, 4 * nbricks))) return rc;
-        for (int k = 0; k < 4; ++k)
-            TC_CUDA_TRY(cudaMemcpyAsync(c.h_pinned + 32 + k, offs + (k + 1) * nbricks, sizeof(int),
-                                        cudaMemcpyDeviceToHost, c.stream));
-        TC_CUDA_TRY(cudaMemcpyAsync(c.h_pinned + 36, meta, sizeof(int) * 4,
-                                    cudaMemcpyDeviceToHost, c.stream));
+        // the lists' totals and meta, written to h_pinned by the scan
+        if ((rc = exclusive_scan(c, counts, offs, 4 * nbricks, nbricks, c.h_pinned + 32, meta)))
+            return rc;
         TC_CUDA_TRY(cudaEventRecord(c.ev_totals, c.stream));
     }
     if (between && (rc = between(c))) {
@@ -986,19 +987,25 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
     c.counts.e2l_pairs = c.counts.n_e2l;
     c.counts.e2p_pairs = c.counts.n_e2p * TILE * TILE;
     c.counts.l2p_targets = (long long)nbricks * TILE * TILE;
-    int *lists;
+    int *lists, *task_brick;
     {
         AuxScope on_aux(c);
-        if ((rc = ensure(c, S_E2L, (size_t)tot[2] + 1, &lists))) return rc;
+        if ((rc = ensure(c, S_E2L, (size_t)tot[2] + 1, &lists)) ||
+            (rc = ensure(c, S_TASKMAP, (size_t)ntasks, &task_brick)))
+            return rc;
         if (!overflow) {
             k_force_lists_copy<<<(int)std::min<long long>((nbricks + 7) / 8,
                                                           (long long)sm_count() * 16),
                                  256, 0, c.stream>>>(nbricks, counts, offs, sstart,
-                                                     static_cast<const int *>(ls.p), lists);
+                                                     static_cast<const int *>(ls.p), lists,
+                                                     task_brick);
         } else {
             k_force_lists<1><<<trgrid, TR_WARPS * 32, 0, c.stream>>>(
                 nbricks, L, x0s, y0s, hs, theta, tnode, c.nnodes, nullptr, offs, lists, nullptr,
                 sl, nullptr, nullptr, err, nullptr, stack_cap, seg);
+            TC_KERNEL_CHECK();
+            k_task_map<<<(int)std::min<long long>((nbricks + 255) / 256, (long long)sm_count() * 8),
+                         256, 0, c.stream>>>(nbricks, offs, task_brick);
         }
         TC_KERNEL_CHECK();
         TC_CUDA_TRY(cudaEventRecord(c.ev_join, c.stream));
@@ -1007,23 +1014,16 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
     // the auxiliary stream as soon as the lists are in place, while the upward pass forms the
     // expansions and the far field is evaluated on the main stream.  The near field writes the
     // outputs, the far field buffers of its own, and k_add_far adds the two once both are done.
-    int *brick_ctr, *task_brick;
     // (measurement mode: the near field waits for the upward pass, the far field for it)
     if (c.serial_eval) TC_CUDA_TRY(cudaEventRecord(c.ev_serial, c.stream));
     {
         AuxScope on_aux(c);
         if (c.serial_eval) TC_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.ev_serial, 0));
-        // everything the near field uses is allocated and written on this stream (the far
-        // field's work counters are the main stream's own, S_FAR_CTR)
+        // everything the near field uses is allocated and written on this stream, but for its
+        // task counter, cleared at the solve's start, which the fork waits for (as the far
+        // field's own, on the main stream)
         double *partial;
-        if ((rc = ensure(c, S_BRICK_CTR, 1, &brick_ctr)) ||
-            (rc = ensure(c, S_FPART, (size_t)ntasks * 4 * 32, &partial)) ||
-            (rc = ensure(c, S_TASKMAP, (size_t)ntasks, &task_brick)))
-            return rc;
-        TC_CUDA_TRY(cudaMemsetAsync(brick_ctr, 0, sizeof(int), c.stream));
-        k_task_map<<<(int)std::min<long long>((nbricks + 255) / 256, (long long)sm_count() * 8),
-                     256, 0, c.stream>>>(nbricks, offs, task_brick);
-        TC_KERNEL_CHECK();
+        if ((rc = ensure(c, S_FPART, (size_t)ntasks * 4 * 32, &partial))) return rc;
         const bool mixed = c.precision == 1;
         constexpr int LBS32 = 5;   // the default block side, 32
         const bool fixed = L.lbs == LBS32;
@@ -1037,7 +1037,7 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
         near<<<neargrid, EV_WARPS * 32, 0, c.stream>>>(
             nbricks, L, x0s, y0s, hs, slot_ptr<int2>(c, S_RANGE), slot_ptr<double>(c, S_XS),
             slot_ptr<double>(c, S_YS), slot_ptr<double>(c, S_VS), offs, lists, xout, yout,
-            partial, 0, nbricks, brick_ctr, task_brick, seg);
+            partial, 0, nbricks, c.ctrl.near_ctr, task_brick, seg);
         TC_KERNEL_CHECK();
         if (ntasks > nbricks) {
             k_force_gather_parts<<<(int)std::min<long long>((nbricks + 7) / 8,
@@ -1085,11 +1085,9 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
         const size_t per_block = (size_t)1 << (2 * L.lbs);
         const size_t nt_all = (size_t)nblocks * per_block;
         double *xfar, *yfar;
-        int *far_ctr;
-        if ((rc2 = ensure(c, S_FARX, nt_all, &xfar)) || (rc2 = ensure(c, S_FARY, nt_all, &yfar)) ||
-            (rc2 = ensure(c, S_FAR_CTR, FORCE_CHUNKS, &far_ctr)))
+        int *far_ctr = c.ctrl.far_ctr;
+        if ((rc2 = ensure(c, S_FARX, nt_all, &xfar)) || (rc2 = ensure(c, S_FARY, nt_all, &yfar)))
             return rc2;
-        TC_CUDA_TRY(cudaMemsetAsync(far_ctr, 0, FORCE_CHUNKS * sizeof(int), c.stream));
         const int nchunks =
             host_x && (size_t)nblocks * per_block >= ((size_t)1 << 21) && nblocks >= FORCE_CHUNKS
                 ? FORCE_CHUNKS

@@ -248,22 +248,28 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
     }
 }
 
-// The lists in CSR order from the scratch runs of k_potential_lists<2>: warp per group.
+// The lists in CSR order from the scratch runs of k_potential_lists<2>, and the task -> group
+// map: warp per group.
 __global__ __launch_bounds__(256) void k_potential_lists_copy(int ngroups,
                                                               const int *__restrict__ counts,
                                                               const int *__restrict__ offs,
                                                               const int *__restrict__ sstart,
                                                               const int2 *__restrict__ scratch,
-                                                              int2 *__restrict__ lists) {
+                                                              int2 *__restrict__ lists,
+                                                              int *__restrict__ task_group) {
     const int lane = lane_id();
+    const int *toff = offs + 2 * ngroups;
+    const int tbase = toff[0];
     for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < ngroups;
-         g += (gridDim.x * blockDim.x) >> 5)
+         g += (gridDim.x * blockDim.x) >> 5) {
         for (int k = 0; k < 2; ++k) {
             const int n = counts[k * ngroups + g];
             const int2 *src = scratch + sstart[k * ngroups + g];
             int2 *dst = lists + offs[k * ngroups + g];
             for (int i = lane; i < n; i += 32) dst[i] = src[i];
         }
+        for (int t = toff[g] + lane; t < toff[g + 1]; t += 32) task_group[t - tbase] = g;
+    }
 }
 
 constexpr int PE_WARPS = 4;
@@ -878,7 +884,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
         (rc = ensure(c, S_POFF, (size_t)3 * ngroups + 1, &offs)))
         return rc;
     const TNode *tnode = slot_ptr<TNode>(c, S_TNODE);
-    unsigned *err = slot_ptr<unsigned>(c, S_ERR);
+    unsigned *err = c.ctrl.err;
     const int grid = (int)std::min<long long>((ngroups + PT_WARPS - 1) / PT_WARPS,
                                               (long long)sm_count_p() * 16);
     int *ko, *vo;
@@ -890,8 +896,8 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
     const int seg = task_segment(ngroups, c.precision == 1);
     ScratchLayout sl;
     ListScratch ls;   // released (when transient) after the copy, in stream order
-    int *sstart, *meta;
-    unsigned long long *stats = slot_ptr<unsigned long long>(c, S_STATS);
+    int *sstart, *meta = c.ctrl.meta;
+    unsigned long long *stats = c.ctrl.stats;
     TC_CUDA_TRY(cudaEventRecord(c.ev_fork, c.stream));
     {
         AuxScope on_aux(c);
@@ -901,20 +907,15 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
                                    &ko, &vo)))
             return rc;
         if ((rc = list_scratch(c, 2, nwarps, ngroups, sizeof(int2), sl, ls)) ||
-            (rc = ensure(c, S_LSTART, (size_t)2 * ngroups, &sstart)) ||
-            (rc = ensure(c, S_LMETA, 4, &meta)))
+            (rc = ensure(c, S_LSTART, (size_t)2 * ngroups, &sstart)))
             return rc;
-        TC_CUDA_TRY(cudaMemsetAsync(meta, 0, sizeof(int) * 4, c.stream));
         k_potential_lists<2><<<grid, PT_WARPS * 32, 0, c.stream>>>(
             ngroups, m, xt, yt, vo, theta, tnode, c.nnodes, counts, nullptr, nullptr,
             static_cast<int2 *>(ls.p), sl, sstart, meta, err, stats, seg);
         TC_KERNEL_CHECK();
-        if ((rc = exclusive_scan(c, counts, offs, 3 * ngroups))) return rc;
-        for (int k = 0; k < 3; ++k)
-            TC_CUDA_TRY(cudaMemcpyAsync(c.h_pinned + 32 + k, offs + (k + 1) * ngroups, sizeof(int),
-                                        cudaMemcpyDeviceToHost, c.stream));
-        TC_CUDA_TRY(cudaMemcpyAsync(c.h_pinned + 36, meta, sizeof(int) * 4,
-                                    cudaMemcpyDeviceToHost, c.stream));
+        // the lists' totals and meta, written to h_pinned by the scan
+        if ((rc = exclusive_scan(c, counts, offs, 3 * ngroups, ngroups, c.h_pinned + 32, meta)))
+            return rc;
         TC_CUDA_TRY(cudaEventRecord(c.ev_totals, c.stream));
     }
     if (between && (rc = between(c))) {
@@ -924,23 +925,27 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
     TC_CUDA_TRY(wait_event(c, c.ev_totals));
     const int n_e2p = (int)c.h_pinned[32], total = (int)c.h_pinned[33];
     const int ntasks = (int)c.h_pinned[34] - total;
-    const bool overflow = c.h_pinned[36] != 0;
+    const bool overflow = c.h_pinned[35] != 0;
     c.list_walks = overflow ? 2 : 1;
-    scratch_learn(c, 2, nwarps, ngroups, c.h_pinned + 37);   // for the next solve
+    scratch_learn(c, 2, nwarps, ngroups, c.h_pinned + 36);   // for the next solve
     c.counts.n_e2p = n_e2p;
     c.counts.n_p2p = total - n_e2p;
     c.counts.n_e2l = 0;
     c.counts.e2l_pairs = 0;
     c.counts.l2p_targets = 0;
     int2 *lists;
+    int *task_group;
     {
         AuxScope on_aux(c);
-        if ((rc = ensure(c, S_PE2P, (size_t)total + 1, &lists))) return rc;
+        if ((rc = ensure(c, S_PE2P, (size_t)total + 1, &lists)) ||
+            (rc = ensure(c, S_TASKMAP, (size_t)ntasks, &task_group)))
+            return rc;
         if (!overflow) {
             k_potential_lists_copy<<<(int)std::min<long long>((ngroups + 7) / 8,
                                                               (long long)sm_count_p() * 16),
                                      256, 0, c.stream>>>(ngroups, counts, offs, sstart,
-                                                         static_cast<const int2 *>(ls.p), lists);
+                                                         static_cast<const int2 *>(ls.p), lists,
+                                                         task_group);
         } else {
             // the second walk adds the work counters again: clear the first walk's
             TC_CUDA_TRY(cudaMemsetAsync(stats + STAT_E2P_PAIRS, 0, 2 * sizeof(unsigned long long),
@@ -948,22 +953,19 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
             k_potential_lists<1><<<grid, PT_WARPS * 32, 0, c.stream>>>(
                 ngroups, m, xt, yt, vo, theta, tnode, c.nnodes, nullptr, offs, lists, nullptr,
                 sl, nullptr, nullptr, err, stats, seg);
+            TC_KERNEL_CHECK();
+            k_task_map_groups<<<(int)std::min<long long>((ngroups + 255) / 256,
+                                                         (long long)sm_count_p() * 8),
+                                256, 0, c.stream>>>(ngroups, offs, task_group);
         }
         TC_KERNEL_CHECK();
         TC_CUDA_TRY(cudaEventRecord(c.ev_join, c.stream));
     }
     TC_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.ev_join, 0));
     phase_mark(c, 4);
-    int *task_ctr, *task_group;
+    int *task_ctr = c.ctrl.near_ctr;   // (cleared at the solve's start)
     double *partial;
-    if ((rc = ensure(c, S_BRICK_CTR, 4, &task_ctr)) ||
-        (rc = ensure(c, S_TASKMAP, (size_t)ntasks, &task_group)) ||
-        (rc = ensure(c, S_FPART, (size_t)ntasks * 32, &partial)))
-        return rc;
-    TC_CUDA_TRY(cudaMemsetAsync(task_ctr, 0, sizeof(int), c.stream));
-    k_task_map_groups<<<(int)std::min<long long>((ngroups + 255) / 256, (long long)sm_count_p() * 8),
-                        256, 0, c.stream>>>(ngroups, offs, task_group);
-    TC_KERNEL_CHECK();
+    if ((rc = ensure(c, S_FPART, (size_t)ntasks * 32, &partial))) return rc;
     // the evaluation for the tree's expansion order
     rc = dispatch_order(c.order, [&](auto order) -> int {
         constexpr int P = decltype(order)::value;

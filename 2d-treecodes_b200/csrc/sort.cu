@@ -791,24 +791,16 @@ int radix_sort_pairs(Context &c, const int *keys_in, const int *vals_in, int n, 
     }
     const int npasses = (nbits + 7) / 8;
     const int ntiles = (n + RS_TILE - 1) / RS_TILE;
-    int *hist, *counter;
-    unsigned *status;
-    int rc;
-    if ((rc = ensure(c, S_RS_HIST, 2 * RS_MAX_PASSES * RS_RADIX, &hist))) return rc;
-    if ((rc = ensure(c, S_RS_COUNTER, RS_MAX_PASSES, &counter))) return rc;
-    if ((rc = ensure(c, S_RS_STATUS, (size_t)RS_MAX_PASSES * ntiles * RS_RADIX, &status))) return rc;
-    int *offsets = hist + RS_MAX_PASSES * RS_RADIX;
-    TC_CUDA_TRY(cudaMemsetAsync(hist, 0, sizeof(int) * RS_MAX_PASSES * RS_RADIX, c.stream));
-    TC_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(int) * RS_MAX_PASSES, c.stream));
-    TC_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(unsigned) * (size_t)npasses * ntiles * RS_RADIX,
-                                c.stream));
-    k_hist<<<grid_for(n, 256, 4), 256, 0, c.stream>>>(keys_in, n, npasses, hist);
+    int *hist = c.ctrl.t_hist, *counter = c.ctrl.t_tile_ctr, *offsets = c.ctrl.t_offsets;
+    unsigned *status = c.ctrl.t_status;   // (cleared at the solve's start)
+    // the kernels follow each other, and the keys' kernel, directly (launch_pdl)
+    TC_CUDA_TRY(launch_pdl(ovl, k_hist, grid_for(n, 256, 4), 256, 0, c.stream, keys_in, n, npasses,
+                           hist));
     TC_KERNEL_CHECK();
-    // the kernels after k_hist follow each other directly (launch_pdl)
     TC_CUDA_TRY(launch_pdl(ovl, k_hist_scan, npasses, RS_RADIX, 0, c.stream, (const int *)hist,
                            offsets));
     TC_KERNEL_CHECK();
-    unsigned *err = slot_ptr<unsigned>(c, S_ERR);
+    unsigned *err = c.ctrl.err;
 
     const int *ki = keys_in, *vi = vals_in;
     int *ko = keys_a, *vo = vals_a;
@@ -846,7 +838,9 @@ __global__ __launch_bounds__(SCAN_THREADS) void k_scan_reduce(const int *__restr
 }
 
 __global__ __launch_bounds__(SCAN_THREADS) void k_scan_blocks(int *block_sums, int nb,
-                                                             int *out_total) {
+                                                             int *out_total, int nparts,
+                                                             volatile unsigned *host,
+                                                             const int *meta) {
     pdl_begin();
     // one CTA: each thread scans a contiguous chunk of the block sums
     const int per = (nb + SCAN_THREADS - 1) / SCAN_THREADS;
@@ -862,12 +856,17 @@ __global__ __launch_bounds__(SCAN_THREADS) void k_scan_blocks(int *block_sums, i
             block_sums[b0 + i] = run;
             run += v;
         }
-    if (threadIdx.x == 0) *out_total = total;
+    if (threadIdx.x == 0) {
+        *out_total = total;
+        if (host) host[nparts - 1] = (unsigned)total;
+    }
+    if (host && threadIdx.x < 4) host[nparts + threadIdx.x] = (unsigned)meta[threadIdx.x];
 }
 
 __global__ __launch_bounds__(SCAN_THREADS) void k_scan_apply(const int *__restrict__ in, int n,
                                                             const int *__restrict__ block_offs,
-                                                            int *__restrict__ out) {
+                                                            int *__restrict__ out, int part,
+                                                            volatile unsigned *host) {
     pdl_begin();
     const int base = blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_ITEMS;
     int v[SCAN_ITEMS];
@@ -882,12 +881,58 @@ __global__ __launch_bounds__(SCAN_THREADS) void k_scan_apply(const int *__restri
     for (int i = 0; i < SCAN_ITEMS; ++i)
         if (base + i < n) {
             out[base + i] = run;
+            if (host && base + i > 0 && (base + i) % part == 0)
+                host[(base + i) / part - 1] = (unsigned)run;
             run += v[i];
         }
 }
 
-int exclusive_scan(Context &c, const int *d_in, int *d_out, int n) {
+// The whole scan in one block, a tile after another, for short inputs: a tile takes about 2 us,
+// the three launches about 8.
+constexpr int SCAN_SMALL = 4 * SCAN_TILE;
+
+__global__ __launch_bounds__(SCAN_THREADS) void k_scan_small(const int *__restrict__ in, int n,
+                                                            int *__restrict__ out, int part,
+                                                            volatile unsigned *host,
+                                                            const int *meta) {
+    pdl_begin();
+    int carry = 0;
+    for (int t0 = 0; t0 < n; t0 += SCAN_TILE) {
+        const int base = t0 + threadIdx.x * SCAN_ITEMS;
+        int v[SCAN_ITEMS];
+        int s = 0, total;
+#pragma unroll
+        for (int i = 0; i < SCAN_ITEMS; ++i) {
+            v[i] = base + i < n ? in[base + i] : 0;
+            s += v[i];
+        }
+        int run = carry + block_exclusive_scan(s, &total);
+#pragma unroll
+        for (int i = 0; i < SCAN_ITEMS; ++i)
+            if (base + i < n) {
+                out[base + i] = run;
+                if (host && base + i > 0 && (base + i) % part == 0)
+                    host[(base + i) / part - 1] = (unsigned)run;
+                run += v[i];
+            }
+        carry += total;
+    }
+    if (threadIdx.x == 0) {
+        out[n] = carry;
+        if (host) host[n / part - 1] = (unsigned)carry;
+    }
+    if (host && threadIdx.x < 4) host[n / part + threadIdx.x] = (unsigned)meta[threadIdx.x];
+}
+
+int exclusive_scan(Context &c, const int *d_in, int *d_out, int n, int part, unsigned *host,
+                   const int *meta) {
     const bool ovl = c.launch_overlap;   // launch_pdl chains (tc_set_launch_overlap)
+    if (n > 0 && n <= SCAN_SMALL) {
+        TC_CUDA_TRY(launch_pdl(ovl, k_scan_small, 1, SCAN_THREADS, 0, c.stream, d_in, n, d_out,
+                               part, (volatile unsigned *)host, meta));
+        TC_KERNEL_CHECK();
+        return TC_OK;
+    }
     const int nb = (n + SCAN_TILE - 1) / SCAN_TILE;
     int *bs;
     int rc;
@@ -896,17 +941,63 @@ int exclusive_scan(Context &c, const int *d_in, int *d_out, int n) {
         TC_CUDA_TRY(cudaMemsetAsync(d_out, 0, sizeof(int), c.stream));
         return TC_OK;
     }
-    k_scan_reduce<<<nb, SCAN_THREADS, 0, c.stream>>>(d_in, n, bs);
+    TC_CUDA_TRY(launch_pdl(ovl, k_scan_reduce, nb, SCAN_THREADS, 0, c.stream, d_in, n, bs));
     TC_KERNEL_CHECK();
-    TC_CUDA_TRY(launch_pdl(ovl, k_scan_blocks, 1, SCAN_THREADS, 0, c.stream, bs, nb, d_out + n));
+    TC_CUDA_TRY(launch_pdl(ovl, k_scan_blocks, 1, SCAN_THREADS, 0, c.stream, bs, nb, d_out + n,
+                           part > 0 ? n / part : 0, (volatile unsigned *)host, meta));
     TC_KERNEL_CHECK();
     TC_CUDA_TRY(launch_pdl(ovl, k_scan_apply, nb, SCAN_THREADS, 0, c.stream, d_in, n,
-                           (const int *)bs, d_out));
+                           (const int *)bs, d_out, part, (volatile unsigned *)host));
     TC_KERNEL_CHECK();
     return TC_OK;
 }
 
 // ---------------------------------------------------------------------------- drivers
+// histograms and their scans: the four radix digits, then the buckets of the records
+constexpr int NHIST = RS_MAX_PASSES + 1;
+
+int ctrl_prepare(Context &c, int n, int m) {
+    const size_t words_s = (size_t)RS_MAX_PASSES * ((n + PS_TILE - 1) / PS_TILE) * RS_RADIX;
+    const size_t words_t = (size_t)RS_MAX_PASSES * ((m + RS_TILE - 1) / RS_TILE) * RS_RADIX;
+    const size_t words_l = tree_list_tiles(n);
+    unsigned *base = nullptr;
+    Ctrl k = {};
+    size_t total = 0, cleared = 0;
+    for (int pass = 0; pass < 2; ++pass) {   // sizes, then pointers
+        size_t at = 0;
+        auto take = [&](auto *&p, size_t words) {
+            p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + at);
+            at += (words + 3) & ~(size_t)3;   // 16-byte steps
+        };
+        take(k.err, 16);
+        take(k.stats, 2 * STAT_SLOTS);
+        take(k.bbox_done, 1);
+        take(k.tile_ctr, RS_MAX_PASSES);
+        take(k.bucket_fill, NB_BUCKETS);
+        take(k.nlist, 1);
+        take(k.tl_ctr, 1);
+        take(k.meta, 4);
+        take(k.near_ctr, 1);
+        take(k.far_ctr, FORCE_CHUNKS);
+        take(k.t_tile_ctr, RS_MAX_PASSES);
+        take(k.hist, NHIST * RS_RADIX);
+        take(k.t_hist, RS_MAX_PASSES * RS_RADIX);
+        take(k.tl_status, words_l);
+        take(k.status, words_s);
+        take(k.t_status, words_t);
+        cleared = at;
+        take(k.offsets, NHIST * RS_RADIX);
+        take(k.t_offsets, RS_MAX_PASSES * RS_RADIX);
+        take(k.sink, RS_RADIX);
+        total = at;
+        if (pass == 0)
+            if (int rc = ensure(c, S_CTRL, total, &base)) return rc;
+    }
+    c.ctrl = k;
+    TC_CUDA_TRY(cudaMemsetAsync(base, 0, cleared * sizeof(unsigned), c.stream));
+    return TC_OK;
+}
+
 int sort_sources(Context &c, const double *x, const double *y, const double *v, int n,
                  cudaEvent_t values_ready) {
     const bool ovl = c.launch_overlap;   // launch_pdl chains (tc_set_launch_overlap)
@@ -920,12 +1011,12 @@ int sort_sources(Context &c, const double *x, const double *y, const double *v, 
         (rc = ensure(c, S_VS, n, &vs)) || (rc = ensure(c, S_KEYS, n, &keys)) ||
         (rc = ensure(c, S_PERM, n, &perm)))
         return rc;
-    // frame + bbox partials + completion counter share one small buffer
+    // frame and bbox partials share one small buffer
     const int gb = grid_for(n, BBOX_THREADS, 8);
-    if ((rc = ensure(c, S_FRAME, sizeof(Frame) + sizeof(double4) * (gb + 1) + 64, (char **)&frame)))
+    if ((rc = ensure(c, S_FRAME, sizeof(Frame) + sizeof(double4) * gb + 64, (char **)&frame)))
         return rc;
     partials = reinterpret_cast<double4 *>(reinterpret_cast<char *>(frame) + 64);
-    unsigned *done = reinterpret_cast<unsigned *>(partials + gb);
+    unsigned *done = c.ctrl.bbox_done;
 
     // four 8-bit passes over the (key, index) items, then one gather of the records
     if (n >= (1 << 30)) {
@@ -934,28 +1025,16 @@ int sort_sources(Context &c, const double *x, const double *y, const double *v, 
     }
     unsigned long long *items_a, *items_b;
     double2 *rec;
-    int *hist, *counter;
-    unsigned *status;
     const int npasses = (2 * LMAX + 7) / 8;
     const int ntiles = (n + PS_TILE - 1) / PS_TILE;
-    // histograms and their scans: the four radix digits, then the buckets of the records
-    constexpr int NHIST = RS_MAX_PASSES + 1;
     if ((rc = ensure(c, S_ITEMS_A, n, &items_a)) || (rc = ensure(c, S_ITEMS_B, n, &items_b)) ||
-        (rc = ensure(c, S_REC, 2 * (size_t)n, &rec)) ||
-        (rc = ensure(c, S_RS_HIST, 2 * NHIST * RS_RADIX, &hist)) ||
-        (rc = ensure(c, S_RS_COUNTER, RS_MAX_PASSES + NB_BUCKETS, &counter)) ||
-        (rc = ensure(c, S_RS_STATUS, ((size_t)RS_MAX_PASSES * ntiles + 1) * RS_RADIX, &status)))
+        (rc = ensure(c, S_REC, 2 * (size_t)n, &rec)))
         return rc;
-    int *offsets = hist + NHIST * RS_RADIX;
-    unsigned *sink = status + (size_t)RS_MAX_PASSES * ntiles * RS_RADIX;   // after every pass
-    int *bucket_fill = counter + RS_MAX_PASSES;
-    // every buffer and counter first, so that the sort's kernels follow each other directly on
-    // the stream (each may then be scheduled while the one before it drains, launch_pdl)
-    TC_CUDA_TRY(cudaMemsetAsync(done, 0, sizeof(unsigned), c.stream));
-    TC_CUDA_TRY(cudaMemsetAsync(hist, 0, sizeof(int) * NHIST * RS_RADIX, c.stream));
-    TC_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(int) * (RS_MAX_PASSES + NB_BUCKETS), c.stream));
-    TC_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(unsigned) * (size_t)npasses * ntiles * RS_RADIX,
-                                c.stream));
+    // every counter is cleared at the solve's start (ctrl_prepare), so that the sort's kernels
+    // follow each other directly on the stream (launch_pdl)
+    int *hist = c.ctrl.hist, *offsets = c.ctrl.offsets, *counter = c.ctrl.tile_ctr;
+    int *bucket_fill = c.ctrl.bucket_fill;
+    unsigned *status = c.ctrl.status, *sink = c.ctrl.sink;
     k_bbox<<<gb, BBOX_THREADS, 0, c.stream>>>(x, y, n, partials, done, frame);
     TC_KERNEL_CHECK();
     // resident values: the records are written by the first pass, in buckets (see FirstPass);
@@ -972,7 +1051,7 @@ int sort_sources(Context &c, const double *x, const double *y, const double *v, 
     TC_CUDA_TRY(launch_pdl(ovl, k_hist_scan, NHIST, RS_RADIX, 0, c.stream, (const int *)hist,
                            offsets));
     TC_KERNEL_CHECK();
-    unsigned *err = slot_ptr<unsigned>(c, S_ERR);
+    unsigned *err = c.ctrl.err;
     const FirstPass fp = {x, y, v, frame, rec, offsets + RS_MAX_PASSES * RS_RADIX, bucket_fill};
     static_assert((2 * LMAX + 7) / 8 % 2 == 0, "an even number of passes ends in items_a");
     for (int p = 0; p < npasses; ++p) {
@@ -1021,7 +1100,7 @@ int finish_sources(Context &c) {
     k_gather_xy<<<grid_for(n, 256, 8), 256, 0, c.stream>>>(perm, c.late_x, c.late_y, n,
                                                           slot_ptr<double>(c, S_XS),
                                                           slot_ptr<double>(c, S_YS),
-                                                          slot_ptr<unsigned>(c, S_ERR));
+                                                          c.ctrl.err);
     TC_KERNEL_CHECK();
     TC_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.late_ready, 0));
     c.late_ready = nullptr;
@@ -1097,7 +1176,7 @@ void kernels_sort(KernelList &v) {
                        (const void *)k_gather_sources, (const void *)k_gather_xy,
                        (const void *)k_gather_v, (const void *)k_items_split,
                        (const void *)k_scan_reduce, (const void *)k_scan_blocks,
-                       (const void *)k_scan_apply});
+                       (const void *)k_scan_apply, (const void *)k_scan_small});
 }
 
 }  // namespace tc

@@ -26,21 +26,19 @@ enum Slot {
     S_XIN, S_YIN, S_VIN, S_XT, S_YT, S_X0, S_Y0, S_H, S_OUTX, S_OUTY,
     // sorted sources
     S_XS, S_YS, S_VS, S_KEYS, S_PERM, S_FRAME, S_ITEMS_A, S_ITEMS_B, S_REC,
-    // radix sort scratch
-    S_RS_STATUS, S_RS_HIST, S_RS_COUNTER,
+    // the solve's counters, histograms and look-back words (Ctrl)
+    S_CTRL,
     // scan scratch
     S_SCAN_BLOCKS,
     // tree build
-    S_TMASK, S_TFLAG, S_TOFF, S_LPOS, S_LMASK, S_LRANK, S_LINV, S_LBLK, S_LEVEL_TOTALS,
+    S_LPOS, S_LMASK, S_LRANK, S_LINV, S_LBLK,
     // nodes
     S_TNODE, S_RANGE, S_CELL, S_MASS, S_W, S_WX, S_WY, S_EXPS, S_UPCNT,
     // force traversal / lists
-    S_FCOUNT, S_FOFF, S_E2L, S_E2P, S_P2P, S_BRICK_CTR, S_FPART, S_SEXP, S_SSCALE, S_TASKMAP,
-    S_LSTART, S_LMETA, S_FARX, S_FARY, S_FAR_CTR,
+    S_FCOUNT, S_FOFF, S_E2L, S_FPART, S_SEXP, S_SSCALE, S_TASKMAP,
+    S_LSTART, S_FARX, S_FARY,
     // potential targets / lists
-    S_TKEYS, S_TPERM, S_TKEYS2, S_TPERM2, S_PCOUNT, S_POFF, S_PE2P, S_PP2P,
-    // misc
-    S_ERR, S_STATS,
+    S_TKEYS, S_TPERM, S_TKEYS2, S_TPERM2, S_PCOUNT, S_POFF, S_PE2P,
     S_NUM_SLOTS
 };
 
@@ -64,7 +62,7 @@ struct Counts {
     long long launches;                   // kernels launched by the last solve
 };
 
-// Device-side work counters (unsigned long long each) in the S_STATS slot.
+// Device-side work counters (unsigned long long each), Ctrl::stats.
 enum { STAT_P2P_SOURCES = 0, STAT_E2P_PAIRS = 1, STAT_P2P_PAIRS = 2, STAT_SLOTS = 8 };
 
 // Expansion orders a context can be set to (tc_set_orders).  The reference fixes its orders at
@@ -95,7 +93,31 @@ struct ScratchLayout {
     int koff[3];
 };
 
+// Runs of blocks whose force outputs are copied to the host while the next run is evaluated.
+constexpr int FORCE_CHUNKS = 4;
+
+// Everything a solve needs zeroed, in one buffer that one memset at its start clears: on a small
+// solve a memset costs as much as a short kernel, and twelve of them took about a tenth of it.
+// The scanned histograms and the test sink lie behind the cleared part.
+struct Ctrl {
+    unsigned *err;                // device error word
+    unsigned long long *stats;    // work counters (STAT_*), read back with err in one copy
+    unsigned *bbox_done;
+    int *tile_ctr, *bucket_fill;  // source sort: tiles taken per pass, record slots claimed
+    int *nlist, *tl_ctr;          // tree: split-list length, tiles taken
+    int *meta;                    // list build: overflow flag, longest runs
+    int *near_ctr, *far_ctr;      // evaluation tasks / far-field bricks taken
+    int *t_tile_ctr;              // target sort
+    int *hist, *t_hist;           // digit histograms of the source and the target sort
+    unsigned *status, *t_status, *tl_status;   // look-back words: sorts, tree list
+    int *offsets, *t_offsets;     // scanned histograms
+    unsigned *sink;               // look-back words of a stalled test tile
+};
+
 struct Context;
+// Lays the buffer out for a solve of n sources and m potential targets and clears it, on the
+// context's current stream.
+int ctrl_prepare(Context &c, int n, int m);
 // Regions for `nkinds` kinds, `nwarps` warps and `nitems` bricks / groups, from the context's
 // learned sizes, at most `max_entries` entries in all (smaller regions when they do not fit);
 // returns the entries used.
@@ -130,7 +152,7 @@ struct Context {
     // host entry points: x/y are copied on `stream`, v (and targets) on `aux` after them;
     // ev_inputs marks v's arrival
     cudaEvent_t ev_inputs = nullptr;
-    cudaEvent_t ev_chunk[4] = {};        // force output runs ready for their host copy
+    cudaEvent_t ev_chunk[FORCE_CHUNKS] = {};        // force output runs ready for their host copy
     cudaEvent_t ev_leafset = nullptr;     // leaf moments written (main stream)
     cudaEvent_t ev_moments = nullptr;     // parent moments written (auxiliary stream)
     cudaEvent_t ev_near = nullptr;        // force near field written (auxiliary stream)
@@ -140,6 +162,7 @@ struct Context {
     const double *late_x = nullptr, *late_y = nullptr, *late_v = nullptr;
     cudaEvent_t late_ready = nullptr;
     DevBuf buf[S_NUM_SLOTS];
+    Ctrl ctrl = {};
     unsigned *h_pinned = nullptr;         // small pinned staging area for readbacks
     int precision = 0;                    // 0 = plain FP64, 1 = mixed
     int order_potential = ORDER_POTENTIAL;  // expansion orders of the next solves
@@ -248,7 +271,10 @@ int blocks_per_sm(int threads, size_t smem) {
 }
 
 // ---- sort.cu
-int exclusive_scan(Context &c, const int *d_in, int *d_out, int n);   // d_out has n+1 entries
+// d_out has n + 1 entries.  With `host` (page-locked), the scan also writes there the offsets at
+// the ends of the n / part parts of the input, then the four words at `meta`.
+int exclusive_scan(Context &c, const int *d_in, int *d_out, int n, int part = 0,
+                   unsigned *host = nullptr, const int *meta = nullptr);
 int radix_sort_pairs(Context &c, const int *keys_in, const int *vals_in, int n, int nbits,
                      int *keys_a, int *vals_a, int *keys_b, int *vals_b, int **keys_out,
                      int **vals_out);
@@ -263,6 +289,7 @@ int target_keys(Context &c, const double *xt, const double *yt, int m, int *keys
 
 // ---- tree.cu
 int build_topology(Context &c, int leafcap);
+int tree_list_tiles(int n);   // look-back words of the build
 
 // ---- upward.cu
 int upward_prepare(Context &c, int order);   // buffers of the upward pass, c.order

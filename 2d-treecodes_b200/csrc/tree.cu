@@ -63,6 +63,7 @@ constexpr int TL_ITEMS = 16;
 constexpr int TL_TILE = TL_THREADS * TL_ITEMS;
 constexpr int TL_HALO = LEAF_POTENTIAL;           // the largest leaf capacity
 constexpr int TL_STAGE = TL_TILE + 1 + TL_HALO;   // staged keys per tile
+int tree_list_tiles(int n) { return (n + TL_TILE - 1) / TL_TILE; }
 constexpr unsigned TL_AGG = 1u << 30, TL_INC = 2u << 30, TL_VAL = (1u << 30) - 1;
 // `stall_tile` (a test setting, -1 otherwise) names a tile that publishes nothing, so that the
 // tile after it waits until `spin_limit` and reports DEVERR_SPIN_LIMIT.
@@ -196,9 +197,11 @@ __global__ __launch_bounds__(RANK_THREADS) void k_rank_count(const unsigned shor
     if (threadIdx.x < LMAX) blk[threadIdx.x * nblk + blockIdx.x] = s_cnt[threadIdx.x];
 }
 
-// One CTA per level: exclusive scan over the blocks' counts; level total -> totals[l].
+// One CTA per level: exclusive scan over the blocks' counts; level total -> host[l], the list's
+// length -> host[LMAX] (page-locked host memory: no copy between the kernel and the host's wait).
 __global__ __launch_bounds__(1024) void k_rank_scan(int *__restrict__ blk, int nblk,
-                                                    int *__restrict__ totals) {
+                                                    const int *__restrict__ d_nlist,
+                                                    volatile unsigned *host) {
     pdl_begin();
     const int l = blockIdx.x;
     int *row = blk + (size_t)l * nblk;
@@ -208,7 +211,10 @@ __global__ __launch_bounds__(1024) void k_rank_scan(int *__restrict__ blk, int n
     for (int i = 0; i < per; ++i)
         if (b0 + i < nblk) s += row[b0 + i];
     int run = block_exclusive_scan(s, &total);
-    if (threadIdx.x == 0) totals[l] = total;
+    if (threadIdx.x == 0) {
+        host[l] = (unsigned)total;
+        if (l == 0) host[LMAX] = (unsigned)*d_nlist;
+    }
     for (int i = 0; i < per; ++i)
         if (b0 + i < nblk) {
             const int v = row[b0 + i];
@@ -266,7 +272,7 @@ __global__ __launch_bounds__(RANK_THREADS) void k_rank_small(const unsigned shor
                                                              const int *__restrict__ d_nlist,
                                                              int *__restrict__ rank,
                                                              int *__restrict__ inv, int stride,
-                                                             int *__restrict__ totals) {
+                                                             volatile unsigned *host) {
     pdl_begin();
     __shared__ int s_w[LMAX][RANK_THREADS / 32 + 1];
     __shared__ int s_run[LMAX];
@@ -308,7 +314,8 @@ __global__ __launch_bounds__(RANK_THREADS) void k_rank_small(const unsigned shor
         __syncthreads();
     }
     __syncthreads();
-    if (threadIdx.x < LMAX) totals[threadIdx.x] = s_run[threadIdx.x];
+    if (threadIdx.x < LMAX) host[threadIdx.x] = (unsigned)s_run[threadIdx.x];
+    if (threadIdx.x == LMAX) host[LMAX] = (unsigned)*d_nlist;
 }
 
 // The root of a tree without inner cells.
@@ -415,48 +422,41 @@ int build_topology(Context &c, int leafcap) {
     const int cap = (int)(bound < n ? bound : n);
     const int ntl = (n + TL_TILE - 1) / TL_TILE;
     const int nblk = (cap + RANK_THREADS - 1) / RANK_THREADS;
-    int *lpos, *rank, *rinv, *blkc, *totals, *tl_counter;
-    unsigned *tl_status;
+    int *lpos, *rank, *rinv, *blkc;
     unsigned short *lmask;
     if ((rc = ensure(c, S_LPOS, (size_t)cap + 1, &lpos)) ||
         (rc = ensure(c, S_LMASK, (size_t)cap + 1, &lmask)) ||
-        (rc = ensure(c, S_TFLAG, (size_t)ntl + 8, &tl_status)) ||
         (rc = ensure(c, S_LRANK, (size_t)LMAX * (cap + 1), &rank)) ||
         (rc = ensure(c, S_LINV, (size_t)LMAX * (cap + 1), &rinv)) ||
-        (rc = ensure(c, S_LBLK, (size_t)LMAX * (nblk + 1), &blkc)) ||
-        (rc = ensure(c, S_LEVEL_TOTALS, LMAX + 4, &totals)))
+        (rc = ensure(c, S_LBLK, (size_t)LMAX * (nblk + 1), &blkc)))
         return rc;
-    int *d_nlist = totals + LMAX;
-    tl_counter = totals + LMAX + 1;
-    TC_CUDA_TRY(cudaMemsetAsync(totals, 0, sizeof(int) * (LMAX + 4), c.stream));
-    TC_CUDA_TRY(cudaMemsetAsync(tl_status, 0, sizeof(unsigned) * ntl, c.stream));
-    unsigned *err = slot_ptr<unsigned>(c, S_ERR);
-    k_tree_list<<<ntl, TL_THREADS, 0, c.stream>>>(keys, n, leafcap, cap, tl_status, tl_counter,
-                                                   lpos, lmask, d_nlist, err, c.spin_limit,
-                                                   c.test_stall == TC_STALL_TREE ? 0 : -1);
+    int *d_nlist = c.ctrl.nlist;
+    unsigned *err = c.ctrl.err;
+    // the kernels of the build follow the sort's, and each other, directly (launch_pdl)
+    TC_CUDA_TRY(launch_pdl(ovl, k_tree_list, ntl, TL_THREADS, 0, c.stream, keys, n, leafcap, cap,
+                           c.ctrl.tl_status, c.ctrl.tl_ctr, lpos, lmask, d_nlist, err,
+                           c.spin_limit, c.test_stall == TC_STALL_TREE ? 0 : -1));
     TC_KERNEL_CHECK();
     // a test stall leaves the list offsets wrong: report it before anything reads them
     if (c.test_stall == TC_STALL_TREE && (rc = check_device_errors(c, "tree build"))) return rc;
-    // the rank kernels follow k_tree_list directly (launch_pdl)
     if (cap <= RANK_SMALL) {
         TC_CUDA_TRY(launch_pdl(ovl, k_rank_small, 1, RANK_THREADS, 0, c.stream,
                                (const unsigned short *)lmask, (const int *)d_nlist, rank, rinv, cap,
-                               totals));
+                               (volatile unsigned *)c.h_pinned));
         TC_KERNEL_CHECK();
     } else {
         TC_CUDA_TRY(launch_pdl(ovl, k_rank_count, nblk, RANK_THREADS, 0, c.stream,
                                (const unsigned short *)lmask, (const int *)d_nlist, blkc, nblk));
         TC_KERNEL_CHECK();
-        TC_CUDA_TRY(launch_pdl(ovl, k_rank_scan, LMAX, 1024, 0, c.stream, blkc, nblk, totals));
+        TC_CUDA_TRY(launch_pdl(ovl, k_rank_scan, LMAX, 1024, 0, c.stream, blkc, nblk,
+                               (const int *)d_nlist, (volatile unsigned *)c.h_pinned));
         TC_KERNEL_CHECK();
         TC_CUDA_TRY(launch_pdl(ovl, k_rank_apply, nblk, RANK_THREADS, 0, c.stream,
                                (const unsigned short *)lmask, (const int *)d_nlist, (const int *)blkc,
                                nblk, rank, rinv, cap));
         TC_KERNEL_CHECK();
     }
-    // the level totals and the list length, in one read-back
-    TC_CUDA_TRY(cudaMemcpyAsync(c.h_pinned, totals, sizeof(int) * (LMAX + 1),
-                                cudaMemcpyDeviceToHost, c.stream));
+    // the level totals and the list length are in h_pinned once the kernels are done
     TC_CUDA_TRY(wait_stream(c, c.stream));
     const int nlist = (int)c.h_pinned[LMAX];
     if (nlist > cap) {

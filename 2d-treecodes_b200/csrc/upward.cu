@@ -689,7 +689,7 @@ int upward_moments(Context &c) {
     const int4 *cell = slot_ptr<int4>(c, S_CELL);
     TNode *tnode = slot_ptr<TNode>(c, S_TNODE);
     const Frame *frame = slot_ptr<Frame>(c, S_FRAME);
-    unsigned *err = slot_ptr<unsigned>(c, S_ERR);
+    unsigned *err = c.ctrl.err;
     double *mass = slot_ptr<double>(c, S_MASS), *w = slot_ptr<double>(c, S_W),
            *wx = slot_ptr<double>(c, S_WX), *wy = slot_ptr<double>(c, S_WY);
     k_leaf_setup<<<(int)(((long long)nn * 4 + 255) / 256), 256, 0, c.stream>>>(
@@ -743,7 +743,7 @@ static int run_expansions(Context &c) {
     const int4 *cell = slot_ptr<int4>(c, S_CELL);
     const TNode *tnode = slot_ptr<TNode>(c, S_TNODE);
     const Frame *frame = slot_ptr<Frame>(c, S_FRAME);
-    unsigned *err = slot_ptr<unsigned>(c, S_ERR);
+    unsigned *err = c.ctrl.err;
     const double *mass = slot_ptr<double>(c, S_MASS), *w = slot_ptr<double>(c, S_W);
     double *exps = slot_ptr<double>(c, S_EXPS);
     const int sms = sm_count_up();
