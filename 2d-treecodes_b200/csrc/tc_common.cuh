@@ -60,9 +60,6 @@ constexpr int near_segment(int nbricks) {
     return seg;
 }
 
-// Runs of blocks whose outputs are copied to the host while the next run is evaluated.
-constexpr int FORCE_CHUNKS = 4;
-
 constexpr unsigned FULL_MASK = 0xffffffffu;
 
 // Reads without progress after which a device wait on another CTA's published state gives up
