@@ -873,10 +873,6 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
               OverlapFn between) {
     if (m == 0) return between ? between(c) : TC_OK;
     int rc;
-    int *tkeys, *tperm, *tkeys2, *tperm2;
-    if ((rc = ensure(c, S_TKEYS, m, &tkeys)) || (rc = ensure(c, S_TPERM, m, &tperm)) ||
-        (rc = ensure(c, S_TKEYS2, m, &tkeys2)) || (rc = ensure(c, S_TPERM2, m, &tperm2)))
-        return rc;
     const int ngroups = (m + 31) / 32;
     // counts / offsets: E2P | P2P list lengths and evaluation tasks, ngroups each
     int *counts, *offs;
@@ -887,7 +883,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
     unsigned *err = c.ctrl.err;
     const int grid = (int)std::min<long long>((ngroups + PT_WARPS - 1) / PT_WARPS,
                                               (long long)sm_count_p() * 16);
-    int *ko, *vo;
+    int *vo;
     // One walk counts the lists and writes them into per-warp scratch runs; after the scan a
     // copy puts them in CSR order.  If a run outgrew its region a second walk writes them
     // instead, and the regions are sized up for the next solve.  The runs live in the sort's
@@ -902,10 +898,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
     {
         AuxScope on_aux(c);
         TC_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.ev_fork, 0));
-        if ((rc = target_keys(c, xt, yt, m, tkeys, nullptr))) return rc;
-        if ((rc = radix_sort_pairs(c, tkeys, nullptr, m, 2 * LMAX, tkeys2, tperm2, tkeys, tperm,
-                                   &ko, &vo)))
-            return rc;
+        if ((rc = sort_targets(c, xt, yt, m, &vo))) return rc;
         if ((rc = list_scratch(c, 2, nwarps, ngroups, sizeof(int2), sl, ls)) ||
             (rc = ensure(c, S_LSTART, (size_t)2 * ngroups, &sstart)))
             return rc;

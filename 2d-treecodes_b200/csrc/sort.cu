@@ -44,6 +44,22 @@ __device__ __forceinline__ void warp_minmax(double &a, double &b, double &c, dou
     }
 }
 
+// The padded square of extrema (xmin, xmax, ymin, ymax): sort-sources.cpp:98-110, with the
+// arithmetic the compiled reference executes: ext = max(ex, ey) * (1 + 2 eps);
+// xmin -= eps * ext; keys use (1/ext) * 2^15.
+__device__ __forceinline__ Frame frame_of(const double4 &r) {
+    const double eps = 10000.0 * DBL_EPSILON;
+    const double ext0 = __dsub_rn(r.y, r.x);
+    const double ext1 = __dsub_rn(r.w, r.z);
+    const double ext = __dmul_rn(ext0 < ext1 ? ext1 : ext0, 1.0 + 2.0 * eps);
+    Frame f;
+    f.xmin = __dsub_rn(r.x, __dmul_rn(eps, ext));
+    f.ymin = __dsub_rn(r.z, __dmul_rn(eps, ext));
+    f.ext = ext;
+    f.scale = __dmul_rn(__ddiv_rn(1.0, ext), (double)(1 << LMAX));
+    return f;
+}
+
 // Per-CTA min/max, then the last CTA to finish reduces the partials and derives the frame.
 // Initial extrema follow upward-common.ispc:132 (min 1e13, max 0) and sort-sources.cpp:48.
 __global__ __launch_bounds__(BBOX_THREADS) void k_bbox(const double *__restrict__ x,
@@ -117,18 +133,7 @@ __global__ __launch_bounds__(BBOX_THREADS) void k_bbox(const double *__restrict_
             r.x = fmin(r.x, s[i].x); r.y = fmax(r.y, s[i].y);
             r.z = fmin(r.z, s[i].z); r.w = fmax(r.w, s[i].w);
         }
-        // sort-sources.cpp:98-110, with the arithmetic the compiled reference executes:
-        // ext = max(ex, ey) * (1 + 2 eps); xmin -= eps * ext; keys use (1/ext) * 2^15.
-        const double eps = 10000.0 * DBL_EPSILON;
-        const double ext0 = __dsub_rn(r.y, r.x);
-        const double ext1 = __dsub_rn(r.w, r.z);
-        const double ext = __dmul_rn(ext0 < ext1 ? ext1 : ext0, 1.0 + 2.0 * eps);
-        Frame f;
-        f.xmin = __dsub_rn(r.x, __dmul_rn(eps, ext));
-        f.ymin = __dsub_rn(r.z, __dmul_rn(eps, ext));
-        f.ext = ext;
-        f.scale = __dmul_rn(__ddiv_rn(1.0, ext), (double)(1 << LMAX));
-        *frame = f;
+        *frame = frame_of(r);
         *done = 0;
     }
 }
@@ -141,20 +146,23 @@ __device__ __forceinline__ int quantize(double v, double vmin, double scale) {
 
 // Target keys in the source frame, clamped to the quantisation range (targets may lie outside
 // the sources' square).  Used only to group nearby targets; it does not affect results.
+__device__ __forceinline__ int target_key(double x, double y, const Frame &f) {
+    const double hi = (double)((1 << LMAX) - 1);
+    double qx = floor((x - f.xmin) * f.scale);
+    double qy = floor((y - f.ymin) * f.scale);
+    qx = fmin(fmax(qx, 0.0), hi);
+    qy = fmin(fmax(qy, 0.0), hi);
+    if (qx != qx) qx = 0;
+    if (qy != qy) qy = 0;
+    return spread_bits((int)qx) | (spread_bits((int)qy) << 1);
+}
+
 __global__ void k_target_keys(const double *__restrict__ x, const double *__restrict__ y, int n,
                               const Frame *__restrict__ frame, int *__restrict__ keys) {
     pdl_begin();
     const Frame f = *frame;
-    const double hi = (double)((1 << LMAX) - 1);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double qx = floor((x[i] - f.xmin) * f.scale);
-        double qy = floor((y[i] - f.ymin) * f.scale);
-        qx = fmin(fmax(qx, 0.0), hi);
-        qy = fmin(fmax(qy, 0.0), hi);
-        if (qx != qx) qx = 0;
-        if (qy != qy) qy = 0;
-        keys[i] = spread_bits((int)qx) | (spread_bits((int)qy) << 1);
-    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        keys[i] = target_key(x[i], y[i], f);
 }
 
 // ---------------------------------------------------------------------------- radix sort
@@ -770,6 +778,177 @@ __global__ __launch_bounds__(256) void k_gather_items_inplace(
     }
 }
 
+// ---------------------------------------------------------------------------- small sorts
+// Up to SMALL_SORT sources (or targets) are sorted by one block, in one launch: bounding square,
+// keys, an LSD radix sort of the items (key << 32 | index) held in shared memory, and the
+// gather.  It is bound by the latency of its phases, about 6 us for 4096 items and 15 us for
+// 16,384, where the eight launches of the general sort take 65 us whatever the size; past 16K
+// items (128 KB of shared memory) one SM would be the slower one.  Same keys, order and values:
+// ties keep input order in both.
+constexpr int SMALL_THREADS = 1024;
+constexpr int SMALL_WARPS = SMALL_THREADS / 32;
+constexpr int SMALL_SORT = 16 * SMALL_THREADS;
+constexpr int SMALL_ROW = RS_RADIX + 1;   // padded: a digit's 32 warp counts in distinct banks
+
+template <int ITEMS>
+constexpr size_t small_smem() {
+    return sizeof(unsigned long long) * SMALL_THREADS * ITEMS + sizeof(int) * SMALL_WARPS * SMALL_ROW;
+}
+
+// Sorts the block's items by their upper 32 bits; warp w holds items [w, w + 1) * 32 ITEMS of the
+// input order in `item`; the sorted items are left in s_items.
+template <int ITEMS>
+__device__ __forceinline__ void block_sort_items(unsigned long long (&item)[ITEMS],
+                                                 unsigned long long *s_items, int *s_hist) {
+    __shared__ int s_total[RS_RADIX];
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    const int first = warp * 32 * ITEMS + lane;
+    const unsigned lt = lanemask_lt();
+    int *hist = s_hist + warp * SMALL_ROW;
+    for (int shift = 32; shift < 64; shift += 8) {
+        if (shift > 32)
+#pragma unroll
+            for (int k = 0; k < ITEMS; ++k) item[k] = s_items[first + 32 * k];
+        for (int i = lane; i < RS_RADIX; i += 32) hist[i] = 0;
+        __syncwarp();
+        int rank[ITEMS];
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const int d = (int)(item[k] >> shift) & 0xFF;
+            const unsigned peers = digit_peers(FULL_MASK, d);
+            const int old = hist[d];
+            __syncwarp();
+            if ((peers & lt) == 0) hist[d] = old + __popc(peers);
+            __syncwarp();
+            rank[k] = old + __popc(peers & lt);
+        }
+        __syncthreads();   // (also: every item has been read)
+        // each warp scans the warp counts of 8 digits, lane = warp
+#pragma unroll
+        for (int q = 0; q < RS_RADIX / SMALL_WARPS; ++q) {
+            const int d = warp * (RS_RADIX / SMALL_WARPS) + q;
+            const int v = s_hist[lane * SMALL_ROW + d];
+            int inc = v;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(FULL_MASK, inc, o);
+                if (lane >= o) inc += t;
+            }
+            s_hist[lane * SMALL_ROW + d] = inc - v;
+            if (lane == 31) s_total[d] = inc;
+        }
+        __syncthreads();
+        const int tot = threadIdx.x < RS_RADIX ? s_total[threadIdx.x] : 0;
+        const int start = block_exclusive_scan(tot, nullptr);
+        if (threadIdx.x < RS_RADIX) s_total[threadIdx.x] = start;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const int d = (int)(item[k] >> shift) & 0xFF;
+            s_items[s_total[d] + hist[d] + rank[k]] = item[k];
+        }
+        __syncthreads();
+    }
+}
+
+// Sources: frame, sorted keys, permutation, x and y, and v where it is there (null: late values).
+template <int ITEMS>
+__global__ __launch_bounds__(SMALL_THREADS) void k_sort_small(
+    const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ v, int n,
+    Frame *frame, int *__restrict__ keys, int *__restrict__ perm, double *__restrict__ xs,
+    double *__restrict__ ys, double *__restrict__ vs) {
+    extern __shared__ __align__(16) unsigned long long small_dyn[];
+    unsigned long long *s_items = small_dyn;
+    int *s_hist = reinterpret_cast<int *>(s_items + SMALL_THREADS * ITEMS);
+    __shared__ double4 s_ext[SMALL_WARPS];
+    __shared__ Frame s_frame;
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    // extrema as k_bbox
+    double xmi = 1e13, xma = 0, ymi = 1e13, yma = 0;
+    for (int i = threadIdx.x; i < n; i += SMALL_THREADS) {
+        const double xv = x[i], yv = y[i];
+        xmi = fmin(xmi, xv);
+        xma = fmax(xma, xv);
+        ymi = fmin(ymi, yv);
+        yma = fmax(yma, yv);
+    }
+    warp_minmax(xmi, xma, ymi, yma);
+    if (lane == 0) s_ext[warp] = make_double4(xmi, xma, ymi, yma);
+    __syncthreads();
+    if (warp == 0) {
+        const double4 r = s_ext[lane];
+        xmi = r.x; xma = r.y; ymi = r.z; yma = r.w;
+        warp_minmax(xmi, xma, ymi, yma);
+        if (lane == 0) *frame = s_frame = frame_of(make_double4(xmi, xma, ymi, yma));
+    }
+    __syncthreads();
+    const Frame f = s_frame;
+    unsigned long long item[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const int i = warp * 32 * ITEMS + 32 * k + lane;
+        // past the end: after every key, and after equal ones (they come last in input order)
+        unsigned key = 0xffffffffu;
+        if (i < n) key = (unsigned)morton_key(x[i], y[i], f);
+        item[k] = ((unsigned long long)key << 32) | (unsigned)i;
+    }
+    block_sort_items<ITEMS>(item, s_items, s_hist);
+    for (int i = threadIdx.x; i < n; i += SMALL_THREADS) {
+        const unsigned long long it = s_items[i];
+        const unsigned j = (unsigned)it;
+        keys[i] = (int)(it >> 32);
+        perm[i] = (int)j;
+        xs[i] = x[j];
+        ys[i] = y[j];
+        if (v) vs[i] = v[j];
+    }
+}
+
+// Targets: the permutation alone.
+template <int ITEMS>
+__global__ __launch_bounds__(SMALL_THREADS) void k_sort_small_targets(
+    const double *__restrict__ x, const double *__restrict__ y, int n,
+    const Frame *__restrict__ frame, int *__restrict__ perm) {
+    extern __shared__ __align__(16) unsigned long long small_dyn[];
+    unsigned long long *s_items = small_dyn;
+    int *s_hist = reinterpret_cast<int *>(s_items + SMALL_THREADS * ITEMS);
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    const Frame f = *frame;
+    unsigned long long item[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const int i = warp * 32 * ITEMS + 32 * k + lane;
+        unsigned key = 0xffffffffu;
+        if (i < n) key = (unsigned)target_key(x[i], y[i], f);
+        item[k] = ((unsigned long long)key << 32) | (unsigned)i;
+    }
+    block_sort_items<ITEMS>(item, s_items, s_hist);
+    for (int i = threadIdx.x; i < n; i += SMALL_THREADS) perm[i] = (int)(unsigned)s_items[i];
+}
+
+template <int ITEMS>
+static int sort_small(Context &c, const double *x, const double *y, const double *v, int n,
+                      Frame *frame, int *keys, int *perm, double *xs, double *ys, double *vs) {
+    static const cudaError_t attr_rc = cudaFuncSetAttribute(
+        k_sort_small<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem<ITEMS>());
+    TC_CUDA_TRY(attr_rc);
+    k_sort_small<ITEMS><<<1, SMALL_THREADS, small_smem<ITEMS>(), c.stream>>>(x, y, v, n, frame, keys,
+                                                                             perm, xs, ys, vs);
+    TC_KERNEL_CHECK();
+    return TC_OK;
+}
+
+template <int ITEMS>
+static int sort_small_targets(Context &c, const double *x, const double *y, int n, int *perm) {
+    static const cudaError_t attr_rc =
+        cudaFuncSetAttribute(k_sort_small_targets<ITEMS>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem<ITEMS>());
+    TC_CUDA_TRY(attr_rc);
+    k_sort_small_targets<ITEMS><<<1, SMALL_THREADS, small_smem<ITEMS>(), c.stream>>>(
+        x, y, n, slot_ptr<Frame>(c, S_FRAME), perm);
+    TC_KERNEL_CHECK();
+    return TC_OK;
+}
+
 static int grid_for(int n, int threads, int per_sm = 8) {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -1017,6 +1196,21 @@ int sort_sources(Context &c, const double *x, const double *y, const double *v, 
         return rc;
     partials = reinterpret_cast<double4 *>(reinterpret_cast<char *>(frame) + 64);
     unsigned *done = c.ctrl.bbox_done;
+    // (the stalled look-back of the test setting is the general sort's)
+    if (n <= SMALL_SORT && c.test_stall != TC_STALL_SORT) {
+        const double *v_now = values_ready ? nullptr : v;
+        rc = n <= 4 * SMALL_THREADS
+                 ? sort_small<4>(c, x, y, v_now, n, frame, keys, perm, xs, ys, vs)
+                 : sort_small<16>(c, x, y, v_now, n, frame, keys, perm, xs, ys, vs);
+        if (rc) return rc;
+        c.nsrc = n;
+        if (values_ready) {
+            c.late_x = c.late_y = nullptr;   // x and y are sorted; v in finish_sources
+            c.late_v = v;
+            c.late_ready = values_ready;
+        }
+        return TC_OK;
+    }
 
     // four 8-bit passes over the (key, index) items, then one gather of the records
     if (n >= (1 << 30)) {
@@ -1097,11 +1291,13 @@ int finish_sources(Context &c) {
     if (!c.late_ready) return TC_OK;
     const int n = c.nsrc;
     const int *perm = slot_ptr<int>(c, S_PERM);
-    k_gather_xy<<<grid_for(n, 256, 8), 256, 0, c.stream>>>(perm, c.late_x, c.late_y, n,
-                                                          slot_ptr<double>(c, S_XS),
-                                                          slot_ptr<double>(c, S_YS),
-                                                          c.ctrl.err);
-    TC_KERNEL_CHECK();
+    if (c.late_x) {
+        k_gather_xy<<<grid_for(n, 256, 8), 256, 0, c.stream>>>(perm, c.late_x, c.late_y, n,
+                                                              slot_ptr<double>(c, S_XS),
+                                                              slot_ptr<double>(c, S_YS),
+                                                              c.ctrl.err);
+        TC_KERNEL_CHECK();
+    }
     TC_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.late_ready, 0));
     c.late_ready = nullptr;
     k_gather_v<<<grid_for(n, 256, 8), 256, 0, c.stream>>>(perm, c.late_v, n,
@@ -1112,12 +1308,22 @@ int finish_sources(Context &c) {
 
 
 
-int target_keys(Context &c, const double *xt, const double *yt, int m, int *keys, int *idx) {
-    (void)idx;
-    Frame *frame = slot_ptr<Frame>(c, S_FRAME);
-    k_target_keys<<<grid_for(m, 256), 256, 0, c.stream>>>(xt, yt, m, frame, keys);
+// The targets' Morton order in the sources' frame: *perm is one of the buffers.
+int sort_targets(Context &c, const double *xt, const double *yt, int m, int **perm) {
+    int *tkeys, *tperm, *tkeys2, *tperm2, rc, *ko;
+    if ((rc = ensure(c, S_TPERM, m, &tperm))) return rc;
+    if (m <= SMALL_SORT) {
+        *perm = tperm;
+        return m <= 4 * SMALL_THREADS ? sort_small_targets<4>(c, xt, yt, m, tperm)
+                                      : sort_small_targets<16>(c, xt, yt, m, tperm);
+    }
+    if ((rc = ensure(c, S_TKEYS, m, &tkeys)) || (rc = ensure(c, S_TKEYS2, m, &tkeys2)) ||
+        (rc = ensure(c, S_TPERM2, m, &tperm2)))
+        return rc;
+    k_target_keys<<<grid_for(m, 256), 256, 0, c.stream>>>(xt, yt, m, slot_ptr<Frame>(c, S_FRAME),
+                                                          tkeys);
     TC_KERNEL_CHECK();
-    return TC_OK;
+    return radix_sort_pairs(c, tkeys, nullptr, m, 2 * LMAX, tkeys2, tperm2, tkeys, tperm, &ko, perm);
 }
 
 // ---------------------------------------------------------------------------- allocation-free
@@ -1176,7 +1382,10 @@ void kernels_sort(KernelList &v) {
                        (const void *)k_gather_sources, (const void *)k_gather_xy,
                        (const void *)k_gather_v, (const void *)k_items_split,
                        (const void *)k_scan_reduce, (const void *)k_scan_blocks,
-                       (const void *)k_scan_apply, (const void *)k_scan_small});
+                       (const void *)k_scan_apply, (const void *)k_scan_small,
+                       (const void *)k_sort_small<4>, (const void *)k_sort_small<16>,
+                       (const void *)k_sort_small_targets<4>,
+                       (const void *)k_sort_small_targets<16>});
 }
 
 }  // namespace tc

@@ -285,7 +285,7 @@ int radix_sort_pairs(Context &c, const int *keys_in, const int *vals_in, int n, 
 int sort_sources(Context &c, const double *x, const double *y, const double *v, int n,
                  cudaEvent_t values_ready = nullptr);
 int finish_sources(Context &c);
-int target_keys(Context &c, const double *xt, const double *yt, int m, int *keys, int *idx);
+int sort_targets(Context &c, const double *xt, const double *yt, int m, int **perm);
 
 // ---- tree.cu
 int build_topology(Context &c, int leafcap);
