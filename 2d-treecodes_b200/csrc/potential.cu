@@ -50,7 +50,9 @@ static int task_segment(int ngroups, bool mixed) {
 // point of the box is clearly far (or clearly near) -- with a relative margin of 1e-12, far
 // above the rounding of the per-target test -- the whole mask follows; otherwise the exact
 // per-target test (r^2 < theta^2 |t - com|^2, treecode-potential.cpp:48-50) runs for each
-// target of the mask.  Far targets give an E2P entry (node, far); the rest give a P2P entry for
+// target of the mask, one target per lane, node after node.  The walk is bound by its issue slots:
+// with a lane looping over its own node's targets the 4M mixture's lists took 0.95 ms, so 0.55.
+// Far targets give an E2P entry (node, far); the rest give a P2P entry for
 // a leaf or push the node's four children with the rest.  Every target thus gets exactly the
 // nodes its own depth-first traversal in the reference would give it.  Entries are written in
 // the (deterministic) processing order; the count pass and the fill pass take the same steps.
@@ -78,10 +80,8 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
     int cur[2] = {0, 0};   // MODE 2: entries this warp has written, per kind
     bool full = false;
     __shared__ int2 stack_all[PT_WARPS][PL_STACK];
-    __shared__ double2 targ_all[PT_WARPS][32];
     const int lane = lane_id(), warp = threadIdx.x >> 5;
     int2 *stack = stack_all[warp];
-    double2 *targ = targ_all[warp];
     const unsigned lt = (1u << lane) - 1u;
     const double theta2 = theta * theta;
     unsigned long long e2p_pairs = 0, p2p_pairs = 0;   // warp-uniform work counters
@@ -113,7 +113,6 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
             l1 = offs[ngroups + g + 1];
         }
         __syncwarp();
-        targ[lane] = make_double2(x, y);
         if (lane == 0) stack[0] = make_int2(0, (int)vmask);
         __syncwarp();
         int n0 = 0, n1 = 0, gsrc = 0, top = 1;
@@ -134,8 +133,9 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
             TNode nd = {};
             if (ok) nd = tnode[ent.x];
             unsigned far = 0;
+            bool unsure = false;
+            const double rr = __dmul_rn(nd.r, nd.r);
             if (ok) {
-                const double rr = __dmul_rn(nd.r, nd.r);
                 const double ex = fmax(fmax(bxlo - nd.xcom, nd.xcom - bxhi), 0.0);
                 const double ey = fmax(fmax(bylo - nd.ycom, nd.ycom - byhi), 0.0);
                 const double fx = fmax(nd.xcom - bxlo, bxhi - nd.xcom);
@@ -146,15 +146,21 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
                 } else if (rr >= theta2 * dmax2 * (1.0 + 1e-12)) {
                     far = 0;                            // every target of the box is near
                 } else {
-                    for (unsigned mm = mask; mm; mm &= mm - 1) {
-                        const int tl = __ffs(mm) - 1;
-                        const double2 tp = targ[tl];
-                        // r2 without contraction, as the compiled reference
-                        const double dx = __dsub_rn(tp.x, nd.xcom), dy = __dsub_rn(tp.y, nd.ycom);
-                        const double r2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-                        if (rr < __dmul_rn(theta2, r2)) far |= 1u << tl;
-                    }
+                    unsure = true;
                 }
+            }
+            // The nodes that the box leaves open, one after another, every lane testing its own
+            // target (r2 without contraction, as the compiled reference): ~15 instructions a node,
+            // where a lane looping over its node's targets held up the batch for ~250.
+            for (unsigned open = __ballot_sync(FULL_MASK, unsure); open; open &= open - 1) {
+                const int src = __ffs(open) - 1;
+                const double cx = __shfl_sync(FULL_MASK, nd.xcom, src);
+                const double cy = __shfl_sync(FULL_MASK, nd.ycom, src);
+                const double nr = __shfl_sync(FULL_MASK, rr, src);
+                const double dx = __dsub_rn(x, cx), dy = __dsub_rn(y, cy);
+                const double r2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
+                const unsigned acc = __ballot_sync(FULL_MASK, nr < __dmul_rn(theta2, r2));
+                if (lane == src) far = acc & mask;
             }
             const unsigned rest = mask & ~far;
             const bool leaf = nd.child < 0;
@@ -294,6 +300,20 @@ __device__ __forceinline__ void two_sum_add(float &hi, float &lo, float x) {
     hi = s;
 }
 
+// The same with x = t l, in the roundings that the mixed evaluation is pinned to: MUL_ADD takes the
+// product into the first sum and into the remainder unrounded (the sparse tiles), otherwise it
+// is rounded first (the dense ones).  Left to the compiler, the choice changed with unrelated
+// code around it and moved results by 1e-9.
+template <bool MUL_ADD>
+__device__ __forceinline__ void two_sum_mul(float &hi, float &lo, float t, float l) {
+    const float x = __fmul_rn(t, l);
+    const float s = MUL_ADD ? __fmaf_rn(t, l, hi) : __fadd_rn(hi, x);
+    const float bb = __fsub_rn(s, hi);
+    const float e = MUL_ADD ? __fmaf_rn(t, l, -bb) : __fsub_rn(x, bb);
+    lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bb)), e));
+    hi = s;
+}
+
 __device__ __forceinline__ void split2(double v, float &hi, float &lo) {
     hi = (float)v;
     lo = (float)(v - (double)hi);
@@ -323,6 +343,7 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval_mixed(
     __shared__ float4 s_ny[PE_WARPS][PE_CHUNK / 2];
     __shared__ float2 s_v2[PE_WARPS][PE_CHUNK / 2];
     __shared__ double s_part[PE_WARPS][32];        // P2P lane partials of a sparse mask
+    __shared__ int s_lane_of[PE_WARPS][32];        // the lane of the mask's q-th target
     __shared__ double s_neg_log_c[LOG_NTAB];       // log_pos's table
     load_log_table(s_neg_log_c);
     const int lane = lane_id(), warp = threadIdx.x >> 5;
@@ -465,6 +486,10 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval_mixed(
             split2(x - xref, txh, txl);
             split2(y - yref, tyh, tyl);
             const float ln2 = 0.6931471805599453f, epsf = (float)eps;
+            // a sparse leaf's spreading (below): its mask, 32 / k, lane / k and the lane's target
+            unsigned spread = 0;
+            int sr = 0, sq = 0;
+            float qxh = 0, qxl = 0, qyh = 0, qyl = 0;
             while (tn > 0) {
                 const int cnt = tn;
                 const unsigned cmask = msk;   // this tile's targets (msk moves on to the next tile)
@@ -520,24 +545,31 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval_mixed(
                             acc = __ffma2_rn(make_float2(lg2_approx(r2.x), lg2_approx(r2.y)),
                                              s_v2[warp][q], acc);
                         }
-                        two_sum_add(nh, nl, (acc.x + acc.y) * ln2);
+                        two_sum_mul<false>(nh, nl, acc.x + acc.y, ln2);
                     }
                 } else if (k > 0) {
-                    const int r = 32 / k;
-                    const int qt = lane % k;
-                    const int tl = (int)__fns(cmask, 0, qt + 1);   // lane of this lane's target
+                    if (cmask != spread) {   // once per leaf: its tiles share the mask
+                        spread = cmask;
+                        __syncwarp();
+                        if (mine) s_lane_of[warp][__popc(cmask & ((1u << lane) - 1u))] = lane;
+                        __syncwarp();
+                        sr = 32 / k;
+                        sq = lane / k;
+                        const int tl = s_lane_of[warp][lane - sq * k];   // lane of this lane's target
+                        qxh = __shfl_sync(FULL_MASK, txh, tl);
+                        qxl = __shfl_sync(FULL_MASK, txl, tl);
+                        qyh = __shfl_sync(FULL_MASK, tyh, tl);
+                        qyl = __shfl_sync(FULL_MASK, tyl, tl);
+                    }
+                    const int r = sr;
                     double part = 0;
                     {
-                        const float qxh = __shfl_sync(FULL_MASK, txh, tl);
-                        const float qxl = __shfl_sync(FULL_MASK, txl, tl);
-                        const float qyh = __shfl_sync(FULL_MASK, tyh, tl);
-                        const float qyl = __shfl_sync(FULL_MASK, tyl, tl);
                         float acc = 0;
                         const float *nx = reinterpret_cast<const float *>(s_nx[warp]);
                         const float *ny = reinterpret_cast<const float *>(s_ny[warp]);
                         const float *sv = reinterpret_cast<const float *>(s_v2[warp]);
                         if (lane < r * k)
-                            for (int q = lane / k; q < cnt; q += r) {
+                            for (int q = sq; q < cnt; q += r) {
                                 const int e = 4 * (q >> 1) + (q & 1);
                                 const float dx = (qxh + nx[e]) + (qxl + nx[e + 2]);
                                 const float dy = (qyh + ny[e]) + (qyl + ny[e + 2]);
@@ -551,7 +583,7 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval_mixed(
                         const int q = __popc(cmask & ((1u << lane) - 1u));
                         double sum = 0;
                         for (int i = 0; i < r; ++i) sum += s_part[warp][q + i * k];
-                        two_sum_add(nh, nl, (float)sum * ln2);
+                        two_sum_mul<true>(nh, nl, (float)sum, ln2);
                     }
                     __syncwarp();
                 }
