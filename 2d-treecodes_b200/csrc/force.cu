@@ -254,13 +254,22 @@ constexpr int EV_WARPS = 4;
 constexpr int EV_CHUNK = 32;
 constexpr int NEAR_MIN_BLOCKS = 8;   // near field: at most 64 registers per thread
 
-template <int P>
+constexpr int E2L_BATCH = 16;   // FP64 E2L: cells whose powers are formed together
+
+template <int P, bool MIXED>
 struct FarShared {
     cplx coef[P];                 // E2L: a_k z^-(k+1); E2P: (k+1) a_k
     cplx local[P + 1];            // local expansion L_1..L_P
-    float4 coef32[P];             // mixed E2P: scaled coefficient j as (re, re, im, im)
-    float2 cf[P];                 // mixed E2L: D_k u^(k+1)
-    float4 lf[P + 1];             // mixed L2P: l M_l as (re, re, im, im)
+    // z0^-l, l = 1..P, of a batch's cells; the odd row length keeps the eight lanes of a 16-byte
+    // access, one cell each, in distinct banks
+    cplx pow[E2L_BATCH][P + 1];
+    double mass[E2L_BATCH];
+};
+template <int P>
+struct FarShared<P, true> {
+    float4 coef32[P];             // E2P: scaled coefficient j as (re, re, im, im)
+    float2 cf[P];                 // E2L: D_k u^(k+1)
+    float4 lf[P + 1];             // L2P: l M_l as (re, re, im, im)
 };
 
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
@@ -284,7 +293,7 @@ __device__ __forceinline__ float2 cpowf_int(float2 z, int e) {
 // to 36 words so that the 8 columns (4 rows) a warp reads at once fall in distinct banks.
 constexpr int NEAR_ROW = EV_CHUNK + 4;
 template <bool MIXED>
-struct NearShared {
+struct __align__(16) NearShared {
     double2 sxy[EV_CHUNK];
     double sv[EV_CHUNK];
 };
@@ -333,9 +342,9 @@ __global__ __launch_bounds__(EV_WARPS * 32, MIXED ? 5 : 4) void k_force_far(
     double *__restrict__ yout, int brick_lo, int brick_hi, int *brick_ctr,
     const float2 *__restrict__ sexp, const float *__restrict__ sscale) {
     const BlockLayout L = LBS ? BlockLayout{LBS, LBS - 3} : L_arg;
-    __shared__ FarShared<P> shared[EV_WARPS];
+    __shared__ FarShared<P, MIXED> shared[EV_WARPS];
     const int lane = lane_id(), warp = threadIdx.x >> 5;
-    FarShared<P> &sh = shared[warp];
+    FarShared<P, MIXED> &sh = shared[warp];
     const int tx = lane & 7, ty = lane >> 3;   // targets (tx, ty) and (tx, ty + 4)
 
     // signed binomials of lane l = lane + 1: (-1)^k C(l+k-1, k-1), k = 1..P, in registers
@@ -447,45 +456,61 @@ __global__ __launch_bounds__(EV_WARPS * 32, MIXED ? 5 : 4) void k_force_far(
             cplx Lc = {0.0, 0.0};
             const int l = lane + 1;
             const double minv = -1.0 / l;
-            // the next cell is loaded while the current one is used
-            TNode nd_n = {};
-            double m_n = 0, ar_n = 0, ai_n = 0;
-            auto fetch = [&](int at) {
-                const int node = lists[at];
-                nd_n = tnode[node];
-                m_n = mass[node];
-                if (lane < P) {
-                    const double *ex = exps + (size_t)node * 2 * P;
-                    ar_n = ex[lane];
-                    ai_n = ex[P + lane];
-                }
-            };
-            if (beg < end) fetch(beg);
-            for (int it = beg; it < end; ++it) {
-                const TNode nd = nd_n;
-                const double m = m_n;
-                const cplx a = {ar_n, ai_n};
-                if (it + 1 < end) fetch(it + 1);
+            // Cells in batches of E2L_BATCH: two lanes per cell form the odd and the even powers
+            // z0^-l by repeated products with z0^-2, and every lane then reads the power it needs.
+            // (Each lane raising z0^-1 to its own l took ~40 of the ~130 FP64 instructions a
+            // cell cost; this takes 3 to 6, and a twelfth of the reciprocals.)
+            // The next cell's coefficients are loaded while the current one is used.
+            const int half = lane / E2L_BATCH;   // 0: odd powers, 1: even ones
+            for (int b0 = beg; b0 < end; b0 += E2L_BATCH) {
+                const int nb = min(E2L_BATCH, end - b0);
+                const int mine = lists[b0 + min(lane & (E2L_BATCH - 1), nb - 1)];
+                const TNode nd = tnode[mine];
                 const double zx = nd.xcom - b.x0b, zy = nd.ycom - b.y0b;
-                const double r2z0 = zx * zx + zy * zy;
-                const cplx zinv = {zx / r2z0, -zy / r2z0};
-                cplx zl = {0.0, 0.0};
-                if (lane < P) {
-                    zl = cpow_int(zinv, l);        // z0^-l
-                    sh.coef[lane] = cmul(a, zl);   // C_l = a_{l-1} z0^-l
-                }
+                const double iz = rcp_nr(zx * zx + zy * zy);
+                const cplx u = {zx * iz, -zy * iz};
+                const cplx u2 = cmul(u, u);
+                cplx p = half ? u2 : u;
+                const int c = lane & (E2L_BATCH - 1);
                 __syncwarp();
-                if (lane < P) {
-                    double tr = l == 1 ? -m : m * minv, ti = 0.0;
+                if (!half) sh.mass[c] = mass[mine];
 #pragma unroll
-                    for (int k = 0; k < P; ++k) {
-                        const cplx ck = sh.coef[k];
-                        tr = fma(bsg[k], ck.re, tr);
-                        ti = fma(bsg[k], ck.im, ti);
-                    }
-                    Lc = cfma({tr, ti}, zl, Lc);
+                for (int q = 0; q < P / 2; ++q) {
+                    sh.pow[c][2 * q + half] = p;
+                    if (q + 1 < P / 2) p = cmul(p, u2);
                 }
                 __syncwarp();
+                double ar_n = 0, ai_n = 0;
+                auto fetch = [&](int node) {
+                    if (lane < P) {
+                        const double *ex = exps + (size_t)node * 2 * P;
+                        ar_n = ex[lane];
+                        ai_n = ex[P + lane];
+                    }
+                };
+                fetch(__shfl_sync(FULL_MASK, mine, 0));
+                for (int k0 = 0; k0 < nb; ++k0) {
+                    const cplx a = {ar_n, ai_n};
+                    if (k0 + 1 < nb) fetch(__shfl_sync(FULL_MASK, mine, k0 + 1));
+                    const double m = sh.mass[k0];
+                    cplx zl = {0.0, 0.0};
+                    if (lane < P) {
+                        zl = sh.pow[k0][lane];         // z0^-l
+                        sh.coef[lane] = cmul(a, zl);   // C_l = a_{l-1} z0^-l
+                    }
+                    __syncwarp();
+                    if (lane < P) {
+                        double tr = l == 1 ? -m : m * minv, ti = 0.0;
+#pragma unroll
+                        for (int k = 0; k < P; ++k) {
+                            const cplx ck = sh.coef[k];
+                            tr = fma(bsg[k], ck.re, tr);
+                            ti = fma(bsg[k], ck.im, ti);
+                        }
+                        Lc = cfma({tr, ti}, zl, Lc);
+                    }
+                    __syncwarp();
+                }
             }
             if (lane < P) sh.local[lane + 1] = Lc;
             __syncwarp();
@@ -508,7 +533,7 @@ __global__ __launch_bounds__(EV_WARPS * 32, MIXED ? 5 : 4) void k_force_far(
         }
 
         // ---------------- E2P (force-kernels.m4:57-98): w = m/z - sum (j+1) a_j z^-(j+2)
-        if (MIXED) {
+        if constexpr (MIXED) {
             // FP32: u = 1/z, u' = R u with R the cell's power-of-two radius, scaled coefficients
             // D_j = (j+1) a_j / R^(j+1), w = u (m - u' Q(u')), Q(u') = sum_j D_j u'^j; the
             // Horner steps of the lane's two targets run side by side in f32x2 registers
@@ -793,8 +818,10 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
             while (tn > 0) {
                 const int cnt = tn;
                 __syncwarp();
-                sh.sxy[lane] = make_double2(px, py);
-                sh.sv[lane] = pv;
+                // (a zero value at the origin past the tile, for the two-source steps)
+                const bool live = lane < cnt;
+                sh.sxy[lane] = make_double2(live ? px : 0.0, live ? py : 0.0);
+                sh.sv[lane] = live ? pv : 0.0;
                 __syncwarp();
                 next_tile(t0, tn);
                 if (lane < tn) {
@@ -802,10 +829,7 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
                     py = ys[t0 + lane];
                     pv = vs[t0 + lane];
                 }
-#pragma unroll 4
-                for (int k = 0; k < cnt; ++k) {
-                    const double2 sp = sh.sxy[k];
-                    const double v = sh.sv[k];
+                auto pair = [&](double2 sp, double v) {
                     const double xr = xt - sp.x;
                     const double xr2e = fma(xr, xr, eps);
                     const double yr0 = yt0 - sp.y, yr1 = yt1 - sp.y;
@@ -816,6 +840,13 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
                     ay0 = fma(yr0, f0, ay0);
                     ax1 = fma(xr, f1, ax1);
                     ay1 = fma(yr1, f1, ay1);
+                };
+                const double2 *v2 = reinterpret_cast<const double2 *>(sh.sv);
+#pragma unroll 2
+                for (int k = 0; k < cnt; k += 2) {
+                    const double2 v = v2[k >> 1];
+                    pair(sh.sxy[k], v.x);
+                    pair(sh.sxy[k + 1], v.y);
                 }
             }
         }
