@@ -254,23 +254,41 @@ constexpr int EV_WARPS = 4;
 constexpr int EV_CHUNK = 32;
 constexpr int NEAR_MIN_BLOCKS = 8;   // near field: at most 64 registers per thread
 
+template <bool MIXED>
+using local_t = typename std::conditional<MIXED, float2, cplx>::type;
+
 constexpr int E2L_BATCH = 16;   // FP64 E2L: cells whose powers are formed together
 
 template <int P, bool MIXED>
-struct FarShared {
-    cplx coef[P];                 // E2L: a_k z^-(k+1); E2P: (k+1) a_k
-    cplx local[P + 1];            // local expansion L_1..L_P
+struct E2lShared {
+    cplx coef[P];                 // a_k z^-(k+1)
     // z0^-l, l = 1..P, of a batch's cells; the odd row length keeps the eight lanes of a 16-byte
     // access, one cell each, in distinct banks
     cplx pow[E2L_BATCH][P + 1];
     double mass[E2L_BATCH];
 };
 template <int P>
+struct E2lShared<P, true> {
+    float2 cf[P];                 // D_k u^(k+1)
+};
+
+template <int P, bool MIXED>
+struct FarShared {
+    cplx coef[P];                 // E2P: (k+1) a_k
+    cplx local[P + 1];            // local expansion L_1..L_P
+};
+template <int P>
 struct FarShared<P, true> {
     float4 coef32[P];             // E2P: scaled coefficient j as (re, re, im, im)
-    float2 cf[P];                 // E2L: D_k u^(k+1)
     float4 lf[P + 1];             // L2P: l M_l as (re, re, im, im)
 };
+
+// Few bricks (at most about twice the far field's resident warps): a block per brick instead of a
+// warp, so that the solve does not wait for one warp's chain of cells.  The far field alone, a
+// warp per brick and this: 1936 bricks, mixed, 160 -> 121 us; 576 bricks, FP64, 56 -> 42 us.
+// With more bricks the separate E2L launch and the idle lanes cost more than they give (65,536
+// bricks, mixed, 578 -> 670 us).
+static bool share_bricks(int nbricks) { return nbricks <= 8192; }
 
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
@@ -326,6 +344,179 @@ __device__ __forceinline__ void split_f32(double v, float &hi, float &lo) {
     lo = (float)(v - (double)hi);
 }
 
+// The signed binomials of lane l = lane + 1: (-1)^k C(l+k-1, k-1), k = 1..P, held in registers (in
+// shared memory, for a higher occupancy, the far field measured 18% slower); the mixed form's
+// FP32 E2L uses them divided by k (its coefficients carry a factor k, see brick_local).
+template <int P, bool MIXED>
+struct SignedBinomials {
+    typename std::conditional<MIXED, float, double>::type v[P];
+    __device__ __forceinline__ SignedBinomials() {
+        const int l = lane_id() < P ? lane_id() + 1 : 1;
+#pragma unroll
+        for (int k = 1; k <= P; ++k) {
+            const double b = (k & 1 ? -1.0 : 1.0) * c_binom_f.c[l + k - 1][k - 1];
+            v[k - 1] = MIXED ? b / k : b;
+        }
+    }
+};
+
+// E2L: the local expansion about a brick's centre from its E2L list
+// (force-kernels.m4:102-155), lane l - 1 forming coefficient l (mixed: the scaled M_l).
+template <int P, bool MIXED>
+__device__ __forceinline__ local_t<MIXED> brick_local(
+    int brick, const Brick &b, const SignedBinomials<P, MIXED> &bin, E2lShared<P, MIXED> &sh,
+    const TNode *__restrict__ tnode, const double *__restrict__ mass,
+    const double *__restrict__ exps, const int *__restrict__ offs, const int *__restrict__ lists,
+    const float2 *__restrict__ sexp, const float *__restrict__ sscale) {
+    const int lane = lane_id();
+    const auto &bsg = bin.v;
+    if constexpr (MIXED) {
+        // FP32 on power-of-two scaled quantities: R the cell's scale, rho >= r_brick the
+        // brick's, u = R / z0, w = rho / z0, D_k = (k+1) a_k / R^(k+1) (sexp).  Scaled local
+        // coefficients M_l = L_l rho^(l-1) = (w^l / rho) [-m/l + sum_k (-1)^k C(l+k-1, k-1)
+        // (D_{k-1} / k) u^k]: an E2L cell has d > 3 r and r >= r_brick, so every term is
+        // bounded by the cell's mass times ((r + rho) / d)^(l+k) < (2/3)^(l+k) (up to the
+        // roundings of R and rho), nothing over- or underflows FP32, and the rounding errors
+        // stay relative to the terms.  Lane l - 1 forms M_l; L2P uses l M_l.
+        const int beg = offs[brick], end = offs[brick + 1];
+        float2 Ml = make_float2(0.f, 0.f);
+        const int l = lane + 1;
+        const float minv = -1.f / (float)l;
+        int erho = 0;
+        frexp(b.rbrick, &erho);
+        const double rho = ldexp(1.0, erho);   // 2^e > r_brick
+        TNode nd_n = {};
+        double m_n = 0;
+        float sc_n = 1.f;
+        float2 c_n = make_float2(0.f, 0.f);
+        auto fetch = [&](int at) {
+            const int node = lists[at];
+            nd_n = tnode[node];
+            m_n = mass[node];
+            sc_n = sscale[node];
+            if (lane < P) c_n = sexp[(size_t)node * P + lane];
+        };
+        if (beg < end) fetch(beg);
+        for (int it = beg; it < end; ++it) {
+            const TNode nd = nd_n;
+            const float m = (float)m_n;
+            const double R = sc_n;
+            const float2 dk = c_n;
+            if (it + 1 < end) fetch(it + 1);
+            const double zx = nd.xcom - b.x0b, zy = nd.ycom - b.y0b;
+            const double iz = rcp_nr(zx * zx + zy * zy);
+            const float2 u = make_float2((float)(R * zx * iz), (float)(-R * zy * iz));
+            const float2 w = make_float2((float)(rho * zx * iz), (float)(-rho * zy * iz));
+            __syncwarp();
+            if (lane < P) sh.cf[lane] = cmulf(dk, cpowf_int(u, l));   // D_{l-1} u^l
+            __syncwarp();
+            if (lane < P) {
+                float tr = l == 1 ? -m : m * minv, ti = 0.f;
+#pragma unroll
+                for (int k = 0; k < P; ++k) {
+                    const float2 ck = sh.cf[k];
+                    tr = fmaf(bsg[k], ck.x, tr);
+                    ti = fmaf(bsg[k], ck.y, ti);
+                }
+                const float2 t = cmulf(make_float2(tr, ti), cpowf_int(w, l));
+                Ml.x += t.x;
+                Ml.y += t.y;
+            }
+        }
+        return Ml;
+    } else {
+        const int beg = offs[brick], end = offs[brick + 1];
+        cplx Lc = {0.0, 0.0};
+        const int l = lane + 1;
+        const double minv = -1.0 / l;
+        // Cells in batches of E2L_BATCH: two lanes per cell form the odd and the even powers
+        // z0^-l by repeated products with z0^-2, and every lane then reads the power it needs.
+        // (Each lane raising z0^-1 to its own l took ~40 of the ~130 FP64 instructions a
+        // cell cost; this takes 3 to 6, and a twelfth of the reciprocals.)
+        // The next cell's coefficients are loaded while the current one is used.
+        const int half = lane / E2L_BATCH;   // 0: odd powers, 1: even ones
+        for (int b0 = beg; b0 < end; b0 += E2L_BATCH) {
+            const int nb = min(E2L_BATCH, end - b0);
+            const int mine = lists[b0 + min(lane & (E2L_BATCH - 1), nb - 1)];
+            const TNode nd = tnode[mine];
+            const double zx = nd.xcom - b.x0b, zy = nd.ycom - b.y0b;
+            const double iz = rcp_nr(zx * zx + zy * zy);
+            const cplx u = {zx * iz, -zy * iz};
+            const cplx u2 = cmul(u, u);
+            cplx p = half ? u2 : u;
+            const int c = lane & (E2L_BATCH - 1);
+            __syncwarp();
+            if (!half) sh.mass[c] = mass[mine];
+#pragma unroll
+            for (int q = 0; q < P / 2; ++q) {
+                sh.pow[c][2 * q + half] = p;
+                if (q + 1 < P / 2) p = cmul(p, u2);
+            }
+            __syncwarp();
+            double ar_n = 0, ai_n = 0;
+            auto fetch = [&](int node) {
+                if (lane < P) {
+                    const double *ex = exps + (size_t)node * 2 * P;
+                    ar_n = ex[lane];
+                    ai_n = ex[P + lane];
+                }
+            };
+            fetch(__shfl_sync(FULL_MASK, mine, 0));
+            for (int k0 = 0; k0 < nb; ++k0) {
+                const cplx a = {ar_n, ai_n};
+                if (k0 + 1 < nb) fetch(__shfl_sync(FULL_MASK, mine, k0 + 1));
+                const double m = sh.mass[k0];
+                cplx zl = {0.0, 0.0};
+                if (lane < P) {
+                    zl = sh.pow[k0][lane];         // z0^-l
+                    sh.coef[lane] = cmul(a, zl);   // C_l = a_{l-1} z0^-l
+                }
+                __syncwarp();
+                if (lane < P) {
+                    double tr = l == 1 ? -m : m * minv, ti = 0.0;
+#pragma unroll
+                    for (int k = 0; k < P; ++k) {
+                        const cplx ck = sh.coef[k];
+                        tr = fma(bsg[k], ck.re, tr);
+                        ti = fma(bsg[k], ck.im, ti);
+                    }
+                    Lc = cfma({tr, ti}, zl, Lc);
+                }
+                __syncwarp();
+            }
+        }
+        return Lc;
+    }
+}
+
+// The local expansions of every brick, for the far field that shares a brick among warps.
+template <int P, bool MIXED>
+__global__ __launch_bounds__(EV_WARPS * 32, MIXED ? 6 : 4) void k_force_e2l(
+    int nbricks, BlockLayout L, const double *__restrict__ x0s, const double *__restrict__ y0s,
+    const double *__restrict__ hs, const TNode *__restrict__ tnode,
+    const double *__restrict__ mass, const double *__restrict__ exps,
+    const int *__restrict__ offs, const int *__restrict__ lists, int *brick_ctr,
+    const float2 *__restrict__ sexp, const float *__restrict__ sscale,
+    local_t<MIXED> *__restrict__ local) {
+    __shared__ E2lShared<P, MIXED> shared[EV_WARPS];
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    const SignedBinomials<P, MIXED> bin;
+    for (;;) {
+        int brick = 0;
+        if (lane == 0) brick = atomicAdd(brick_ctr, 1);
+        brick = __shfl_sync(FULL_MASK, brick, 0);
+        if (brick < 0 || brick >= nbricks) break;   // (a counter not reset: no access)
+        int blk, bx, by;
+        brick_of(L, brick, blk, bx, by);
+        const Brick b = brick_geometry(x0s[blk], y0s[blk], hs[blk], bx, by);
+        const local_t<MIXED> c = brick_local<P, MIXED>(brick, b, bin, shared[warp], tnode, mass,
+                                                       exps, offs, lists, sexp, sscale);
+        if (lane < P) local[(size_t)brick * P + lane] = c;
+        __syncwarp();
+    }
+}
+
+// The far field of every brick: E2L, L2P and E2P, two targets per lane.
 // MIXED = false: plain FP64.  MIXED = true: E2L, L2P and E2P in FP32 on power-of-two scaled
 // quantities (scaled multipole coefficients, scaled local coefficients, offsets over the
 // brick's scale), the two targets of a lane side by side in paired-FP32 (f32x2) registers,
@@ -333,203 +524,114 @@ __device__ __forceinline__ void split_f32(double v, float &hi, float &lo) {
 // LBS > 0: the block layout of side 2^LBS fixed at compile time (the default side 32 has its
 // own instances: the layout arithmetic on kernel arguments measured 3% slower); LBS = 0: the
 // layout L given at run time.
-template <int P, bool MIXED, int LBS>
-__global__ __launch_bounds__(EV_WARPS * 32, MIXED ? 5 : 4) void k_force_far(
+// WPB = 1: a warp per brick, persistent.  WPB = EV_WARPS: a block per brick, for few bricks
+// (share_bricks): the local expansions come from k_force_e2l (null: no brick has an E2L cell), the
+// block's warps take the brick's E2P entries in turn, and their sums are added in warp order.
+template <int P, bool MIXED, int LBS, int WPB>
+__global__ __launch_bounds__(EV_WARPS * 32, WPB > 1 ? (MIXED ? 8 : 5) : (MIXED ? 5 : 4))
+    void k_force_far(
     int nbricks, BlockLayout L_arg, const double *__restrict__ x0s, const double *__restrict__ y0s,
     const double *__restrict__ hs, const TNode *__restrict__ tnode,
     const double *__restrict__ mass, const double *__restrict__ exps,
     const int *__restrict__ offs, const int *__restrict__ lists, double *__restrict__ xout,
     double *__restrict__ yout, int brick_lo, int brick_hi, int *brick_ctr,
-    const float2 *__restrict__ sexp, const float *__restrict__ sscale) {
+    const float2 *__restrict__ sexp, const float *__restrict__ sscale,
+    const local_t<MIXED> *__restrict__ local) {
     const BlockLayout L = LBS ? BlockLayout{LBS, LBS - 3} : L_arg;
-    __shared__ FarShared<P, MIXED> shared[EV_WARPS];
+    constexpr bool SHARED_BRICK = WPB > 1;
+    using binom_t = typename std::conditional<SHARED_BRICK, char, SignedBinomials<P, MIXED>>::type;
+    union WarpShared {
+        FarShared<P, MIXED> far;
+        typename std::conditional<SHARED_BRICK, char, E2lShared<P, MIXED>>::type e2l;
+    };
+    __shared__ WarpShared shared[EV_WARPS];
+    __shared__ double s_sum[SHARED_BRICK ? 4 * (WPB - 1) : 1][32];
+    __shared__ int s_brick;
     const int lane = lane_id(), warp = threadIdx.x >> 5;
-    FarShared<P, MIXED> &sh = shared[warp];
+    FarShared<P, MIXED> &sh = shared[warp].far;
     const int tx = lane & 7, ty = lane >> 3;   // targets (tx, ty) and (tx, ty + 4)
-
-    // signed binomials of lane l = lane + 1: (-1)^k C(l+k-1, k-1), k = 1..P, in registers
-    // (in shared memory, for a higher occupancy, the kernel measured 18% slower); the mixed
-    // form's FP32 E2L uses them divided by k (its coefficients carry a factor k, see E2L)
-    using bsg_t = typename std::conditional<MIXED, float, double>::type;
-    bsg_t bsg[P];
-    {
-        const int l = lane < P ? lane + 1 : 1;
-#pragma unroll
-        for (int k = 1; k <= P; ++k) {
-            const double b = (k & 1 ? -1.0 : 1.0) * c_binom_f.c[l + k - 1][k - 1];
-            bsg[k - 1] = (bsg_t)(MIXED ? b / k : b);
-        }
-    }
+    [[maybe_unused]] const binom_t bin{};
 
     for (;;) {
         int brick = 0;
-        if (lane == 0) brick = brick_lo + atomicAdd(brick_ctr, 1);
-        brick = __shfl_sync(FULL_MASK, brick, 0);
+        if constexpr (SHARED_BRICK) {
+            if (threadIdx.x == 0) s_brick = brick_lo + atomicAdd(brick_ctr, 1);
+            __syncthreads();
+            brick = s_brick;
+        } else {
+            if (lane == 0) brick = brick_lo + atomicAdd(brick_ctr, 1);
+            brick = __shfl_sync(FULL_MASK, brick, 0);
+        }
         if (brick < brick_lo || brick >= brick_hi) break;   // (a counter not reset: no access)
+        const int part = SHARED_BRICK ? warp : 0;
         int blk, bx, by;
         brick_of(L, brick, blk, bx, by);
         const double h = hs[blk];
         const Brick b = brick_geometry(x0s[blk], y0s[blk], h, bx, by);
         double ax0 = 0, ay0 = 0, ax1 = 0, ay1 = 0;
 
-        // ---------------- E2L: local expansion about the brick centre (force-kernels.m4:102-155)
-        if constexpr (MIXED) {
-            // FP32 on power-of-two scaled quantities: R the cell's scale, rho >= r_brick the
-            // brick's, u = R / z0, w = rho / z0, D_k = (k+1) a_k / R^(k+1) (sexp).  Scaled local
-            // coefficients M_l = L_l rho^(l-1) = (w^l / rho) [-m/l + sum_k (-1)^k C(l+k-1, k-1)
-            // (D_{k-1} / k) u^k]: an E2L cell has d > 3 r and r >= r_brick, so every term is
-            // bounded by the cell's mass times ((r + rho) / d)^(l+k) < (2/3)^(l+k) (up to the
-            // roundings of R and rho), nothing over- or underflows FP32, and the rounding errors
-            // stay relative to the terms.  Lane l - 1 forms M_l; L2P uses l M_l.
-            const int beg = offs[brick], end = offs[brick + 1];
-            float2 Ml = make_float2(0.f, 0.f);
-            const int l = lane + 1;
-            const float minv = -1.f / (float)l;
-            int erho = 0;
-            frexp(b.rbrick, &erho);
-            const double rho = ldexp(1.0, erho);   // 2^e > r_brick
-            TNode nd_n = {};
-            double m_n = 0;
-            float sc_n = 1.f;
-            float2 c_n = make_float2(0.f, 0.f);
-            auto fetch = [&](int at) {
-                const int node = lists[at];
-                nd_n = tnode[node];
-                m_n = mass[node];
-                sc_n = sscale[node];
-                if (lane < P) c_n = sexp[(size_t)node * P + lane];
-            };
-            if (beg < end) fetch(beg);
-            for (int it = beg; it < end; ++it) {
-                const TNode nd = nd_n;
-                const float m = (float)m_n;
-                const double R = sc_n;
-                const float2 dk = c_n;
-                if (it + 1 < end) fetch(it + 1);
-                const double zx = nd.xcom - b.x0b, zy = nd.ycom - b.y0b;
-                const double iz = rcp_nr(zx * zx + zy * zy);
-                const float2 u = make_float2((float)(R * zx * iz), (float)(-R * zy * iz));
-                const float2 w = make_float2((float)(rho * zx * iz), (float)(-rho * zy * iz));
-                __syncwarp();
-                if (lane < P) sh.cf[lane] = cmulf(dk, cpowf_int(u, l));   // D_{l-1} u^l
-                __syncwarp();
-                if (lane < P) {
-                    float tr = l == 1 ? -m : m * minv, ti = 0.f;
-#pragma unroll
-                    for (int k = 0; k < P; ++k) {
-                        const float2 ck = sh.cf[k];
-                        tr = fmaf(bsg[k], ck.x, tr);
-                        ti = fmaf(bsg[k], ck.y, ti);
-                    }
-                    const float2 t = cmulf(make_float2(tr, ti), cpowf_int(w, l));
-                    Ml.x += t.x;
-                    Ml.y += t.y;
-                }
+        // ---------------- the local expansion and L2P
+        if (!SHARED_BRICK || (local && part == 0)) {
+            local_t<MIXED> loc = {};
+            if constexpr (SHARED_BRICK) {
+                if (lane < P) loc = local[(size_t)brick * P + lane];
+            } else {
+                loc = brick_local<P, MIXED>(brick, b, bin, shared[warp].e2l, tnode, mass, exps,
+                                            offs, lists, sexp, sscale);
             }
-            __syncwarp();
-            if (lane < P)
-                sh.lf[lane + 1] = make_float4(l * Ml.x, l * Ml.x, l * Ml.y, l * Ml.y);
-            __syncwarp();
-            // L2P (force-kernels.m4:157-191): sum_l l M_l (z / rho)^(l-1) / rho, the lane's two
-            // targets side by side in f32x2 registers
-            const float inv_rho = (float)(1.0 / rho);
-            const float zxr = (float)((-3.5 * h + tx * h) / rho);
-            const float2 zre = make_float2(zxr, zxr);
-            const float2 zim = make_float2((float)((-3.5 * h + ty * h) / rho),
-                                           (float)((-3.5 * h + (ty + 4) * h) / rho));
-            const float2 nzim = make_float2(-zim.x, -zim.y);
-            const float4 top = sh.lf[P];
-            float2 are = make_float2(top.x, top.y), aim = make_float2(top.z, top.w);
-#pragma unroll
-            for (int q = P - 1; q >= 1; --q) {
-                const float4 c = sh.lf[q];
-                const float2 nre = __ffma2_rn(are, zre, __ffma2_rn(aim, nzim, make_float2(c.x, c.y)));
-                aim = __ffma2_rn(are, zim, __ffma2_rn(aim, zre, make_float2(c.z, c.w)));
-                are = nre;
-            }
-            ax0 += (double)(are.x * inv_rho);
-            ay0 -= (double)(aim.x * inv_rho);
-            ax1 += (double)(are.y * inv_rho);
-            ay1 -= (double)(aim.y * inv_rho);
-        } else {
-            const int beg = offs[brick], end = offs[brick + 1];
-            cplx Lc = {0.0, 0.0};
-            const int l = lane + 1;
-            const double minv = -1.0 / l;
-            // Cells in batches of E2L_BATCH: two lanes per cell form the odd and the even powers
-            // z0^-l by repeated products with z0^-2, and every lane then reads the power it needs.
-            // (Each lane raising z0^-1 to its own l took ~40 of the ~130 FP64 instructions a
-            // cell cost; this takes 3 to 6, and a twelfth of the reciprocals.)
-            // The next cell's coefficients are loaded while the current one is used.
-            const int half = lane / E2L_BATCH;   // 0: odd powers, 1: even ones
-            for (int b0 = beg; b0 < end; b0 += E2L_BATCH) {
-                const int nb = min(E2L_BATCH, end - b0);
-                const int mine = lists[b0 + min(lane & (E2L_BATCH - 1), nb - 1)];
-                const TNode nd = tnode[mine];
-                const double zx = nd.xcom - b.x0b, zy = nd.ycom - b.y0b;
-                const double iz = rcp_nr(zx * zx + zy * zy);
-                const cplx u = {zx * iz, -zy * iz};
-                const cplx u2 = cmul(u, u);
-                cplx p = half ? u2 : u;
-                const int c = lane & (E2L_BATCH - 1);
+            if constexpr (MIXED) {
+                const float2 Ml = loc;
+                const int l = lane + 1;
+                int erho = 0;
+                frexp(b.rbrick, &erho);
+                const double rho = ldexp(1.0, erho);   // 2^e > r_brick
                 __syncwarp();
-                if (!half) sh.mass[c] = mass[mine];
-#pragma unroll
-                for (int q = 0; q < P / 2; ++q) {
-                    sh.pow[c][2 * q + half] = p;
-                    if (q + 1 < P / 2) p = cmul(p, u2);
-                }
+                if (lane < P)
+                    sh.lf[lane + 1] = make_float4(l * Ml.x, l * Ml.x, l * Ml.y, l * Ml.y);
                 __syncwarp();
-                double ar_n = 0, ai_n = 0;
-                auto fetch = [&](int node) {
-                    if (lane < P) {
-                        const double *ex = exps + (size_t)node * 2 * P;
-                        ar_n = ex[lane];
-                        ai_n = ex[P + lane];
-                    }
-                };
-                fetch(__shfl_sync(FULL_MASK, mine, 0));
-                for (int k0 = 0; k0 < nb; ++k0) {
-                    const cplx a = {ar_n, ai_n};
-                    if (k0 + 1 < nb) fetch(__shfl_sync(FULL_MASK, mine, k0 + 1));
-                    const double m = sh.mass[k0];
-                    cplx zl = {0.0, 0.0};
-                    if (lane < P) {
-                        zl = sh.pow[k0][lane];         // z0^-l
-                        sh.coef[lane] = cmul(a, zl);   // C_l = a_{l-1} z0^-l
-                    }
-                    __syncwarp();
-                    if (lane < P) {
-                        double tr = l == 1 ? -m : m * minv, ti = 0.0;
+                // L2P (force-kernels.m4:157-191): sum_l l M_l (z / rho)^(l-1) / rho, the lane's two
+                // targets side by side in f32x2 registers
+                const float inv_rho = (float)(1.0 / rho);
+                const float zxr = (float)((-3.5 * h + tx * h) / rho);
+                const float2 zre = make_float2(zxr, zxr);
+                const float2 zim = make_float2((float)((-3.5 * h + ty * h) / rho),
+                                               (float)((-3.5 * h + (ty + 4) * h) / rho));
+                const float2 nzim = make_float2(-zim.x, -zim.y);
+                const float4 top = sh.lf[P];
+                float2 are = make_float2(top.x, top.y), aim = make_float2(top.z, top.w);
 #pragma unroll
-                        for (int k = 0; k < P; ++k) {
-                            const cplx ck = sh.coef[k];
-                            tr = fma(bsg[k], ck.re, tr);
-                            ti = fma(bsg[k], ck.im, ti);
-                        }
-                        Lc = cfma({tr, ti}, zl, Lc);
-                    }
-                    __syncwarp();
+                for (int q = P - 1; q >= 1; --q) {
+                    const float4 c = sh.lf[q];
+                    const float2 nre = __ffma2_rn(are, zre, __ffma2_rn(aim, nzim, make_float2(c.x, c.y)));
+                    aim = __ffma2_rn(are, zim, __ffma2_rn(aim, zre, make_float2(c.z, c.w)));
+                    are = nre;
                 }
-            }
-            if (lane < P) sh.local[lane + 1] = Lc;
-            __syncwarp();
+                ax0 += (double)(are.x * inv_rho);
+                ay0 -= (double)(aim.x * inv_rho);
+                ax1 += (double)(are.y * inv_rho);
+                ay1 -= (double)(aim.y * inv_rho);
+            } else {
+                const cplx Lc = loc;
+                __syncwarp();
+                if (lane < P) sh.local[lane + 1] = Lc;
+                __syncwarp();
 
-            // L2P (force-kernels.m4:157-191): sum_l l L_l z^(l-1), z about the centre
-            const double xr = -3.5 * h + tx * h;
-            const double yr0 = -3.5 * h + ty * h, yr1 = -3.5 * h + (ty + 4) * h;
-            cplx acc0 = {P * sh.local[P].re, P * sh.local[P].im}, acc1 = acc0;
-            const cplx z0 = {xr, yr0}, z1 = {xr, yr1};
+                // L2P (force-kernels.m4:157-191): sum_l l L_l z^(l-1), z about the centre
+                const double xr = -3.5 * h + tx * h;
+                const double yr0 = -3.5 * h + ty * h, yr1 = -3.5 * h + (ty + 4) * h;
+                cplx acc0 = {P * sh.local[P].re, P * sh.local[P].im}, acc1 = acc0;
+                const cplx z0 = {xr, yr0}, z1 = {xr, yr1};
 #pragma unroll
-            for (int l = P - 1; l >= 1; --l) {
-                const cplx cl = {l * sh.local[l].re, l * sh.local[l].im};
-                acc0 = cfma(acc0, z0, cl);
-                acc1 = cfma(acc1, z1, cl);
+                for (int l = P - 1; l >= 1; --l) {
+                    const cplx cl = {l * sh.local[l].re, l * sh.local[l].im};
+                    acc0 = cfma(acc0, z0, cl);
+                    acc1 = cfma(acc1, z1, cl);
+                }
+                ax0 += acc0.re;
+                ay0 -= acc0.im;
+                ax1 += acc1.re;
+                ay1 -= acc1.im;
             }
-            ax0 += acc0.re;
-            ay0 -= acc0.im;
-            ax1 += acc1.re;
-            ay1 -= acc1.im;
         }
 
         // ---------------- E2P (force-kernels.m4:57-98): w = m/z - sum (j+1) a_j z^-(j+2)
@@ -537,7 +639,7 @@ __global__ __launch_bounds__(EV_WARPS * 32, MIXED ? 5 : 4) void k_force_far(
             // FP32: u = 1/z, u' = R u with R the cell's power-of-two radius, scaled coefficients
             // D_j = (j+1) a_j / R^(j+1), w = u (m - u' Q(u')), Q(u') = sum_j D_j u'^j; the
             // Horner steps of the lane's two targets run side by side in f32x2 registers
-            const int beg = offs[nbricks + brick], end = offs[nbricks + brick + 1];
+            const int beg = offs[nbricks + brick] + part, end = offs[nbricks + brick + 1];
             float hx0 = 0, lx0 = 0, hy0 = 0, ly0 = 0, hx1 = 0, lx1 = 0, hy1 = 0, ly1 = 0;
             TNode nd_n = {};
             double m_n = 0;
@@ -551,13 +653,13 @@ __global__ __launch_bounds__(EV_WARPS * 32, MIXED ? 5 : 4) void k_force_far(
                 if (lane < P) c_n = sexp[(size_t)node * P + lane];
             };
             if (beg < end) fetch(beg);
-            for (int it = beg; it < end; ++it) {
+            for (int it = beg; it < end; it += WPB) {
                 const TNode nd = nd_n;
                 const float m = (float)m_n, R = sc_n;
                 __syncwarp();
                 if (lane < P) sh.coef32[lane] = make_float4(c_n.x, c_n.x, c_n.y, c_n.y);
                 __syncwarp();
-                if (it + 1 < end) fetch(it + 1);
+                if (it + WPB < end) fetch(it + WPB);
                 const float rx = (float)((b.xlo - nd.xcom) + tx * h);
                 const float ry0 = (float)((b.ylo - nd.ycom) + ty * h);
                 const float ry1 = (float)((b.ylo - nd.ycom) + (ty + 4) * h);
@@ -589,7 +691,7 @@ __global__ __launch_bounds__(EV_WARPS * 32, MIXED ? 5 : 4) void k_force_far(
             ax1 += (double)hx1 + (double)lx1;
             ay1 += (double)hy1 + (double)ly1;
         } else {
-            const int beg = offs[nbricks + brick], end = offs[nbricks + brick + 1];
+            const int beg = offs[nbricks + brick] + part, end = offs[nbricks + brick + 1];
             // the next cell's record and coefficients are loaded while the current one is used
             TNode nd_n = {};
             double m_n = 0, cr_n = 0, ci_n = 0;
@@ -604,13 +706,13 @@ __global__ __launch_bounds__(EV_WARPS * 32, MIXED ? 5 : 4) void k_force_far(
                 }
             };
             if (beg < end) fetch(beg);
-            for (int it = beg; it < end; ++it) {
+            for (int it = beg; it < end; it += WPB) {
                 const TNode nd = nd_n;
                 const double m = m_n;
                 __syncwarp();
                 if (lane < P) sh.coef[lane] = {cr_n, ci_n};
                 __syncwarp();
-                if (it + 1 < end) fetch(it + 1);
+                if (it + WPB < end) fetch(it + WPB);
                 const double rx = (b.xlo - nd.xcom) + tx * h;
                 const double ry0 = (b.ylo - nd.ycom) + ty * h;
                 const double ry1 = (b.ylo - nd.ycom) + (ty + 4) * h;
@@ -635,6 +737,25 @@ __global__ __launch_bounds__(EV_WARPS * 32, MIXED ? 5 : 4) void k_force_far(
             }
         }
 
+        if constexpr (SHARED_BRICK) {
+            if (warp > 0) {
+                double(*q)[32] = &s_sum[4 * (warp - 1)];
+                q[0][lane] = ax0;
+                q[1][lane] = ay0;
+                q[2][lane] = ax1;
+                q[3][lane] = ay1;
+            }
+            __syncthreads();
+            if (warp > 0) continue;   // (s_sum is written again after the next brick's barrier)
+#pragma unroll
+            for (int w = 0; w < WPB - 1; ++w) {
+                ax0 += s_sum[4 * w][lane];
+                ay0 += s_sum[4 * w + 1][lane];
+                ax1 += s_sum[4 * w + 2][lane];
+                ay1 += s_sum[4 * w + 3][lane];
+            }
+        }
+
         // the far field alone, in the output layout; k_add_far adds it to the near field
         const size_t o0 = target_index(L, blk, bx, by, tx, ty);
         const size_t o1 = o0 + ((size_t)4 << L.lbs);
@@ -656,7 +777,9 @@ __global__ __launch_bounds__(EV_WARPS * 32, MIXED ? 5 : 4) void k_force_far(
 //    target column and row formed once per tile from float hi + lo parts, so the separation
 //    keeps a few float ulps of itself), two sources per step in f32x2 registers, FP32 sums per
 //    tile added into compensated per-target sums.
-template <bool MIXED, int LBS>
+// CUT: tasks of less than a segment (with whole segments the extra position bound would spill, 11%
+// of the mixed kernel on the 16M sheet).
+template <bool MIXED, int LBS, bool CUT>
 __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
     int nbricks, BlockLayout L_arg, const double *__restrict__ x0s, const double *__restrict__ y0s,
     const double *__restrict__ hs, const int2 *__restrict__ range, const double *__restrict__ xs,
@@ -693,27 +816,47 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
         double ax0 = 0, ay0 = 0, ax1 = 0, ay1 = 0;
 
         // Tiles of up to EV_CHUNK consecutive sources of one leaf and one segment walk the
-        // listed leaves in order; positions count the brick's near-field sources.
-        int it = beg, pos = 0, s_next = 0, e_next = 0;
+        // listed leaves in order.
+        int it = beg, s_next = 0, e_next = 0;
         auto take = [&]() { return range[lists[it++]]; };
-        const int lo = part * seg, hi = lo + seg;
-        const int seg0 = lo - (lo & (P2P_SEG - 1)), pos_seg = seg0 + P2P_SEG;
-        // the first tile that starts at or after lo
-        while (it < end) {
-            const int2 rg = take();
-            const int cnt = rg.y - rg.x;
-            if (pos + cnt > lo) {
-                const int first = max(0, seg0 - pos);   // the leaf's first tile of the segment
-                const int skip = first + (max(0, lo - pos - first) + EV_CHUNK - 1) / EV_CHUNK *
-                                             EV_CHUNK;
+        // sources left to the segment's end; a task ends `tail` before it
+        int budget = P2P_SEG;
+        int tail = 0;
+        if constexpr (CUT) {
+            // the first tile that starts at or after source `lo`; positions count the brick's
+            // near-field sources
+            int pos = 0;
+            const int lo = part * seg, seg0 = lo - (lo & (P2P_SEG - 1));
+            while (it < end) {
+                const int2 rg = take();
+                const int cnt = rg.y - rg.x;
+                if (pos + cnt > lo) {
+                    const int first = max(0, seg0 - pos);   // the leaf's first tile of the segment
+                    const int skip = first + (max(0, lo - pos - first) + EV_CHUNK - 1) /
+                                                 EV_CHUNK * EV_CHUNK;
+                    if (skip < cnt) {
+                        s_next = rg.x + skip;
+                        e_next = rg.y;
+                        pos += skip;
+                        break;
+                    }
+                }
+                pos += cnt;
+            }
+            budget = seg0 + P2P_SEG - pos;
+            tail = seg0 + P2P_SEG - lo - seg;
+        } else {
+            int skip = part * P2P_SEG;
+            while (it < end) {
+                const int2 rg = take();
+                const int cnt = rg.y - rg.x;
                 if (skip < cnt) {
                     s_next = rg.x + skip;
                     e_next = rg.y;
-                    pos += skip;
                     break;
                 }
+                skip -= cnt;
             }
-            pos += cnt;
         }
         auto next_tile = [&](int &t0, int &tn) {
             while (s_next >= e_next && it < end) {
@@ -722,10 +865,10 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
                 e_next = rg.y;
             }
             t0 = s_next;
-            tn = pos < hi ? min(min(EV_CHUNK, e_next - s_next), pos_seg - pos) : 0;
-            if (tn < 0) tn = 0;
+            tn = min(min(EV_CHUNK, e_next - s_next), budget);
+            if (tn < 0 || (CUT && budget <= tail)) tn = 0;
             s_next += tn;
-            pos += tn;
+            budget -= tn;
         };
         int t0, tn;
         next_tile(t0, tn);
@@ -1058,10 +1201,15 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
         const bool mixed = c.precision == 1;
         constexpr int LBS32 = 5;   // the default block side, 32
         const bool fixed = L.lbs == LBS32;
-        auto near = mixed ? (fixed ? k_force_near<true, LBS32> : k_force_near<true, 0>)
-                          : (fixed ? k_force_near<false, LBS32> : k_force_near<false, 0>);
-        const int occ_near = mixed ? blocks_per_sm<k_force_near<true, LBS32>>(EV_WARPS * 32, 0)
-                                   : blocks_per_sm<k_force_near<false, LBS32>>(EV_WARPS * 32, 0);
+        auto near_of = [&](auto cut) {
+            constexpr bool CUT = decltype(cut)::value;
+            return mixed ? (fixed ? k_force_near<true, LBS32, CUT> : k_force_near<true, 0, CUT>)
+                         : (fixed ? k_force_near<false, LBS32, CUT> : k_force_near<false, 0, CUT>);
+        };
+        auto near = seg < P2P_SEG ? near_of(std::true_type{}) : near_of(std::false_type{});
+        const int occ_near =
+            mixed ? blocks_per_sm<k_force_near<true, LBS32, false>>(EV_WARPS * 32, 0)
+                  : blocks_per_sm<k_force_near<false, LBS32, false>>(EV_WARPS * 32, 0);
         const int neargrid = (int)std::min<long long>((ntasks + EV_WARPS - 1) / EV_WARPS,
                                                       (long long)sm_count() * occ_near);
         phase_mark(c, 9);
@@ -1102,12 +1250,54 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
         }
         constexpr int LBS32 = 5;   // the default block side, 32
         const bool fixed = L.lbs == LBS32;
-        auto far = mixed ? (fixed ? k_force_far<P, true, LBS32> : k_force_far<P, true, 0>)
-                         : (fixed ? k_force_far<P, false, LBS32> : k_force_far<P, false, 0>);
-        const int occ_far = mixed ? blocks_per_sm<k_force_far<P, true, LBS32>>(EV_WARPS * 32, 0)
-                                  : blocks_per_sm<k_force_far<P, false, LBS32>>(EV_WARPS * 32, 0);
-        const int fargrid = (int)std::min<long long>((nbricks + EV_WARPS - 1) / EV_WARPS,
-                                                     (long long)sm_count() * occ_far);
+        const bool shared_bricks = share_bricks(nbricks);
+        // few bricks: their local expansions, unless no brick has an E2L cell
+        void *local = nullptr;
+        if (shared_bricks && tot[0] > 0) {
+            char *buf;
+            if ((rc2 = ensure(c, S_LOCAL,
+                              (size_t)nbricks * P * (mixed ? sizeof(float2) : sizeof(cplx)), &buf)))
+                return rc2;
+            local = buf;
+        }
+        if (c.serial_eval) TC_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.ev_near, 0));
+        phase_mark(c, 6);
+        auto e2l = [&](auto kernel, int occ, auto *out) -> int {
+            const int grid = (int)std::min<long long>((nbricks + EV_WARPS - 1) / EV_WARPS,
+                                                      (long long)sm_count() * occ);
+            kernel<<<grid, EV_WARPS * 32, 0, c.stream>>>(
+                nbricks, L, x0s, y0s, hs, tnode, slot_ptr<double>(c, S_MASS),
+                slot_ptr<double>(c, S_EXPS), offs, lists, c.ctrl.e2l_ctr, sexp, sscale, out);
+            TC_KERNEL_CHECK();
+            return TC_OK;
+        };
+        if (local &&
+            (rc2 = mixed ? e2l(k_force_e2l<P, true>,
+                               blocks_per_sm<k_force_e2l<P, true>>(EV_WARPS * 32, 0),
+                               static_cast<float2 *>(local))
+                         : e2l(k_force_e2l<P, false>,
+                               blocks_per_sm<k_force_e2l<P, false>>(EV_WARPS * 32, 0),
+                               static_cast<cplx *>(local))))
+            return rc2;
+        // the far field of bricks [b0, b1)
+        auto far_launch = [&](auto form, double *xo, double *yo, int b0, int b1, int *ctr) -> int {
+            constexpr bool M = decltype(form)::value;
+            auto kernel = shared_bricks
+                              ? (fixed ? k_force_far<P, M, LBS32, EV_WARPS>
+                                       : k_force_far<P, M, 0, EV_WARPS>)
+                              : (fixed ? k_force_far<P, M, LBS32, 1> : k_force_far<P, M, 0, 1>);
+            const int occ =
+                shared_bricks
+                    ? blocks_per_sm<k_force_far<P, M, LBS32, EV_WARPS>>(EV_WARPS * 32, 0)
+                    : blocks_per_sm<k_force_far<P, M, LBS32, 1>>(EV_WARPS * 32, 0);
+            const int blocks = shared_bricks ? nbricks : (nbricks + EV_WARPS - 1) / EV_WARPS;
+            kernel<<<(int)std::min<long long>(blocks, (long long)sm_count() * occ), EV_WARPS * 32, 0,
+                     c.stream>>>(nbricks, L, x0s, y0s, hs, tnode, slot_ptr<double>(c, S_MASS),
+                                 slot_ptr<double>(c, S_EXPS), offs, lists, xo, yo, b0, b1, ctr,
+                                 sexp, sscale, static_cast<const local_t<M> *>(local));
+            TC_KERNEL_CHECK();
+            return TC_OK;
+        };
         // With host outputs of 2^21 targets or more (a copy of >= 32 MB, ~0.6 ms over PCIe) the
         // blocks are evaluated in FORCE_CHUNKS runs, each copied to the host on the auxiliary
         // stream while the next one is evaluated; below that the runs' tails cost more than
@@ -1123,17 +1313,13 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
             host_x && (size_t)nblocks * per_block >= ((size_t)1 << 21) && nblocks >= FORCE_CHUNKS
                 ? FORCE_CHUNKS
                 : 1;
-        if (c.serial_eval) TC_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.ev_near, 0));
-        phase_mark(c, 6);
         for (int k = 0; k < nchunks; ++k) {
             const int blk0 = (int)((long long)nblocks * k / nchunks);
             const int blk1 = (int)((long long)nblocks * (k + 1) / nchunks);
             const int b0 = blk0 << (2 * L.lbps), b1 = blk1 << (2 * L.lbps);
-            far<<<fargrid, EV_WARPS * 32, 0, c.stream>>>(
-                nbricks, L, x0s, y0s, hs, tnode, slot_ptr<double>(c, S_MASS),
-                slot_ptr<double>(c, S_EXPS), offs, lists, xfar, yfar, b0, b1, far_ctr + k, sexp,
-                sscale);
-            TC_KERNEL_CHECK();
+            if ((rc2 = mixed ? far_launch(std::true_type{}, xfar, yfar, b0, b1, far_ctr + k)
+                             : far_launch(std::false_type{}, xfar, yfar, b0, b1, far_ctr + k)))
+                return rc2;
             if (k == nchunks - 1) phase_mark(c, 7);
             const size_t o = blk0 * per_block, cnt = (size_t)(blk1 - blk0) * per_block;
             if (k == 0) TC_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.ev_near, 0));
@@ -1161,15 +1347,27 @@ void kernels_force(KernelList &v) {
     v.insert(v.end(), {(const void *)k_force_lists<1>, (const void *)k_force_lists<2>,
                        (const void *)k_force_lists_copy, (const void *)k_task_map,
                        (const void *)k_add_far,
-                       (const void *)k_force_gather_parts, (const void *)k_force_near<true, 5>,
-                       (const void *)k_force_near<true, 0>, (const void *)k_force_near<false, 5>,
-                       (const void *)k_force_near<false, 0>});
-#define TC_FORCE_KERNELS(P)                                                                      \
-    v.insert(v.end(), {(const void *)k_force_far<P, true, 5>, (const void *)k_force_far<P, true, 0>, \
-                       (const void *)k_force_far<P, false, 5>,                                   \
-                       (const void *)k_force_far<P, false, 0>, (const void *)k_scale_coeffs<P, true>});
+                       (const void *)k_force_gather_parts});
+#define TC_NEAR_KERNELS(CUT)                                                                      \
+    v.insert(v.end(), {(const void *)k_force_near<true, 5, CUT>,                                  \
+                       (const void *)k_force_near<true, 0, CUT>,                                  \
+                       (const void *)k_force_near<false, 5, CUT>,                                 \
+                       (const void *)k_force_near<false, 0, CUT>});
+    TC_NEAR_KERNELS(true)
+    TC_NEAR_KERNELS(false)
+#undef TC_NEAR_KERNELS
+#define TC_FAR_KERNELS(P, M)                                                                 \
+    v.insert(v.end(), {(const void *)k_force_far<P, M, 5, 1>, (const void *)k_force_far<P, M, 0, 1>, \
+                       (const void *)k_force_far<P, M, 5, EV_WARPS>,                          \
+                       (const void *)k_force_far<P, M, 0, EV_WARPS>,                          \
+                       (const void *)k_force_e2l<P, M>});
+#define TC_FORCE_KERNELS(P) \
+    TC_FAR_KERNELS(P, true) \
+    TC_FAR_KERNELS(P, false) \
+    v.push_back((const void *)k_scale_coeffs<P, true>);
     TC_FOR_EACH_ORDER(TC_FORCE_KERNELS)
 #undef TC_FORCE_KERNELS
+#undef TC_FAR_KERNELS
 }
 
 }  // namespace tc

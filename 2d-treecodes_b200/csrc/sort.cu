@@ -1162,6 +1162,7 @@ int ctrl_prepare(Context &c, int n, int m) {
         take(k.meta, 4);
         take(k.near_ctr, 1);
         take(k.far_ctr, FORCE_CHUNKS);
+        take(k.e2l_ctr, 1);
         take(k.t_tile_ctr, RS_MAX_PASSES);
         take(k.hist, NHIST * RS_RADIX);
         take(k.t_hist, RS_MAX_PASSES * RS_RADIX);
@@ -1283,8 +1284,8 @@ int sort_sources(Context &c, const double *x, const double *y, const double *v, 
         return TC_OK;
     }
     // a window of the sorted order in flight at a time (4 CTAs per SM): its records come from
-    // a compact range of buckets, which stays in L2 (one 32-byte load per record instead of two of 16:
-    // the random loads are bound by the L1 tag lookups; 300 -> 265 us on the 16M sheet)
+    // a compact range of buckets, which stays in L2.  One 32-byte load per record instead of two
+    // of 16 bytes: the random loads are bound by the L1 tag lookups (300 -> 265 us, 16M sheet)
     TC_CUDA_TRY(launch_pdl(ovl, k_gather_sources, grid_for(n, GS_THREADS * GS_ITEMS, 4),
                            GS_THREADS, 0, c.stream, (const unsigned long long *)items_a,
                            (const double2 *)rec, n, keys, perm, xs, ys, vs, err));
