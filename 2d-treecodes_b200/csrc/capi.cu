@@ -252,6 +252,7 @@ static int preload_kernels(int device) {
         cudaFuncAttributes a;
         TC_CUDA_TRY(cudaFuncGetAttributes(&a, k));
     }
+    if (int rc = prefer_force_carveout()) return rc;
     loaded.push_back(device);
     return TC_OK;
 }

@@ -316,6 +316,9 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
                int nblocks, double *xout, double *yout, OverlapFn between,
                double *host_x = nullptr, double *host_y = nullptr);
 
+// Shared-memory preferences of kernels that run beside others (once per device).
+int prefer_force_carveout();
+
 // ---- potential.cu
 int potential(Context &c, double theta, const double *xt, const double *yt, int m, double *out,
               OverlapFn between);
