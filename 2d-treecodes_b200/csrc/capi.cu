@@ -375,6 +375,7 @@ static int build_tree_moments(Context &c, int kind, const double *x, const doubl
 static int build_tree(Context &c, int kind, const double *x, const double *y, const double *v,
                       int n) {
     int rc;
+    c.single = false;
     if ((rc = build_tree_moments(c, kind, x, y, v, n)) || (rc = upward_expansions(c))) return rc;
     phase_mark(c, 3);
     return TC_OK;
@@ -402,6 +403,7 @@ static int potential_device(Context &c, double theta, const double *xs, const do
     }
     int rc;
     phase_mark(c, 0);
+    c.single = single_stream(n, (m + 31) / 32) && !values_ready;
     if ((rc = build_tree_moments(c, 0, xs, ys, vs, n, m, values_ready))) return rc;
     if ((rc = potential(c, theta, xt, yt, m, out, expansions_then_mark))) return rc;
     phase_mark(c, 5);
@@ -436,6 +438,7 @@ static int force_device(Context &c, double theta, const double *xs, const double
     }
     int rc;
     phase_mark(c, 0);
+    c.single = false;
     if ((rc = build_tree_moments(c, 1, xs, ys, vs, n, 0, values_ready))) return rc;
     if ((rc = force_mrag(c, theta, x0s, y0s, hs, nb, xo, yo, expansions_then_mark, host_x,
                          host_y)))
@@ -468,8 +471,15 @@ struct StagedArray {
 };
 
 static int stage_split(Context &c, std::initializer_list<StagedArray> first,
-                       std::initializer_list<StagedArray> later) {
+                       std::initializer_list<StagedArray> later, bool one_stream) {
     int rc;
+    if (one_stream) {   // a small solve: all of them on the main stream
+        for (const StagedArray &a : first)
+            if ((rc = stage(c, a.slot, a.host, a.n, a.dev))) return rc;
+        for (const StagedArray &a : later)
+            if ((rc = stage(c, a.slot, a.host, a.n, a.dev))) return rc;
+        return TC_OK;
+    }
     for (const StagedArray &a : first)
         if ((rc = stage(c, a.slot, a.host, a.n, a.dev))) return rc;
     for (const StagedArray &a : later)
@@ -505,13 +515,15 @@ static int potential_host(Context &c, double theta, const double *xs, const doub
     if (m == 0) return TC_OK;
     int rc;
     double *dx, *dy, *dv, *dxt, *dyt, *dout;
+    const bool single = single_stream(n, (m + 31) / 32);
     // the targets follow the values on the auxiliary stream, where the target sort runs
     if ((rc = stage_split(c, {{S_XIN, xs, (size_t)n, &dx}, {S_YIN, ys, (size_t)n, &dy}},
                           {{S_VIN, vs, (size_t)n, &dv}, {S_XT, xt, (size_t)m, &dxt},
-                           {S_YT, yt, (size_t)m, &dyt}})) ||
+                           {S_YT, yt, (size_t)m, &dyt}}, single)) ||
         (rc = ensure(c, S_OUTX, m, &dout)))
         return drain_and_fail(c, rc);
-    rc = potential_device(c, theta, dx, dy, dv, n, dxt, dyt, m, dout, c.ev_inputs);
+    rc = potential_device(c, theta, dx, dy, dv, n, dxt, dyt, m, dout,
+                          single ? nullptr : c.ev_inputs);
     // the copies on the auxiliary stream read the caller's memory: done before returning
     const cudaError_t e = wait_stream(c, c.aux);
     if (rc) return rc;
@@ -536,7 +548,7 @@ static int force_host(Context &c, double theta, const double *xs, const double *
     if ((rc = stage_split(c, {{S_XIN, xs, (size_t)n, &dx}, {S_YIN, ys, (size_t)n, &dy},
                               {S_X0, x0s, (size_t)nb, &d0x}, {S_Y0, y0s, (size_t)nb, &d0y},
                               {S_H, hs, (size_t)nb, &dh}},
-                          {{S_VIN, vs, (size_t)n, &dv}})) ||
+                          {{S_VIN, vs, (size_t)n, &dv}}, false)) ||
         (rc = ensure(c, S_OUTX, nt, &dox)) || (rc = ensure(c, S_OUTY, nt, &doy)))
         return drain_and_fail(c, rc);
     // the outputs come back run by run while later runs are evaluated (force_mrag)

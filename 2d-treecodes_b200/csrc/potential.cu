@@ -75,6 +75,7 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
     int *__restrict__ counts, const int *__restrict__ offs, int2 *__restrict__ lists,
     int2 *__restrict__ scratch, ScratchLayout sl, int *__restrict__ sstart, int *meta,
     unsigned *err, unsigned long long *stats, int seg) {
+    pdl_begin();
     constexpr bool FILL = MODE == 1;
     const int wglob = blockIdx.x * PT_WARPS + (threadIdx.x >> 5);
     int cur[2] = {0, 0};   // MODE 2: entries this warp has written, per kind
@@ -263,6 +264,7 @@ __global__ __launch_bounds__(256) void k_potential_lists_copy(int ngroups,
                                                               const int2 *__restrict__ scratch,
                                                               int2 *__restrict__ lists,
                                                               int *__restrict__ task_group) {
+    pdl_begin();
     const int lane = lane_id();
     const int *toff = offs + 2 * ngroups;
     const int tbase = toff[0];
@@ -333,6 +335,7 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval_mixed(
     const int *__restrict__ offs, const int2 *__restrict__ lists, double *__restrict__ out,
     double *__restrict__ partial, int *task_ctr, const int *__restrict__ task_group,
     const float2 *__restrict__ sexp, const float *__restrict__ sscale) {
+    pdl_begin();
     // E2P coefficients in pairs (D_2j.re, D_2j+1.re, D_2j.im, D_2j+1.im): the even and
     // the odd series run side by side in f32x2 lanes
     __shared__ float4 s_coef32[PE_WARPS][P / 2];
@@ -642,7 +645,8 @@ __global__ __launch_bounds__(PD_WARPS * 32, PD_MIN_BLOCKS) void k_potential_eval
     double *__restrict__ partial, int *task_ctr, const int *__restrict__ task_group, int seg) {
     extern __shared__ __align__(16) unsigned char eval_dyn[];
     double2 *s_tab = reinterpret_cast<double2 *>(eval_dyn);
-    load_near_log_table(s_tab);
+    load_near_log_table(s_tab);   // (a constant table: before the kernel before this one is done)
+    pdl_begin();
     const int lane = lane_id(), warp = threadIdx.x >> 5;
     const unsigned tab = shared_address(s_tab);
     const int copy = (lane & (NLOG_COPIES - 1)) * (int)sizeof(double2);
@@ -866,6 +870,7 @@ __global__ void k_potential_gather_parts(int ngroups, int m, const int *__restri
                                          const int *__restrict__ offs,
                                          const double *__restrict__ partial,
                                          double *__restrict__ out) {
+    pdl_begin();
     const int lane = lane_id();
     const int *toff = offs + 2 * ngroups;
     const int tbase = toff[0];
@@ -885,6 +890,7 @@ template <int P>
 __global__ void k_scale_coeffs_pot(int nnodes, const TNode *__restrict__ tnode,
                                    const double *__restrict__ exps, float2 *__restrict__ sexp,
                                    float *__restrict__ sscale) {
+    pdl_begin();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)nnodes * P;
          i += (long long)gridDim.x * blockDim.x) {
         const int node = (int)(i / P), k = (int)(i % P);
@@ -926,17 +932,18 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
     ListScratch ls;   // released (when transient) after the copy, in stream order
     int *sstart, *meta = c.ctrl.meta;
     unsigned long long *stats = c.ctrl.stats;
-    TC_CUDA_TRY(cudaEventRecord(c.ev_fork, c.stream));
+    const bool chain = c.launch_overlap && c.single;   // on one stream: launch_pdl
+    TC_CUDA_TRY(stream_after(c, c.aux, c.stream, c.ev_fork));
     {
         AuxScope on_aux(c);
-        TC_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.ev_fork, 0));
         if ((rc = sort_targets(c, xt, yt, m, &vo))) return rc;
         if ((rc = list_scratch(c, 2, nwarps, ngroups, sizeof(int2), sl, ls)) ||
             (rc = ensure(c, S_LSTART, (size_t)2 * ngroups, &sstart)))
             return rc;
-        k_potential_lists<2><<<grid, PT_WARPS * 32, 0, c.stream>>>(
-            ngroups, m, xt, yt, vo, theta, tnode, c.nnodes, counts, nullptr, nullptr,
-            static_cast<int2 *>(ls.p), sl, sstart, meta, err, stats, seg);
+        TC_CUDA_TRY(launch_pdl(c.launch_overlap, k_potential_lists<2>, grid, PT_WARPS * 32, 0,
+                               c.stream, ngroups, m, xt, yt, (const int *)vo, theta, tnode, c.nnodes,
+                               counts, (const int *)nullptr, (int2 *)nullptr,
+                               static_cast<int2 *>(ls.p), sl, sstart, meta, err, stats, seg));
         TC_KERNEL_CHECK();
         // the lists' totals and meta, written to h_pinned by the scan
         if ((rc = exclusive_scan(c, counts, offs, 3 * ngroups, ngroups, c.h_pinned + 32, meta)))
@@ -966,11 +973,11 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
             (rc = ensure(c, S_TASKMAP, (size_t)ntasks, &task_group)))
             return rc;
         if (!overflow) {
-            k_potential_lists_copy<<<(int)std::min<long long>((ngroups + 7) / 8,
-                                                              (long long)sm_count_p() * 16),
-                                     256, 0, c.stream>>>(ngroups, counts, offs, sstart,
-                                                         static_cast<const int2 *>(ls.p), lists,
-                                                         task_group);
+            TC_CUDA_TRY(launch_pdl(
+                chain, k_potential_lists_copy,
+                (int)std::min<long long>((ngroups + 7) / 8, (long long)sm_count_p() * 16), 256, 0,
+                c.stream, ngroups, (const int *)counts, (const int *)offs, (const int *)sstart,
+                static_cast<const int2 *>(ls.p), lists, task_group));
         } else {
             // the second walk adds the work counters again: clear the first walk's
             TC_CUDA_TRY(cudaMemsetAsync(stats + STAT_E2P_PAIRS, 0, 2 * sizeof(unsigned long long),
@@ -984,9 +991,9 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
                                 256, 0, c.stream>>>(ngroups, offs, task_group);
         }
         TC_KERNEL_CHECK();
-        TC_CUDA_TRY(cudaEventRecord(c.ev_join, c.stream));
+        TC_CUDA_TRY(mark_event(c, c.ev_join));
     }
-    TC_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.ev_join, 0));
+    TC_CUDA_TRY(await_event(c, c.ev_join));
     phase_mark(c, 4);
     int *task_ctr = c.ctrl.near_ctr;   // (cleared at the solve's start)
     double *partial;
@@ -1003,9 +1010,11 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
                 (rc2 = ensure(c, S_SSCALE, (size_t)c.nnodes, &sscale)))
                 return rc2;
             const long long items = (long long)c.nnodes * P;
-            k_scale_coeffs_pot<P>
-                <<<(int)std::min<long long>((items + 255) / 256, (long long)sm_count_p() * 8), 256, 0,
-                   c.stream>>>(c.nnodes, tnode, slot_ptr<double>(c, S_EXPS), sexp, sscale);
+            TC_CUDA_TRY(launch_pdl(
+                chain, k_scale_coeffs_pot<P>,
+                (int)std::min<long long>((items + 255) / 256, (long long)sm_count_p() * 8), 256, 0,
+                c.stream, c.nnodes, tnode, (const double *)slot_ptr<double>(c, S_EXPS), sexp,
+                sscale));
             TC_KERNEL_CHECK();
         }
         if (mixed) {
@@ -1013,11 +1022,14 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
             const int egrid = (int)std::min<long long>((ntasks + PE_WARPS - 1) / PE_WARPS,
                                                        (long long)sm_count_p() * occ);
             phase_mark(c, 6);
-            k_potential_eval_mixed<P><<<egrid, PE_WARPS * 32, 0, c.stream>>>(
-                ngroups, m, xt, yt, vo, tnode, slot_ptr<double>(c, S_MASS),
-                slot_ptr<int2>(c, S_RANGE), slot_ptr<double>(c, S_XS), slot_ptr<double>(c, S_YS),
-                slot_ptr<double>(c, S_VS), offs, lists, out, partial, task_ctr, task_group, sexp,
-                sscale);
+            TC_CUDA_TRY(launch_pdl(
+                chain, k_potential_eval_mixed<P>, egrid, PE_WARPS * 32, 0, c.stream, ngroups, m, xt,
+                yt, (const int *)vo, tnode, (const double *)slot_ptr<double>(c, S_MASS),
+                (const int2 *)slot_ptr<int2>(c, S_RANGE), (const double *)slot_ptr<double>(c, S_XS),
+                (const double *)slot_ptr<double>(c, S_YS),
+                (const double *)slot_ptr<double>(c, S_VS), (const int *)offs, (const int2 *)lists,
+                out, partial, task_ctr, (const int *)task_group, (const float2 *)sexp,
+                (const float *)sscale));
         } else {
             static const cudaError_t attr_rc =
                 cudaFuncSetAttribute(k_potential_eval<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1027,11 +1039,14 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
             const int egrid = (int)std::min<long long>((ntasks + PD_WARPS - 1) / PD_WARPS,
                                                        (long long)sm_count_p() * occ);
             phase_mark(c, 6);
-            k_potential_eval<P><<<egrid, PD_WARPS * 32, eval_smem<P>(), c.stream>>>(
-                ngroups, m, xt, yt, vo, tnode, slot_ptr<double>(c, S_MASS),
-                slot_ptr<double>(c, S_EXPS), slot_ptr<int2>(c, S_RANGE), slot_ptr<double>(c, S_XS),
-                slot_ptr<double>(c, S_YS), slot_ptr<double>(c, S_VS), offs, lists, out, partial,
-                task_ctr, task_group, seg);
+            TC_CUDA_TRY(launch_pdl(
+                chain, k_potential_eval<P>, egrid, PD_WARPS * 32, eval_smem<P>(), c.stream, ngroups,
+                m, xt, yt, (const int *)vo, tnode, (const double *)slot_ptr<double>(c, S_MASS),
+                (const double *)slot_ptr<double>(c, S_EXPS),
+                (const int2 *)slot_ptr<int2>(c, S_RANGE), (const double *)slot_ptr<double>(c, S_XS),
+                (const double *)slot_ptr<double>(c, S_YS),
+                (const double *)slot_ptr<double>(c, S_VS), (const int *)offs, (const int2 *)lists,
+                out, partial, task_ctr, (const int *)task_group, seg));
         }
         TC_KERNEL_CHECK();
         return TC_OK;
@@ -1039,8 +1054,10 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
     if (rc) return rc;
     phase_mark(c, 7);
     if (ntasks > ngroups) {
-        k_potential_gather_parts<<<(int)std::min<long long>((ngroups + 7) / 8, (long long)sm_count_p() * 16),
-                                   256, 0, c.stream>>>(ngroups, m, vo, offs, partial, out);
+        TC_CUDA_TRY(launch_pdl(
+            c.launch_overlap, k_potential_gather_parts,
+            (int)std::min<long long>((ngroups + 7) / 8, (long long)sm_count_p() * 16), 256, 0,
+            c.stream, ngroups, m, (const int *)vo, (const int *)offs, (const double *)partial, out));
         TC_KERNEL_CHECK();
     }
     return TC_OK;

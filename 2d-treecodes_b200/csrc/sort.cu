@@ -915,6 +915,7 @@ __global__ __launch_bounds__(SMALL_THREADS) void k_sort_small_targets(
     extern __shared__ __align__(16) unsigned long long small_dyn[];
     unsigned long long *s_items = small_dyn;
     int *s_hist = reinterpret_cast<int *>(s_items + SMALL_THREADS * ITEMS);
+    pdl_begin();
     const int lane = lane_id(), warp = threadIdx.x >> 5;
     const Frame f = *frame;
     unsigned long long item[ITEMS];
@@ -947,8 +948,9 @@ static int sort_small_targets(Context &c, const double *x, const double *y, int 
         cudaFuncSetAttribute(k_sort_small_targets<ITEMS>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem<ITEMS>());
     TC_CUDA_TRY(attr_rc);
-    k_sort_small_targets<ITEMS><<<1, SMALL_THREADS, small_smem<ITEMS>(), c.stream>>>(
-        x, y, n, slot_ptr<Frame>(c, S_FRAME), perm);
+    TC_CUDA_TRY(launch_pdl(c.launch_overlap && c.single, k_sort_small_targets<ITEMS>, 1,
+                           SMALL_THREADS, small_smem<ITEMS>(), c.stream, x, y, n,
+                           (const Frame *)slot_ptr<Frame>(c, S_FRAME), perm));
     TC_KERNEL_CHECK();
     return TC_OK;
 }

@@ -370,7 +370,11 @@ __global__ __launch_bounds__(256) void k_moments_level(int l, LevelOffsets lo, i
 }
 
 // levels ltop .. 0 in one block, a block barrier between levels
-__global__ __launch_bounds__(1024) void k_moments_top(int ltop, LevelOffsets lo, int nnodes,
+// Levels with at most this many inner nodes: one block.  With 1024 the single SM's share of the
+// L2 bandwidth bound it (28 words a node: 43 us on the 16M sheet); at 64 the wide levels get
+// launches of their own: the upward phase of a 300K-source solve 127 -> 102 us.
+constexpr int MOM_TOP_MAX = 64;
+__global__ __launch_bounds__(MOM_TOP_MAX) void k_moments_top(int ltop, LevelOffsets lo, int nnodes,
                                                       const int4 *__restrict__ cell, TNode *tnode,
                                                       double *mass, double *wgt, double *wxs,
                                                       double *wys, const Frame *__restrict__ frame,
@@ -677,10 +681,6 @@ static LevelOffsets level_offsets(const Context &c) {
     return offs;
 }
 
-// Levels with at most this many inner nodes: one block.  With 1024 the single SM's share of the
-// L2 bandwidth bound it (28 words a node: 43 us on the 16M sheet); at 64 the wide levels get
-// launches of their own: the upward phase of a 300K-source solve 127 -> 102 us.
-constexpr int MOM_TOP_MAX = 64;
 
 int upward_moments(Context &c) {
     const bool ovl = c.launch_overlap;   // launch_pdl chains (tc_set_launch_overlap)
@@ -692,21 +692,24 @@ int upward_moments(Context &c) {
     unsigned *err = c.ctrl.err;
     double *mass = slot_ptr<double>(c, S_MASS), *w = slot_ptr<double>(c, S_W),
            *wx = slot_ptr<double>(c, S_WX), *wy = slot_ptr<double>(c, S_WY);
-    k_leaf_setup<<<(int)(((long long)nn * 4 + 255) / 256), 256, 0, c.stream>>>(
-        nn, c.nsrc, c.leafcap, slot_ptr<double>(c, S_XS), slot_ptr<double>(c, S_YS),
-        slot_ptr<double>(c, S_VS), range, cell, tnode, mass, w, wx, wy, frame, err);
+    TC_CUDA_TRY(launch_pdl(ovl, k_leaf_setup, (int)(((long long)nn * 4 + 255) / 256), 256, 0,
+                           c.stream, nn, c.nsrc, c.leafcap,
+                           (const double *)slot_ptr<double>(c, S_XS),
+                           (const double *)slot_ptr<double>(c, S_YS),
+                           (const double *)slot_ptr<double>(c, S_VS), range, cell, tnode, mass, w,
+                           wx, wy, frame, err));
     TC_KERNEL_CHECK();
     // The parent moments run on the auxiliary stream, beside the leaves' P2E on the main one
     // (P2E reads only the leaves' own moments; the E2E waits for ev_moments, and anything
     // queued later on the auxiliary stream, such as the interaction lists, follows them).
-    TC_CUDA_TRY(cudaEventRecord(c.ev_leafset, c.stream));
+    TC_CUDA_TRY(stream_after(c, c.aux, c.stream, c.ev_leafset));
     AuxScope on_aux(c);
-    TC_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.ev_leafset, 0));
     // inner nodes exist on levels 0 .. LMAX-1, deepest first
     const LevelOffsets offs = level_offsets(c);
     const int ltop = small_top(c, MOM_TOP_MAX);
-    // the first launch follows the event wait; each later one follows a kernel (launch_pdl)
-    bool after_kernel = false;
+    // the first launch follows the event wait (on one stream: the leaves' kernel); each later one
+    // follows a kernel (launch_pdl)
+    bool after_kernel = c.single;
     for (int l = LMAX - 1; l > ltop; --l) {
         const int ninner = (c.level_off[l + 2] - c.level_off[l + 1]) / 4;
         if (ninner <= 0) continue;
@@ -729,7 +732,7 @@ int upward_moments(Context &c) {
                                                            wx, wy, frame, err);
         TC_KERNEL_CHECK();
     }
-    TC_CUDA_TRY(cudaEventRecord(c.ev_moments, c.stream));
+    TC_CUDA_TRY(mark_event(c, c.ev_moments));
     return TC_OK;
 }
 
@@ -761,17 +764,17 @@ static int run_expansions(Context &c) {
                           : blocks_per_sm<k_leaf_p2e<P, false>>(UP_WARPS * 32, smem64);
     const int grid = (int)std::min<long long>((nn + UP_WARPS - 1) / UP_WARPS, (long long)sms * occ);
     auto p2e = mixed ? k_leaf_p2e<P, true> : k_leaf_p2e<P, false>;
-    p2e<<<grid, UP_WARPS * 32, smem, c.stream>>>(nn, c.nsrc, c.leafcap, xs, ys, vs, range, cell,
-                                                 tnode, exps, frame);
+    TC_CUDA_TRY(launch_pdl(ovl, p2e, grid, UP_WARPS * 32, smem, c.stream, nn, c.nsrc, c.leafcap,
+                           xs, ys, vs, range, cell, tnode, exps, frame));
     TC_KERNEL_CHECK();
     // the parents' moments (expansion centres) come from the auxiliary stream
-    TC_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.ev_moments, 0));
+    TC_CUDA_TRY(await_event(c, c.ev_moments));
     // E2E deepest level first: wide levels thread per node, narrow ones warp per node, the
     // small top levels in one single-block launch
     const LevelOffsets offs = level_offsets(c);
     const int ltop = small_top(c, UP_TOP_MAX_NODES);
     // the first launch follows the event wait; each later one follows a kernel (launch_pdl)
-    bool after_kernel = false;
+    bool after_kernel = c.single;
     for (int l = LMAX - 1; l > ltop; --l) {
         const int ninner = (c.level_off[l + 2] - c.level_off[l + 1]) / 4;
         if (ninner <= 0) continue;
