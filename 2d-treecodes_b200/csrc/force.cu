@@ -1298,21 +1298,21 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
             TC_KERNEL_CHECK();
             return TC_OK;
         };
-        // With host outputs of 2^21 targets or more (a copy of >= 32 MB, ~0.6 ms over PCIe) the
-        // blocks are evaluated in FORCE_CHUNKS runs, each copied to the host on the auxiliary
-        // stream while the next one is evaluated; below that the runs' tails cost more than
-        // the overlap gains (measured: 16M sheet e2e 11.07 -> 10.67 ms, 1M vortex 2.01 ->
-        // 2.27 ms if split).
+        // Large host outputs: the blocks are evaluated in runs, each copied to the host on the
+        // auxiliary stream while the next one is evaluated.  Four runs from 2^21 targets on (a
+        // copy of >= 32 MB, ~0.6 ms over PCIe: 16M sheet e2e 11.07 -> 10.67 ms), two from 2^19 on
+        // (1M targets: 1347 -> 1318 us; four took 1412, the runs' tails costing more than
+        // the overlap gains).
         const size_t per_block = (size_t)1 << (2 * L.lbs);
         const size_t nt_all = (size_t)nblocks * per_block;
         double *xfar, *yfar;
         int *far_ctr = c.ctrl.far_ctr;
         if ((rc2 = ensure(c, S_FARX, nt_all, &xfar)) || (rc2 = ensure(c, S_FARY, nt_all, &yfar)))
             return rc2;
-        const int nchunks =
-            host_x && (size_t)nblocks * per_block >= ((size_t)1 << 21) && nblocks >= FORCE_CHUNKS
-                ? FORCE_CHUNKS
-                : 1;
+        const int nchunks = !host_x || nblocks < FORCE_CHUNKS ? 1
+                            : nt_all >= ((size_t)1 << 21)     ? FORCE_CHUNKS
+                            : nt_all >= ((size_t)1 << 19)     ? 2
+                                                              : 1;
         for (int k = 0; k < nchunks; ++k) {
             const int blk0 = (int)((long long)nblocks * k / nchunks);
             const int blk1 = (int)((long long)nblocks * (k + 1) / nchunks);
@@ -1327,14 +1327,17 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
                                                  (long long)sm_count() * 8),
                         256, 0, c.stream>>>(xout, yout, xfar, yfar, o, cnt);
             TC_KERNEL_CHECK();
-            if (nchunks > 1) {
-                TC_CUDA_TRY(cudaEventRecord(c.ev_chunk[k], c.stream));
-                TC_CUDA_TRY(cudaStreamWaitEvent(c.aux, c.ev_chunk[k], 0));
-                TC_CUDA_TRY(cudaMemcpyAsync(host_x + o, xout + o, sizeof(double) * cnt,
-                                            cudaMemcpyDeviceToHost, c.aux));
-                TC_CUDA_TRY(cudaMemcpyAsync(host_y + o, yout + o, sizeof(double) * cnt,
-                                            cudaMemcpyDeviceToHost, c.aux));
-            }
+            if (nchunks > 1) TC_CUDA_TRY(cudaEventRecord(c.ev_chunk[k], c.stream));
+        }
+        // the copies after every run's launches: a copy to pageable memory holds the host up
+        for (int k = 0; nchunks > 1 && k < nchunks; ++k) {
+            const size_t o = (size_t)((long long)nblocks * k / nchunks) * per_block;
+            const size_t e = (size_t)((long long)nblocks * (k + 1) / nchunks) * per_block;
+            TC_CUDA_TRY(cudaStreamWaitEvent(c.aux, c.ev_chunk[k], 0));
+            TC_CUDA_TRY(cudaMemcpyAsync(host_x + o, xout + o, sizeof(double) * (e - o),
+                                        cudaMemcpyDeviceToHost, c.aux));
+            TC_CUDA_TRY(cudaMemcpyAsync(host_y + o, yout + o, sizeof(double) * (e - o),
+                                        cudaMemcpyDeviceToHost, c.aux));
         }
         c.host_copied = nchunks > 1;
         return TC_OK;
