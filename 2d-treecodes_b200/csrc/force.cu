@@ -77,11 +77,23 @@ __device__ __forceinline__ Brick brick_geometry(double x0, double y0, double h, 
 
 enum { K_E2L = 0, K_E2P = 1, K_P2P = 2, K_DESCEND = 3, K_SKIP = 4 };
 
+// The E2L test, dist / r - 1 > 1 / theta, needs a square root and a division, most of the walk's
+// instructions.  It is decided on the squares, d^2 against (r (1 + 1 / theta))^2, when they differ by
+// more than 1e-12 of themselves, far above every rounding involved, and t is positive with a square
+// well inside the normal range; otherwise as the reference computes it.  Lists of the 16M sheet's
+// 65,536 bricks 130 -> 86 us.
 __device__ __forceinline__ int classify(const TNode &nd, const Brick &b, double inv_theta,
                                         double theta2) {
     const double dx = __dsub_rn(b.x0b, nd.xcom), dy = __dsub_rn(b.y0b, nd.ycom);
-    const double dist = __dsqrt_rn(__fma_rn(dx, dx, __dmul_rn(dy, dy)));
-    if (__dsub_rn(__ddiv_rn(dist, nd.r), 1.0) > inv_theta && b.rbrick <= nd.r) return K_E2L;
+    if (b.rbrick <= nd.r) {
+        const double d2 = __fma_rn(dx, dx, __dmul_rn(dy, dy));
+        const double t = nd.r * (1.0 + inv_theta), t2 = t * t;
+        bool e2l;
+        if (t > 1e-140 && d2 > t2 * (1.0 + 1e-12)) e2l = true;
+        else if (t > 1e-140 && d2 < t2 * (1.0 - 1e-12)) e2l = false;
+        else e2l = __dsub_rn(__ddiv_rn(__dsqrt_rn(d2), nd.r), 1.0) > inv_theta;
+        if (e2l) return K_E2L;
+    }
     const double xt = fmax(b.xlo, fmin(b.xhi, nd.xcom));
     const double yt = fmax(b.ylo, fmin(b.yhi, nd.ycom));
     const double ex = __dsub_rn(xt, nd.xcom), ey = __dsub_rn(yt, nd.ycom);
