@@ -147,6 +147,8 @@ size_t footprint_estimate(int kind, long long n, long long ntargets, long long n
         b += (size_t)ntargets * 210;
         // FP64: with few target groups the near field runs in more tasks, 256 B each
         if (!precision) b += (size_t)std::min(ntargets, 1ll << 19) * 256;
+        // FP64: the common far fields of sets of 128 targets (two lists, 32 coefficients)
+        if (!precision) b += (size_t)ntargets * 18;
     }
     return b + (4u << 20);
 }

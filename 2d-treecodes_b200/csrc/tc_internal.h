@@ -39,6 +39,7 @@ enum Slot {
     S_LSTART, S_FARX, S_FARY, S_LOCAL,
     // potential targets / lists
     S_TKEYS, S_TPERM, S_TKEYS2, S_TPERM2, S_PCOUNT, S_POFF, S_PE2P,
+    S_SETLIST, S_SETNUM, S_SETGEO, S_SETLOCAL,
     S_NUM_SLOTS
 };
 

@@ -68,3 +68,39 @@ def test_force_of_a_subset_equals_the_whole(precision, side):
     # (the mixed form's tiles and FP32 sums are the same; its compensated sums add in FP64)
     for a, b in zip(part, whole):
         assert rel(a, b[:1024 * nb]) < (TOL if precision == 0 else 1e-9)
+
+
+@pytest.mark.parametrize("theta,order", [(0.3, 12), (0.5, 12), (0.7, 8), (0.5, 28), (1.0, 4)])
+def test_common_far_fields_equal_the_groups_own(theta, order):
+    """FP64 targets enough for sets with a common far field (262,144) against the same targets in
+    solves too small for them: spread and clustered, some of them far outside the sources, some
+    coincident (sets of one point), and one at infinity, which must not reach its neighbours.  The
+    local expansions leave out 1e-17 of a cell's weight; FP64 sums are regrouped."""
+    import torch
+    import treecodes as T
+
+    d = lambda a: torch.tensor(a, device="cuda")
+    xs, ys, vs = map(d, clustered(30011, 6))
+    r = np.random.default_rng(9)
+    m = 270001
+    x, y, _ = clustered(m, 10)
+    x[:20000] = 3 * x[:20000] - 1
+    x[20000:20200] = x[20000]
+    y[20000:20200] = y[20000]
+    x[30000] = np.inf
+    p = r.permutation(m)
+    xt, yt = d(x[p]), d(y[p])
+    ctx = T.Context()
+    ctx.set_orders(potential_order=order)
+    whole = torch.empty(m, device="cuda", dtype=torch.float64)
+    torch.cuda.synchronize()
+    ctx.potential_device(theta, xs, ys, vs, xt, yt, whole)
+    part = torch.empty_like(whole)
+    for a in range(0, m, 90000):
+        o = torch.empty(min(90000, m - a), device="cuda", dtype=torch.float64)
+        torch.cuda.synchronize()
+        ctx.potential_device(theta, xs, ys, vs, xt[a:a + 90000].clone(), yt[a:a + 90000].clone(), o)
+        part[a:a + 90000] = o
+    fin = torch.isfinite(xt)
+    assert bool(torch.isfinite(whole[fin]).all())
+    assert rel(whole[fin], part[fin]) < TOL
