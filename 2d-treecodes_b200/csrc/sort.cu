@@ -693,7 +693,7 @@ __global__ __launch_bounds__(GS_THREADS) void k_gather_sources(
 #pragma unroll
         for (int k = 0; k < GS_ITEMS; ++k) {
             const int i = base + k * GS_THREADS;
-            it[k] = i < n ? items[i] : 0ull;
+            it[k] = i < n ? __ldcs(items + i) : 0ull;
         }
 #pragma unroll
         for (int k = 0; k < GS_ITEMS; ++k) {
@@ -709,11 +709,11 @@ __global__ __launch_bounds__(GS_THREADS) void k_gather_sources(
                 atomicOr(err, DEVERR_BOUNDS);
                 continue;
             }
-            keys[i] = (int)(it[k] >> 32);
-            perm[i] = (int)__double_as_longlong(b[k].y);
-            xs[i] = a[k].x;
-            ys[i] = a[k].y;
-            vs[i] = b[k].x;
+            __stcs(keys + i, (int)(it[k] >> 32));
+            __stcs(perm + i, (int)__double_as_longlong(b[k].y));
+            __stcs(xs + i, a[k].x);
+            __stcs(ys + i, a[k].y);
+            __stcs(vs + i, b[k].x);
         }
     }
 }
@@ -1285,10 +1285,12 @@ int sort_sources(Context &c, const double *x, const double *y, const double *v, 
         c.late_ready = values_ready;
         return TC_OK;
     }
-    // a window of the sorted order in flight at a time (4 CTAs per SM): its records come from
-    // a compact range of buckets, which stays in L2.  One 32-byte load per record instead of two
-    // of 16 bytes: the random loads are bound by the L1 tag lookups (300 -> 265 us, 16M sheet)
-    TC_CUDA_TRY(launch_pdl(ovl, k_gather_sources, grid_for(n, GS_THREADS * GS_ITEMS, 4),
+    // a window of the sorted order in flight at a time: its records come from a compact range of
+    // buckets, which stays in L2.  The grid is what is resident (2 CTAs per SM): with twice that,
+    // half of the stripes ran after the others, and the buckets were read twice (16M sheet, sort
+    // phase 1163 -> 1110 us; 1, 3 CTAs or half-size batches: 1190-1240).  One 32-byte load per
+    // record instead of two of 16 bytes: the random loads are bound by the L1 tag lookups
+    TC_CUDA_TRY(launch_pdl(ovl, k_gather_sources, grid_for(n, GS_THREADS * GS_ITEMS, 2),
                            GS_THREADS, 0, c.stream, (const unsigned long long *)items_a,
                            (const double2 *)rec, n, keys, perm, xs, ys, vs, err));
     TC_KERNEL_CHECK();
