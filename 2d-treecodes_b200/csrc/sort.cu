@@ -532,12 +532,12 @@ __global__ __launch_bounds__(PS_THREADS, FIRST ? 3 : 4) void k_onesweep_items(
 
     unsigned long long item[PS_ITEMS];
     int rank[PS_ITEMS];
+    constexpr int FB = 4;   // the first pass's loads in flight
+    static_assert(PS_ITEMS % FB == 0, "whole batches");
     if constexpr (FIRST) {
-        // keys and each source's slot among the tile's sources of its bucket; the loads are
-        // issued in batches of FB before the shared atomics that consume them
+        // keys, digit counts and each source's slot among the tile's sources of its bucket; the
+        // loads are issued in batches of FB before the shared atomics that consume them
         const Frame f = *fp.frame;
-        constexpr int FB = 4;
-        static_assert(PS_ITEMS % FB == 0, "whole batches");
 #pragma unroll
         for (int k0 = 0; k0 < PS_ITEMS; k0 += FB) {
             double xv[FB], yv[FB];
@@ -554,16 +554,48 @@ __global__ __launch_bounds__(PS_THREADS, FIRST ? 3 : 4) void k_onesweep_items(
                 if (idx < n) {
                     key = morton_key(xv[k], yv[k], f);
                     slot = atomicAdd(&s_global[(unsigned)key >> BUCKET_SHIFT], 1);
+                    atomicAdd(&s_count[(key >> (shift - 32)) & 0xFF], 1);
                 }
                 item[k0 + k] = ((unsigned long long)(unsigned)key << 32) | (unsigned)slot;
             }
         }
-        __syncthreads();
-        // the tile's slots in each bucket, one global claim per bucket
-        {
-            const int c = s_global[tid];
-            if (c) s_tile_start[tid] = fp.bucket_off[tid] + atomicAdd(&fp.bucket_fill[tid], c);
+    } else {
+#pragma unroll
+        for (int k = 0; k < PS_ITEMS; ++k) {
+            const int idx = warp_base + k * 32 + lane;
+            item[k] = idx < n ? in[idx] : 0ull;
         }
+#pragma unroll
+        for (int k = 0; k < PS_ITEMS; ++k)
+            if (warp_base + k * 32 + lane < n)
+                atomicAdd(&s_count[(int)(item[k] >> shift) & 0xFF], 1);
+    }
+    // Early counts: the tile's digit totals first (shared atomics), so that its aggregate is
+    // published and the look-back done before the ranking (and the first pass's records), not
+    // after it: the tiles behind wait for it.  (The first pass with its look-back after the
+    // records and the bucket claims: 341 us on the 16M sheet, so ~285.)
+    const int d = tid;   // one digit per thread
+    __syncthreads();
+    const int total = s_count[d];
+    int bucket_base = 0;
+    if constexpr (FIRST) {
+        // the tile's slots in each bucket, one global claim per bucket (used after the look-back)
+        const int c = s_global[tid];
+        if (c) bucket_base = fp.bucket_off[tid] + atomicAdd(&fp.bucket_fill[tid], c);
+    }
+    // tile == stall_tile (a test setting): this tile publishes into `sink`, which no look-back
+    // reads, so the tiles after it wait until spin_limit
+    unsigned *mine = (STALL && tile == stall_tile ? sink : status + (size_t)tile * RS_RADIX) + d;
+    int excl = 0;
+    if (tile == 0) {
+        atomicExch(mine, RS_FLAG_INC | (unsigned)total);
+    } else {
+        atomicExch(mine, RS_FLAG_AGG | (unsigned)total);
+        excl = lookback(status, tile, d, err, spin_limit);
+        atomicExch(mine, RS_FLAG_INC | (unsigned)(excl + total));
+    }
+    if constexpr (FIRST) {
+        s_tile_start[tid] = bucket_base;
         __syncthreads();
         // each record with one 32-byte store (one whole DRAM sector), batches of FB loads first
 #pragma unroll
@@ -591,32 +623,6 @@ __global__ __launch_bounds__(PS_THREADS, FIRST ? 3 : 4) void k_onesweep_items(
                 item[k0 + k] = ((unsigned long long)key << 32) | (unsigned)pos;
             }
         }
-        __syncthreads();   // s_tile_start is reused below
-    } else {
-#pragma unroll
-        for (int k = 0; k < PS_ITEMS; ++k) {
-            const int idx = warp_base + k * 32 + lane;
-            item[k] = idx < n ? in[idx] : 0ull;
-        }
-    }
-    // Early counts: the tile's digit totals first (shared atomics), so that its aggregate is
-    // published and the look-back done before the ranking, not after it.
-    const int d = tid;   // one digit per thread
-#pragma unroll
-    for (int k = 0; k < PS_ITEMS; ++k)
-        if (warp_base + k * 32 + lane < n) atomicAdd(&s_count[(int)(item[k] >> shift) & 0xFF], 1);
-    __syncthreads();
-    const int total = s_count[d];
-    // tile == stall_tile (a test setting): this tile publishes into `sink`, which no look-back
-    // reads, so the tiles after it wait until spin_limit
-    unsigned *mine = (STALL && tile == stall_tile ? sink : status + (size_t)tile * RS_RADIX) + d;
-    int excl = 0;
-    if (tile == 0) {
-        atomicExch(mine, RS_FLAG_INC | (unsigned)total);
-    } else {
-        atomicExch(mine, RS_FLAG_AGG | (unsigned)total);
-        excl = lookback(status, tile, d, err, spin_limit);
-        atomicExch(mine, RS_FLAG_INC | (unsigned)(excl + total));
     }
 
     const unsigned lt = lanemask_lt();
