@@ -224,15 +224,15 @@ __global__ __launch_bounds__(TR_WARPS * 32) void k_force_lists(
     }
 }
 
-// The lists in CSR order from the scratch runs of k_force_lists<2>, and the task -> brick map:
-// warp per brick.
+// The lists in CSR order from the scratch runs of k_force_lists<2>, and (tasks not null) the
+// near-field tasks in order: warp per brick.
 __global__ __launch_bounds__(256) void k_force_lists_copy(int nbricks,
                                                           const int *__restrict__ counts,
                                                           const int *__restrict__ offs,
                                                           const int *__restrict__ sstart,
                                                           const int *__restrict__ scratch,
                                                           int *__restrict__ lists,
-                                                          int *__restrict__ task_brick) {
+                                                          int2 *__restrict__ tasks) {
     const int lane = lane_id();
     const int *toff = offs + 3 * nbricks;
     const int tbase = toff[0];
@@ -244,7 +244,9 @@ __global__ __launch_bounds__(256) void k_force_lists_copy(int nbricks,
             int *dst = lists + offs[k * nbricks + brick];
             for (int i = lane; i < n; i += 32) dst[i] = src[i];
         }
-        for (int t = toff[brick] + lane; t < toff[brick + 1]; t += 32) task_brick[t - tbase] = brick;
+        if (tasks)
+            for (int t = toff[brick] + lane; t < toff[brick + 1]; t += 32)
+                tasks[t - tbase] = make_int2(t - tbase, brick);
     }
 }
 
@@ -528,6 +530,29 @@ __global__ __launch_bounds__(EV_WARPS * 32, MIXED ? 6 : 4) void k_force_e2l(
     }
 }
 
+// The bricks [lo, lo + n) in bins of falling far-field work (list entries), for the persistent warps
+// of k_force_far<.., 1>: bricks on dense regions have hundreds of cells, most have a few, and in
+// index order the last ones taken kept the kernel running (see TaskBins; 16M sheet, the far field
+// alone, FP64 869 -> 761 us, mixed 571 -> 533).  A lane per brick, one atomic per warp and bin.
+__global__ __launch_bounds__(256) void k_far_order(int nbricks, int lo, int n,
+                                                   const int *__restrict__ counts, int *fill,
+                                                   int *__restrict__ order) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, brick = lo + i;
+    const bool valid = i < n;
+    int bin = TASK_BINS;
+    if (valid) {
+        // bins of 0-7, 8-15, 16-31, .. entries, the longest first
+        const int work = counts[brick] + counts[nbricks + brick];
+        bin = TASK_BINS - 1 - min(TASK_BINS - 1, 29 - __clz(work | 4));
+    }
+    const unsigned peers = __match_any_sync(FULL_MASK, bin);
+    const int leader = __ffs(peers) - 1;
+    int at = 0;
+    if (valid && lane_id() == leader) at = atomicAdd(&fill[bin], __popc(peers));
+    at = __shfl_sync(FULL_MASK, at, leader) + __popc(peers & lanemask_lt());
+    if (valid && at < n) order[(size_t)bin * n + at] = brick;
+}
+
 // The far field of every brick: E2L, L2P and E2P, two targets per lane.
 // MIXED = false: plain FP64.  MIXED = true: E2L, L2P and E2P in FP32 on power-of-two scaled
 // quantities (scaled multipole coefficients, scaled local coefficients, offsets over the
@@ -548,7 +573,8 @@ __global__ __launch_bounds__(EV_WARPS * 32, WPB > 1 ? (MIXED ? 8 : 5) : (MIXED ?
     const int *__restrict__ offs, const int *__restrict__ lists, double *__restrict__ xout,
     double *__restrict__ yout, int brick_lo, int brick_hi, int *brick_ctr,
     const float2 *__restrict__ sexp, const float *__restrict__ sscale,
-    const local_t<MIXED> *__restrict__ local) {
+    const local_t<MIXED> *__restrict__ local, const int *__restrict__ order,
+    const int *__restrict__ fill) {
     const BlockLayout L = LBS ? BlockLayout{LBS, LBS - 3} : L_arg;
     constexpr bool SHARED_BRICK = WPB > 1;
     using binom_t = typename std::conditional<SHARED_BRICK, char, SignedBinomials<P, MIXED>>::type;
@@ -563,6 +589,7 @@ __global__ __launch_bounds__(EV_WARPS * 32, WPB > 1 ? (MIXED ? 8 : 5) : (MIXED ?
     FarShared<P, MIXED> &sh = shared[warp].far;
     const int tx = lane & 7, ty = lane >> 3;   // targets (tx, ty) and (tx, ty + 4)
     [[maybe_unused]] const binom_t bin{};
+    [[maybe_unused]] const TaskBins bins(SHARED_BRICK ? nullptr : fill);
 
     for (;;) {
         int brick = 0;
@@ -575,6 +602,10 @@ __global__ __launch_bounds__(EV_WARPS * 32, WPB > 1 ? (MIXED ? 8 : 5) : (MIXED ?
             brick = __shfl_sync(FULL_MASK, brick, 0);
         }
         if (brick < brick_lo || brick >= brick_hi) break;   // (a counter not reset: no access)
+        if (!SHARED_BRICK && order) {
+            brick = order[bins.place(brick - brick_lo, brick_hi - brick_lo)];
+            if ((unsigned)brick >= (unsigned)nbricks) break;
+        }
         const int part = SHARED_BRICK ? warp : 0;
         int blk, bx, by;
         brick_of(L, brick, blk, bx, by);
@@ -797,8 +828,8 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
     const double *__restrict__ hs, const int2 *__restrict__ range, const double *__restrict__ xs,
     const double *__restrict__ ys, const double *__restrict__ vs, const int *__restrict__ offs,
     const int *__restrict__ lists, double *__restrict__ xout, double *__restrict__ yout,
-    double *__restrict__ partial, int brick_lo, int brick_hi, int *task_ctr,
-    const int *__restrict__ task_brick, int seg) {
+    double *__restrict__ partial, int *task_ctr,
+    const int2 *__restrict__ tasks, const int *__restrict__ fill, int seg) {
     const BlockLayout L = LBS ? BlockLayout{LBS, LBS - 3} : L_arg;
     __shared__ NearShared<MIXED> shared[EV_WARPS];
     const int lane = lane_id(), warp = threadIdx.x >> 5;
@@ -807,17 +838,20 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
     const double eps = 10 * DBL_EPSILON;
 
     // Tasks: brick b owns tasks [toff[b], toff[b+1]) (relative to toff[0]); task p covers the
-    // tiles that start in sources [p * seg, (p + 1) * seg) of the brick's P2P sequence.  This
-    // launch evaluates the tasks of bricks [brick_lo, brick_hi).
+    // tiles that start in sources [p * seg, (p + 1) * seg) of the brick's P2P sequence.
     const int *toff = offs + 3 * nbricks;
     const int tbase = toff[0];
-    const int task_lo = toff[brick_lo] - tbase, task_hi = toff[brick_hi] - tbase;
+    const int ntasks = toff[nbricks] - tbase;
+    const TaskBins bins(fill);
     for (;;) {
         int task = 0;
-        if (lane == 0) task = task_lo + atomicAdd(task_ctr, 1);
+        if (lane == 0) task = atomicAdd(task_ctr, 1);
         task = __shfl_sync(FULL_MASK, task, 0);
-        if (task < task_lo || task >= task_hi) break;
-        const int brick = task_brick[task];
+        if ((unsigned)task >= (unsigned)ntasks) break;
+        const int2 entry = tasks[fill ? bins.place(task, ntasks) : task];
+        task = entry.x;
+        const int brick = entry.y;
+        if ((unsigned)task >= (unsigned)ntasks || (unsigned)brick >= (unsigned)nbricks) break;
         const int part = task - (toff[brick] - tbase);
         const int nparts = toff[brick + 1] - toff[brick];
         const int beg = offs[2 * nbricks + brick], end = offs[2 * nbricks + brick + 1];
@@ -1039,13 +1073,35 @@ __global__ __launch_bounds__(256) void k_add_far(double *__restrict__ xout,
     }
 }
 
-// task -> brick map of the evaluation tasks (when a second walk wrote the lists)
-__global__ void k_task_map(int nbricks, const int *__restrict__ offs, int *__restrict__ task_brick) {
+// The near-field tasks as (task, brick), in bins of falling work (TaskBins): whole segments first,
+// then the bricks' last tasks by an estimate of their length (64 sources a leaf; half a segment
+// after a whole one).  A lane per brick.
+__global__ __launch_bounds__(256) void k_near_order(int nbricks, int ntasks, int seg,
+                                                    const int *__restrict__ offs, int *fill,
+                                                    int2 *__restrict__ tasks) {
+    const int brick = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = brick < nbricks;
     const int *toff = offs + 3 * nbricks;
-    const int tbase = toff[0];
-    for (int brick = blockIdx.x * blockDim.x + threadIdx.x; brick < nbricks;
-         brick += gridDim.x * blockDim.x)
-        for (int t = toff[brick]; t < toff[brick + 1]; ++t) task_brick[t - tbase] = brick;
+    int bin = TASK_BINS, t1 = 0;
+    if (valid) {
+        const int t0 = toff[brick] - toff[0];
+        t1 = toff[brick + 1] - toff[0] - 1;
+        if (t1 > t0) {
+            const int at = atomicAdd(&fill[0], t1 - t0);
+            for (int t = t0; t < t1; ++t)
+                if ((unsigned)(at + t - t0) < (unsigned)ntasks)
+                    tasks[at + t - t0] = make_int2(t, brick);
+        }
+        const int leaves = offs[2 * nbricks + brick + 1] - offs[2 * nbricks + brick];
+        const int work = t1 > t0 ? seg / 2 : min(seg, 64 * leaves);
+        bin = TASK_BINS - 1 - min(TASK_BINS - 2, work * (TASK_BINS - 1) / seg);
+    }
+    const unsigned peers = __match_any_sync(FULL_MASK, bin);
+    const int leader = __ffs(peers) - 1;
+    int at = 0;
+    if (valid && lane_id() == leader) at = atomicAdd(&fill[bin], __popc(peers));
+    at = __shfl_sync(FULL_MASK, at, leader) + __popc(peers & lanemask_lt());
+    if (valid && at < ntasks) tasks[(size_t)bin * ntasks + at] = make_int2(t1, brick);
 }
 
 // Mixed form: multipole coefficients scaled by the cell's power-of-two radius R >= r,
@@ -1173,28 +1229,35 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
     c.counts.e2l_pairs = c.counts.n_e2l;
     c.counts.e2p_pairs = c.counts.n_e2p * TILE * TILE;
     c.counts.l2p_targets = (long long)nbricks * TILE * TILE;
-    int *lists, *task_brick;
+    int *lists;
+    int2 *tasks;
+    // many bricks: the near field's longest tasks first too (solves of 1M sources FP64 1337 ->
+    // 1316 us, mixed 1041 -> 1038; few bricks have short, cut tasks and gain nothing); a second
+    // walk writes no task table, so it takes that way as well
+    const bool by_length = !share_bricks(nbricks) || overflow;
     {
         AuxScope on_aux(c);
         if ((rc = ensure(c, S_E2L, (size_t)tot[2] + 1, &lists)) ||
-            (rc = ensure(c, S_TASKMAP, (size_t)ntasks, &task_brick)))
+            (rc = ensure(c, S_TASKMAP, (size_t)(by_length ? TASK_BINS : 1) * ntasks, &tasks)))
             return rc;
         if (!overflow) {
             k_force_lists_copy<<<(int)std::min<long long>((nbricks + 7) / 8,
                                                           (long long)sm_count() * 16),
                                  256, 0, c.stream>>>(nbricks, counts, offs, sstart,
                                                      static_cast<const int *>(ls.p), lists,
-                                                     task_brick);
+                                                     by_length ? nullptr : tasks);
         } else {
             k_force_lists<1><<<trgrid, TR_WARPS * 32, 0, c.stream>>>(
                 nbricks, L, x0s, y0s, hs, theta, tnode, c.nnodes, nullptr, offs, lists, nullptr,
                 sl, nullptr, nullptr, err, nullptr, stack_cap, seg);
-            TC_KERNEL_CHECK();
-            k_task_map<<<(int)std::min<long long>((nbricks + 255) / 256, (long long)sm_count() * 8),
-                         256, 0, c.stream>>>(nbricks, offs, task_brick);
         }
         TC_KERNEL_CHECK();
         TC_CUDA_TRY(cudaEventRecord(c.ev_join, c.stream));
+        if (by_length) {
+            k_near_order<<<(nbricks + 255) / 256, 256, 0, c.stream>>>(nbricks, ntasks, seg, offs,
+                                                                      c.ctrl.near_fill, tasks);
+            TC_KERNEL_CHECK();
+        }
     }
     // The near field reads the sources and the P2P lists only, not the expansions: it runs on
     // the auxiliary stream as soon as the lists are in place, while the upward pass forms the
@@ -1228,7 +1291,7 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
         near<<<neargrid, EV_WARPS * 32, 0, c.stream>>>(
             nbricks, L, x0s, y0s, hs, slot_ptr<int2>(c, S_RANGE), slot_ptr<double>(c, S_XS),
             slot_ptr<double>(c, S_YS), slot_ptr<double>(c, S_VS), offs, lists, xout, yout,
-            partial, 0, nbricks, c.ctrl.near_ctr, task_brick, seg);
+            partial, c.ctrl.near_ctr, tasks, by_length ? c.ctrl.near_fill : nullptr, seg);
         TC_KERNEL_CHECK();
         if (ntasks > nbricks) {
             k_force_gather_parts<<<(int)std::min<long long>((nbricks + 7) / 8,
@@ -1262,6 +1325,17 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
         }
         constexpr int LBS32 = 5;   // the default block side, 32
         const bool fixed = L.lbs == LBS32;
+        // Large host outputs: the blocks are evaluated in runs, each copied to the host on the
+        // auxiliary stream while the next one is evaluated.  Four runs from 2^21 targets on (a
+        // copy of >= 32 MB, ~0.6 ms over PCIe: 16M sheet e2e 11.07 -> 10.67 ms), two from 2^19 on
+        // (1M targets: 1347 -> 1318 us; four took 1412, the runs' tails costing more than
+        // the overlap gains).
+        const size_t per_block = (size_t)1 << (2 * L.lbs);
+        const size_t nt_all = (size_t)nblocks * per_block;
+        const int nchunks = !host_x || nblocks < FORCE_CHUNKS ? 1
+                            : nt_all >= ((size_t)1 << 21)     ? FORCE_CHUNKS
+                            : nt_all >= ((size_t)1 << 19)     ? 2
+                                                              : 1;
         const bool shared_bricks = share_bricks(nbricks);
         // few bricks: their local expansions, unless no brick has an E2L cell
         void *local = nullptr;
@@ -1291,8 +1365,21 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
                                blocks_per_sm<k_force_e2l<P, false>>(EV_WARPS * 32, 0),
                                static_cast<cplx *>(local))))
             return rc2;
+        // many bricks: each run's longest lists first
+        int *by_work = nullptr;
+        if (!shared_bricks) {
+            if ((rc2 = ensure(c, S_FARORDER, (size_t)TASK_BINS * nbricks, &by_work))) return rc2;
+            for (int k = 0; k < nchunks; ++k) {
+                const int b0 = (int)((long long)nblocks * k / nchunks) << (2 * L.lbps);
+                const int b1 = (int)((long long)nblocks * (k + 1) / nchunks) << (2 * L.lbps);
+                k_far_order<<<(b1 - b0 + 255) / 256, 256, 0, c.stream>>>(
+                    nbricks, b0, b1 - b0, counts, c.ctrl.task_fill + k * TASK_BINS,
+                    by_work + (size_t)TASK_BINS * b0);
+                TC_KERNEL_CHECK();
+            }
+        }
         // the far field of bricks [b0, b1)
-        auto far_launch = [&](auto form, double *xo, double *yo, int b0, int b1, int *ctr) -> int {
+        auto far_launch = [&](auto form, double *xo, double *yo, int b0, int b1, int k) -> int {
             constexpr bool M = decltype(form)::value;
             auto kernel = shared_bricks
                               ? (fixed ? k_force_far<P, M, LBS32, EV_WARPS>
@@ -1305,32 +1392,22 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
             const int blocks = shared_bricks ? nbricks : (nbricks + EV_WARPS - 1) / EV_WARPS;
             kernel<<<(int)std::min<long long>(blocks, (long long)sm_count() * occ), EV_WARPS * 32, 0,
                      c.stream>>>(nbricks, L, x0s, y0s, hs, tnode, slot_ptr<double>(c, S_MASS),
-                                 slot_ptr<double>(c, S_EXPS), offs, lists, xo, yo, b0, b1, ctr,
-                                 sexp, sscale, static_cast<const local_t<M> *>(local));
+                                 slot_ptr<double>(c, S_EXPS), offs, lists, xo, yo, b0, b1, c.ctrl.far_ctr + k,
+                                 sexp, sscale, static_cast<const local_t<M> *>(local),
+                                 by_work ? by_work + (size_t)TASK_BINS * b0 : nullptr,
+                                 c.ctrl.task_fill + k * TASK_BINS);
             TC_KERNEL_CHECK();
             return TC_OK;
         };
-        // Large host outputs: the blocks are evaluated in runs, each copied to the host on the
-        // auxiliary stream while the next one is evaluated.  Four runs from 2^21 targets on (a
-        // copy of >= 32 MB, ~0.6 ms over PCIe: 16M sheet e2e 11.07 -> 10.67 ms), two from 2^19 on
-        // (1M targets: 1347 -> 1318 us; four took 1412, the runs' tails costing more than
-        // the overlap gains).
-        const size_t per_block = (size_t)1 << (2 * L.lbs);
-        const size_t nt_all = (size_t)nblocks * per_block;
         double *xfar, *yfar;
-        int *far_ctr = c.ctrl.far_ctr;
         if ((rc2 = ensure(c, S_FARX, nt_all, &xfar)) || (rc2 = ensure(c, S_FARY, nt_all, &yfar)))
             return rc2;
-        const int nchunks = !host_x || nblocks < FORCE_CHUNKS ? 1
-                            : nt_all >= ((size_t)1 << 21)     ? FORCE_CHUNKS
-                            : nt_all >= ((size_t)1 << 19)     ? 2
-                                                              : 1;
         for (int k = 0; k < nchunks; ++k) {
             const int blk0 = (int)((long long)nblocks * k / nchunks);
             const int blk1 = (int)((long long)nblocks * (k + 1) / nchunks);
             const int b0 = blk0 << (2 * L.lbps), b1 = blk1 << (2 * L.lbps);
-            if ((rc2 = mixed ? far_launch(std::true_type{}, xfar, yfar, b0, b1, far_ctr + k)
-                             : far_launch(std::false_type{}, xfar, yfar, b0, b1, far_ctr + k)))
+            if ((rc2 = mixed ? far_launch(std::true_type{}, xfar, yfar, b0, b1, k)
+                             : far_launch(std::false_type{}, xfar, yfar, b0, b1, k)))
                 return rc2;
             if (k == nchunks - 1) phase_mark(c, 7);
             const size_t o = blk0 * per_block, cnt = (size_t)(blk1 - blk0) * per_block;
@@ -1374,8 +1451,8 @@ int prefer_force_carveout() {
 
 void kernels_force(KernelList &v) {
     v.insert(v.end(), {(const void *)k_force_lists<1>, (const void *)k_force_lists<2>,
-                       (const void *)k_force_lists_copy, (const void *)k_task_map,
-                       (const void *)k_add_far,
+                       (const void *)k_force_lists_copy, (const void *)k_near_order,
+                       (const void *)k_add_far, (const void *)k_far_order,
                        (const void *)k_force_gather_parts});
 #define TC_NEAR_KERNELS(CUT)                                                                      \
     v.insert(v.end(), {(const void *)k_force_near<true, 5, CUT>,                                  \

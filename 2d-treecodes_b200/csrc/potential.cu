@@ -496,6 +496,7 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
             if (MODE == 2) {
                 sstart[g] = sl.koff[0] + wglob * sl.cap[0] + cur[0];
                 sstart[ngroups + g] = sl.koff[1] + wglob * sl.cap[1] + cur[1];
+                sstart[2 * ngroups + g] = gsrc;   // (for put_task)
             }
         }
         if (MODE == 2) {
@@ -517,6 +518,36 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
     }
 }
 
+// Few groups (up to PT_LPT_GROUPS): tasks in bins of falling work, the longest first (TaskBins), so
+// that no long one is left for the end: mixed solves of 700,001 targets 1569 -> 1517 us, FP64 ones
+// of 131,072 905 -> 881 us, 1,048,576 (theta 0.3) 3221 -> 3157 us.  Above it the tail is a small
+// share, and neighbouring groups evaluated together share list sources in cache.
+constexpr int PT_LPT_GROUPS = 32768;
+
+// Where the evaluation's tasks go: entry (task, group) t at t, or (stride > 0) in its bin.
+struct TaskTable {
+    int2 *entry;
+    int stride;
+    int *fill;
+    const int *near_sources;   // per group
+    int seg;
+};
+
+// Puts task t (the p-th of group g's) in the table.
+__device__ __forceinline__ void put_task(const TaskTable &tt, int t, int p, int g, int nfar) {
+    if (tt.stride == 0) {
+        tt.entry[t] = make_int2(t, g);
+        return;
+    }
+    // work: near-field sources, and three for a far-field cell
+    const int np = tt.seg < PT_SEG && nfar > 0 ? p - 1 : p;
+    int work = p == 0 ? 3 * nfar : 0;
+    if (np >= 0) work += max(0, min(tt.seg, tt.near_sources[g] - np * tt.seg));
+    const int bin = TASK_BINS - 1 - min(TASK_BINS - 1, (int)((long long)work * TASK_BINS / tt.seg));
+    const int at = atomicAdd(&tt.fill[bin], 1);
+    if (at < tt.stride) tt.entry[(size_t)bin * tt.stride + at] = make_int2(t, g);
+}
+
 // The lists in CSR order from the scratch runs of k_potential_lists<2>, and the task -> group
 // map: warp per group.
 __global__ __launch_bounds__(256) void k_potential_lists_copy(int ngroups,
@@ -525,7 +556,7 @@ __global__ __launch_bounds__(256) void k_potential_lists_copy(int ngroups,
                                                               const int *__restrict__ sstart,
                                                               const int2 *__restrict__ scratch,
                                                               int2 *__restrict__ lists,
-                                                              int *__restrict__ task_group) {
+                                                              TaskTable tt) {
     pdl_begin();
     const int lane = lane_id();
     const int *toff = offs + 2 * ngroups;
@@ -538,7 +569,8 @@ __global__ __launch_bounds__(256) void k_potential_lists_copy(int ngroups,
             int2 *dst = lists + offs[k * ngroups + g];
             for (int i = lane; i < n; i += 32) dst[i] = src[i];
         }
-        for (int t = toff[g] + lane; t < toff[g + 1]; t += 32) task_group[t - tbase] = g;
+        for (int t = toff[g] + lane; t < toff[g + 1]; t += 32)
+            put_task(tt, t - tbase, t - toff[g], g, counts[g]);
     }
 }
 
@@ -595,7 +627,7 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval_mixed(
     const double *__restrict__ mass, const int2 *__restrict__ range, const double *__restrict__ xs,
     const double *__restrict__ ys, const double *__restrict__ vs,
     const int *__restrict__ offs, const int2 *__restrict__ lists, double *__restrict__ out,
-    double *__restrict__ partial, int *task_ctr, const int *__restrict__ task_group,
+    double *__restrict__ partial, int *task_ctr, TaskTable tt,
     const float2 *__restrict__ sexp, const float *__restrict__ sscale) {
     pdl_begin();
     // E2P coefficients in pairs (D_2j.re, D_2j+1.re, D_2j.im, D_2j+1.im): the even and
@@ -616,13 +648,17 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval_mixed(
     const int *toff = offs + 2 * ngroups;
     const int tbase = toff[0];
     const int ntasks = toff[ngroups] - tbase;
+    const TaskBins bins(tt.stride ? tt.fill : nullptr);
 
     for (;;) {
         int task = 0;
         if (lane == 0) task = atomicAdd(task_ctr, 1);
         task = __shfl_sync(FULL_MASK, task, 0);
         if (task >= ntasks) break;
-        const int g = task_group[task];
+        const int2 entry = tt.entry[tt.stride ? bins.place(task, tt.stride) : task];
+        task = entry.x;
+        const int g = entry.y;
+        if ((unsigned)task >= (unsigned)ntasks || (unsigned)g >= (unsigned)ngroups) break;
         const int part = task - (toff[g] - tbase);
         const int nparts = toff[g + 1] - toff[g];
         const int t = g * 32 + lane;
@@ -905,7 +941,7 @@ __global__ __launch_bounds__(PD_WARPS * 32, PD_MIN_BLOCKS) void k_potential_eval
     const int2 *__restrict__ range, const double *__restrict__ xs,
     const double *__restrict__ ys, const double *__restrict__ vs,
     const int *__restrict__ offs, const int2 *__restrict__ lists, double *__restrict__ out,
-    double *__restrict__ partial, int *task_ctr, const int *__restrict__ task_group, int seg,
+    double *__restrict__ partial, int *task_ctr, TaskTable tt, int seg,
     const double4 *__restrict__ geo, const cplx *__restrict__ local) {
     extern __shared__ __align__(16) unsigned char eval_dyn[];
     double2 *s_tab = reinterpret_cast<double2 *>(eval_dyn);
@@ -920,13 +956,17 @@ __global__ __launch_bounds__(PD_WARPS * 32, PD_MIN_BLOCKS) void k_potential_eval
     const int *toff = offs + 2 * ngroups;
     const int tbase = toff[0];
     const int ntasks = toff[ngroups] - tbase;
+    const TaskBins bins(tt.stride ? tt.fill : nullptr);
 
     for (;;) {
         int task = 0;
         if (lane == 0) task = atomicAdd(task_ctr, 1);
         task = __shfl_sync(FULL_MASK, task, 0);
         if (task >= ntasks) break;
-        const int g = task_group[task];
+        const int2 entry = tt.entry[tt.stride ? bins.place(task, tt.stride) : task];
+        task = entry.x;
+        const int g = entry.y;
+        if ((unsigned)task >= (unsigned)ntasks || (unsigned)g >= (unsigned)ngroups) break;
         const int part = task - (toff[g] - tbase);
         const int nparts = toff[g + 1] - toff[g];
         // the near-field task of this part; -1: the far field alone
@@ -1133,12 +1173,13 @@ __global__ __launch_bounds__(PD_WARPS * 32, PD_MIN_BLOCKS) void k_potential_eval
     }
 }
 
-__global__ void k_task_map_groups(int ngroups, const int *__restrict__ offs,
-                                  int *__restrict__ task_group) {
+__global__ void k_task_map_groups(int ngroups, const int *__restrict__ counts,
+                                  const int *__restrict__ offs, TaskTable tt) {
     const int *toff = offs + 2 * ngroups;
     const int tbase = toff[0];
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += gridDim.x * blockDim.x)
-        for (int t = toff[g]; t < toff[g + 1]; ++t) task_group[t - tbase] = g;
+        for (int t = toff[g]; t < toff[g + 1]; ++t)
+            put_task(tt, t - tbase, t - toff[g], g, counts[g]);
 }
 
 // Sum of the parts of every multi-task group, in task order (deterministic).
@@ -1221,7 +1262,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
         AuxScope on_aux(c);
         if ((rc = sort_targets(c, xt, yt, m, &vo))) return rc;
         if ((rc = list_scratch(c, 2, nwarps, ngroups, sizeof(int2), sl, ls)) ||
-            (rc = ensure(c, S_LSTART, (size_t)2 * ngroups, &sstart)))
+            (rc = ensure(c, S_LSTART, (size_t)3 * ngroups, &sstart)))
             return rc;
         if (with_sets) {
             int *lists2, *num;
@@ -1267,18 +1308,19 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
     c.counts.e2l_pairs = 0;
     c.counts.l2p_targets = 0;
     int2 *lists;
-    int *task_group;
+    TaskTable tt = {nullptr, ngroups <= PT_LPT_GROUPS ? ntasks : 0, c.ctrl.task_fill,
+                    sstart + 2 * (size_t)ngroups, seg};
     {
         AuxScope on_aux(c);
         if ((rc = ensure(c, S_PE2P, (size_t)total + 1, &lists)) ||
-            (rc = ensure(c, S_TASKMAP, (size_t)ntasks, &task_group)))
+            (rc = ensure(c, S_TASKMAP, (size_t)(tt.stride ? TASK_BINS : 1) * ntasks, &tt.entry)))
             return rc;
         if (!overflow) {
             TC_CUDA_TRY(launch_pdl(
                 chain, k_potential_lists_copy,
                 (int)std::min<long long>((ngroups + 7) / 8, (long long)sm_count_p() * 16), 256, 0,
                 c.stream, ngroups, (const int *)counts, (const int *)offs, (const int *)sstart,
-                static_cast<const int2 *>(ls.p), lists, task_group));
+                static_cast<const int2 *>(ls.p), lists, tt));
         } else {
             // (the second walk does not add to the work counters)
             k_potential_lists<1><<<grid, PT_WARPS * 32, 0, c.stream>>>(
@@ -1287,7 +1329,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
             TC_KERNEL_CHECK();
             k_task_map_groups<<<(int)std::min<long long>((ngroups + 255) / 256,
                                                          (long long)sm_count_p() * 8),
-                                256, 0, c.stream>>>(ngroups, offs, task_group);
+                                256, 0, c.stream>>>(ngroups, counts, offs, tt);
         }
         TC_KERNEL_CHECK();
         TC_CUDA_TRY(mark_event(c, c.ev_join));
@@ -1327,7 +1369,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
                 (const int2 *)slot_ptr<int2>(c, S_RANGE), (const double *)slot_ptr<double>(c, S_XS),
                 (const double *)slot_ptr<double>(c, S_YS),
                 (const double *)slot_ptr<double>(c, S_VS), (const int *)offs, (const int2 *)lists,
-                out, partial, task_ctr, (const int *)task_group, (const float2 *)sexp,
+                out, partial, task_ctr, tt, (const float2 *)sexp,
                 (const float *)sscale));
         } else {
             static const cudaError_t attr_rc[2] = {
@@ -1361,7 +1403,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
                 (const int2 *)slot_ptr<int2>(c, S_RANGE), (const double *)slot_ptr<double>(c, S_XS),
                 (const double *)slot_ptr<double>(c, S_YS),
                 (const double *)slot_ptr<double>(c, S_VS), (const int *)offs, (const int2 *)lists,
-                out, partial, task_ctr, (const int *)task_group, seg, sets.geo,
+                out, partial, task_ctr, tt, seg, sets.geo,
                 (const cplx *)set_local));
         }
         TC_KERNEL_CHECK();

@@ -140,6 +140,7 @@ size_t footprint_estimate(int kind, long long n, long long ntargets, long long n
         const long long bricks = m / (tc::TILE * tc::TILE);
         b += (size_t)bricks * (1024 / tc::near_segment((int)std::min<long long>(bricks, 1 << 24))) *
              1024;
+        b += (size_t)bricks * 160;   // the tables of tasks and of the far field's bricks by length
     } else {
         // staged targets, output, target sort, partials and the per-group lists, whose far
         // part grows as 1/theta^2 (about 14 entries per target at theta = 0.3); the list
@@ -149,6 +150,8 @@ size_t footprint_estimate(int kind, long long n, long long ntargets, long long n
         if (!precision) b += (size_t)std::min(ntargets, 1ll << 19) * 256;
         // FP64: the common far fields of sets of 128 targets (two lists, 32 coefficients)
         if (!precision) b += (size_t)ntargets * 18;
+        // up to 2^20 targets: the tasks' table by length, 64 B a task
+        b += (size_t)std::min(ntargets, 1ll << 20) * (precision ? 8 : 64);
     }
     return b + (4u << 20);
 }

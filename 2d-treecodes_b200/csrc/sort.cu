@@ -1171,6 +1171,8 @@ int ctrl_prepare(Context &c, int n, int m) {
         take(k.near_ctr, 1);
         take(k.far_ctr, FORCE_CHUNKS);
         take(k.e2l_ctr, 1);
+        take(k.task_fill, TASK_BINS * FORCE_CHUNKS);
+        take(k.near_fill, TASK_BINS);
         take(k.t_tile_ctr, RS_MAX_PASSES);
         take(k.hist, NHIST * RS_RADIX);
         take(k.t_hist, RS_MAX_PASSES * RS_RADIX);

@@ -124,6 +124,30 @@ struct __align__(32) TNode {
     int count;
 };
 
+// Longest tasks first: persistent warps that take tasks from a counter end together only if no long
+// task is taken late.  Tasks are appended to TASK_BINS bins of falling work, bin b at b * stride;
+// `fill` counts each bin's tasks.  A consumer reads the counts once (every lane of the warp) and maps
+// the i-th task to its place.
+constexpr int TASK_BINS = 8;
+struct TaskBins {
+    int incl;   // lane b < TASK_BINS: tasks in bins 0 .. b
+    __device__ __forceinline__ explicit TaskBins(const int *fill) {
+        const int lane = threadIdx.x & 31;
+        incl = fill && lane < TASK_BINS ? fill[lane] : 0;
+        for (int o = 1; o < TASK_BINS; o <<= 1) {
+            const int t = __shfl_up_sync(FULL_MASK, incl, o);
+            if (lane >= o) incl += t;
+        }
+    }
+    // place of the i-th task, i below the total
+    __device__ __forceinline__ int place(int i, int stride) const {
+        const int lane = threadIdx.x & 31;
+        const int bin = __popc(__ballot_sync(FULL_MASK, lane < TASK_BINS - 1 && incl <= i));
+        const int before = __shfl_sync(FULL_MASK, incl, bin ? bin - 1 : 0);
+        return bin * stride + i - (bin ? before : 0);
+    }
+};
+
 // Block-wide exclusive scan of one int per thread (blockDim.x a multiple of 32, <= 1024); the
 // block total goes to *total when total is not null.  Every thread of the block must call it.
 __device__ __forceinline__ int block_exclusive_scan(int v, int *total) {

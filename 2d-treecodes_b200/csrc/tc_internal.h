@@ -36,7 +36,7 @@ enum Slot {
     S_TNODE, S_RANGE, S_CELL, S_MASS, S_W, S_WX, S_WY, S_EXPS, S_UPCNT,
     // force traversal / lists
     S_FCOUNT, S_FOFF, S_E2L, S_FPART, S_SEXP, S_SSCALE, S_TASKMAP,
-    S_LSTART, S_FARX, S_FARY, S_LOCAL,
+    S_LSTART, S_FARX, S_FARY, S_LOCAL, S_FARORDER,
     // potential targets / lists
     S_TKEYS, S_TPERM, S_TKEYS2, S_TPERM2, S_PCOUNT, S_POFF, S_PE2P,
     S_SETLIST, S_SETNUM, S_SETGEO, S_SETLOCAL,
@@ -108,6 +108,8 @@ struct Ctrl {
     int *nlist, *tl_ctr;          // tree: split-list length, tiles taken
     int *meta;                    // list build: overflow flag, longest runs
     int *near_ctr, *far_ctr, *e2l_ctr;   // evaluation tasks / far-field bricks taken
+    // tasks per bin (TaskBins): far-field bricks (per run) or potential tasks; near-field tasks
+    int *task_fill, *near_fill;
     int *t_tile_ctr;              // target sort
     int *hist, *t_hist;           // digit histograms of the source and the target sort
     unsigned *status, *t_status, *tl_status;   // look-back words: sorts, tree list
