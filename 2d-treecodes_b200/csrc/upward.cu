@@ -1,7 +1,7 @@
 // upward.cu -- the upward pass, in two parts.
 //
-// Moments (what the traversals read): k_leaf_setup (four threads per node) runs the leaf setup
-// with the reference's four strided accumulators (drivers/upward.cpp:61-93,
+// Moments (what the traversals read): k_leaf_setup_warp (a warp per node) or k_leaf_setup (four
+// threads per node, for many nodes) runs the leaf setup with the reference's four strided accumulators (drivers/upward.cpp:61-93,
 // kernels/upward-common.ispc:13-57); k_moments_level / k_moments_top then form every inner
 // node's mass, weights, com and radius level by level, deepest first (upward.cpp:95-218).
 // Expansions: k_leaf_p2e (one warp per leaf, lanes over sources, FP32 lane sums in the
@@ -60,6 +60,30 @@ __device__ __forceinline__ bool is_leaf(int2 rg, int4 cl, int leafcap) {
 }
 
 // ------------------------------------------------------------------------------ leaves
+// A leaf's moments from its sums: com (upward.cpp:71-72; x0 = fma(cx, h, xmin) as in build_tree).
+__device__ __forceinline__ void leaf_record(int node, int4 cl, double msum, double wsum,
+                                            double xsum, double ysum, double r2, TNode *tnode,
+                                            double *mass, double *wgt, double *wxs, double *wys,
+                                            const Frame *__restrict__ frame) {
+    double xcom, ycom;
+    if (wsum != 0) {
+        xcom = __ddiv_rn(xsum, wsum);
+        ycom = __ddiv_rn(ysum, wsum);
+    } else {
+        const Frame f = *frame;
+        const double h = __ddiv_rn(f.ext, (double)(1 << cl.x));
+        xcom = __fma_rn(0.5, h, __fma_rn((double)cl.y, h, f.xmin));
+        ycom = __fma_rn(0.5, h, __fma_rn((double)cl.z, h, f.ymin));
+    }
+    tnode[node].xcom = xcom;
+    tnode[node].ycom = ycom;
+    tnode[node].r = __dsqrt_rn(r2);
+    mass[node] = msum;
+    wgt[node] = wsum;
+    wxs[node] = xsum;
+    wys[node] = ysum;
+}
+
 // k_leaf_setup: lane quad per node (4 threads each, in the order of the node ids).  Only the
 // quads of leaves do work; the others still take part in the quad shuffles.
 __global__ __launch_bounds__(256) void k_leaf_setup(
@@ -119,25 +143,100 @@ __global__ __launch_bounds__(256) void k_leaf_setup(
     r2 = fmax(r2, __shfl_xor_sync(FULL_MASK, r2, 1));
     r2 = fmax(r2, __shfl_xor_sync(FULL_MASK, r2, 2));
     if (act && q == 0) {
-        // com (upward.cpp:71-72; x0 = fma(cx, h, xmin) as in build_tree)
-        double xcom, ycom;
-        if (wsum != 0) {
-            xcom = __ddiv_rn(xsum, wsum);
-            ycom = __ddiv_rn(ysum, wsum);
-        } else {
-            const Frame f = *frame;
-            const double h = __ddiv_rn(f.ext, (double)(1 << cl.x));
-            xcom = __fma_rn(0.5, h, __fma_rn((double)cl.y, h, f.xmin));
-            ycom = __fma_rn(0.5, h, __fma_rn((double)cl.z, h, f.ymin));
-        }
-        tnode[node].xcom = xcom;
-        tnode[node].ycom = ycom;
-        tnode[node].r = __dsqrt_rn(r2);
-        mass[node] = msum;
-        wgt[node] = wsum;
-        wxs[node] = xsum;
-        wys[node] = ysum;
+        leaf_record(node, cl, msum, wsum, xsum, ysum, r2, tnode, mass, wgt, wxs, wys, frame);
     }
+}
+
+// The same for fewer nodes: a warp per node.  Few leaves of up to 512 sources are bound by the
+// latency of a lane's serial loads; here the warp loads LS_BATCH sources at a time, coalesced,
+// leaves v, |v|, x|v|, y|v| in shared memory, and 16 lanes run the 16 chains (four per quantity) of
+// the same sums.  The radius is a maximum, so all 32 lanes take part, each about the centre of the
+// chain that its sources belong to.  Solves of 4096 sources: potential 172 -> 164 us, force 171 ->
+// 164; potential 64K 412 -> 390, 700,001 mixed 1522 -> 1490; force 1M mixed 1044 -> 1030 us.
+// The quads do with 0.4 of the instructions and waits per leaf, which counts once the nodes are
+// many times the resident warps: equal at 60,000 and 120,000 nodes, at 236,000 (16M sheet) the
+// warp form takes 143 us for the quads' 121.
+constexpr int LS_WARPS = 4;
+constexpr int LS_BATCH = 128;
+constexpr int LS_ROW = LS_BATCH + 4;   // padded: the 16 chains' operands in distinct banks
+constexpr int LS_U = LS_BATCH / 32;
+constexpr int LS_QUAD_NODES = 1 << 16;   // from here on, a quad per node
+
+__global__ __launch_bounds__(LS_WARPS * 32) void k_leaf_setup_warp(
+    int nnodes, int nsrc, int leafcap, const double *__restrict__ xs, const double *__restrict__ ys,
+    const double *__restrict__ vs, const int2 *__restrict__ range, const int4 *__restrict__ cell,
+    TNode *tnode, double *mass, double *wgt, double *wxs, double *wys,
+    const Frame *__restrict__ frame, unsigned *err) {
+    __shared__ double s_val[LS_WARPS][4][LS_ROW];
+    pdl_begin();
+    const int lane = lane_id(), q = lane & 3, warp = threadIdx.x >> 5;
+    const int node = blockIdx.x * LS_WARPS + warp;
+    if (node >= nnodes) return;
+    const int2 rg = range[node];
+    const int4 cl = cell[node];
+    if (!is_leaf(rg, cl, leafcap)) return;
+    if (rg.x < 0 || rg.y < rg.x || rg.y > nsrc || cl.w >= nnodes || cl.x < 0 || cl.x > LMAX) {
+        if (lane == 0) atomicOr(err, DEVERR_BOUNDS);
+        return;
+    }
+    const int s = rg.x, e = rg.y;
+    double(&val)[4][LS_ROW] = s_val[warp];
+    // lane 4 c + q holds chain q of quantity c (lanes 16-31 idle); past the end zeros are added,
+    // which change no sum
+    const double *chain = &val[(lane >> 2) & 3][q];
+    double sum = 0;
+    double x[LS_U], y[LS_U];
+    for (int base = s; base < e; base += LS_BATCH) {
+        double m[LS_U];
+#pragma unroll
+        for (int u = 0; u < LS_U; ++u) {
+            const int j = base + 32 * u + lane;
+            const bool ok = j < e;
+            x[u] = ok ? __ldg(xs + j) : 0.0;
+            y[u] = ok ? __ldg(ys + j) : 0.0;
+            m[u] = ok ? __ldg(vs + j) : 0.0;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < LS_U; ++u) {
+            const double w = fabs(m[u]);
+            val[0][32 * u + lane] = m[u];
+            val[1][32 * u + lane] = w;
+            val[2][32 * u + lane] = __dmul_rn(x[u], w);
+            val[3][32 * u + lane] = __dmul_rn(y[u], w);
+        }
+        __syncwarp();
+        if (lane < 16) {
+            const int n = (min(LS_BATCH, e - base) + 3) & ~3;
+#pragma unroll 8
+            for (int i = 0; i < n; i += 4) sum = __dadd_rn(sum, chain[i]);
+        }
+    }
+    __syncwarp();
+    // (l0 + l1) + (l2 + l3) of each quantity, broadcast
+    const double pair = __dadd_rn(sum, __shfl_down_sync(FULL_MASK, sum, 1));
+    const double quad = __dadd_rn(pair, __shfl_down_sync(FULL_MASK, pair, 2));
+    const double msum = __shfl_sync(FULL_MASK, quad, 0), wsum = __shfl_sync(FULL_MASK, quad, 4),
+                 xsum = __shfl_sync(FULL_MASK, quad, 8), ysum = __shfl_sync(FULL_MASK, quad, 12);
+    const double ws = __shfl_sync(FULL_MASK, sum, 4 + q);
+    const double lx = ws != 0 ? __ddiv_rn(xsum, wsum) : 0.0;
+    const double ly = ws != 0 ? __ddiv_rn(ysum, wsum) : 0.0;
+    double r2 = 0;
+    auto reach = [&](double xj, double yj) {
+        const double xr = __dsub_rn(xj, lx), yr = __dsub_rn(yj, ly);
+        r2 = fmax(r2, __dadd_rn(__dmul_rn(xr, xr), __dmul_rn(yr, yr)));
+    };
+    if (e - s <= LS_BATCH) {   // still in registers
+#pragma unroll
+        for (int u = 0; u < LS_U; ++u)
+            if (s + 32 * u + lane < e) reach(x[u], y[u]);
+    } else {
+#pragma unroll 8
+        for (int j = s + lane; j < e; j += 32) reach(__ldg(xs + j), __ldg(ys + j));
+    }
+    for (int o = 1; o < 32; o <<= 1) r2 = fmax(r2, __shfl_xor_sync(FULL_MASK, r2, o));
+    if (lane == 0)
+        leaf_record(node, cl, msum, wsum, xsum, ysum, r2, tnode, mass, wgt, wxs, wys, frame);
 }
 
 // k_leaf_p2e: a_n = -1/(n+1) sum_i v_i (z_i - c)^(n+1), one warp per leaf, lanes over sources
@@ -720,7 +819,11 @@ int upward_moments(Context &c) {
     unsigned *err = c.ctrl.err;
     double *mass = slot_ptr<double>(c, S_MASS), *w = slot_ptr<double>(c, S_W),
            *wx = slot_ptr<double>(c, S_WX), *wy = slot_ptr<double>(c, S_WY);
-    TC_CUDA_TRY(launch_pdl(ovl, k_leaf_setup, (int)(((long long)nn * 4 + 255) / 256), 256, 0,
+    const bool quads = nn >= LS_QUAD_NODES;
+    TC_CUDA_TRY(launch_pdl(ovl, quads ? k_leaf_setup : k_leaf_setup_warp,
+                           quads ? (int)(((long long)nn * 4 + 255) / 256)
+                                 : (nn + LS_WARPS - 1) / LS_WARPS,
+                           quads ? 256 : LS_WARPS * 32, 0,
                            c.stream, nn, c.nsrc, c.leafcap,
                            (const double *)slot_ptr<double>(c, S_XS),
                            (const double *)slot_ptr<double>(c, S_YS),
@@ -866,7 +969,7 @@ int upward_pass(Context &c, int order) {
 }
 
 void kernels_upward(KernelList &v) {
-    v.insert(v.end(), {(const void *)k_leaf_setup, (const void *)k_moments_level,
+    v.insert(v.end(), {(const void *)k_leaf_setup, (const void *)k_leaf_setup_warp, (const void *)k_moments_level,
                        (const void *)k_moments_top});
 #define TC_UPWARD_KERNELS(P)                                                                     \
     v.insert(v.end(), {(const void *)k_leaf_p2e<P, true>, (const void *)k_leaf_p2e<P, false>,    \
