@@ -355,12 +355,13 @@ static void finish_timing(Context &c) {
 // formed while the interaction lists are built.
 static int build_tree_moments(Context &c, int kind, const double *x, const double *y,
                               const double *v, int n, int m = 0,
-                              cudaEvent_t values_ready = nullptr) {
+                              cudaEvent_t values_ready = nullptr, const double *xt = nullptr,
+                              const double *yt = nullptr) {
     int rc;
     g_launches = 0;
     c.near_marked = false;
     if ((rc = ctrl_prepare(c, n, m))) return rc;
-    if ((rc = sort_sources(c, x, y, v, n, values_ready))) return rc;
+    if ((rc = sort_sources(c, x, y, v, n, values_ready, xt, yt, m))) return rc;
     phase_mark(c, 1);
     if ((rc = build_topology(c, kind ? LEAF_FORCE : LEAF_POTENTIAL))) return rc;
     if ((rc = finish_sources(c))) return rc;
@@ -404,7 +405,7 @@ static int potential_device(Context &c, double theta, const double *xs, const do
     int rc;
     phase_mark(c, 0);
     c.single = single_stream(n, (m + 31) / 32) && !values_ready;
-    if ((rc = build_tree_moments(c, 0, xs, ys, vs, n, m, values_ready))) return rc;
+    if ((rc = build_tree_moments(c, 0, xs, ys, vs, n, m, values_ready, xt, yt))) return rc;
     if ((rc = potential(c, theta, xt, yt, m, out, expansions_then_mark))) return rc;
     phase_mark(c, 5);
     if ((rc = check_device_errors(c, "treecode_potential"))) return rc;

@@ -154,6 +154,7 @@ struct Context {
     // a small solve: everything on `stream`, in order (single_stream); AuxScope and stream_after
     // then do nothing
     bool single = false;
+    bool targets_sorted = false;   // the solve's target order was formed with the sources'
     cudaEvent_t ev_fork = nullptr, ev_totals = nullptr, ev_join = nullptr;
     // host entry points: x/y are copied on `stream`, v (and targets) on `aux` after them;
     // ev_inputs marks v's arrival
@@ -289,7 +290,8 @@ int radix_sort_pairs(Context &c, const int *keys_in, const int *vals_in, int n, 
 // tree build run while v is still being copied in; without it x/y/v are all sorted here and
 // finish_sources() does nothing.
 int sort_sources(Context &c, const double *x, const double *y, const double *v, int n,
-                 cudaEvent_t values_ready = nullptr);
+                 cudaEvent_t values_ready = nullptr, const double *xt = nullptr,
+                 const double *yt = nullptr, int m = 0);
 int finish_sources(Context &c);
 int sort_targets(Context &c, const double *xt, const double *yt, int m, int **perm);
 

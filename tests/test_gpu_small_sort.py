@@ -64,3 +64,24 @@ def test_small_solves_host_and_device_agree(m):
     ref = torch.empty_like(out)
     T.Context().direct_potential_device(*d, ref)
     assert float((out - ref).norm()) < 1e-5 * float(ref.norm())
+
+
+@pytest.mark.parametrize("n", [1, 4096, 4097, 16384, 16385])
+def test_sources_and_targets_sorted_side_by_side(n):
+    """One context, the targets' count moving between the forms (with the sources, by themselves,
+    general): every target's value, against the direct sum (order 12 at theta 0.5, as above)."""
+    import torch
+    import treecodes as T
+
+    x, y, v = inputs(n, n)
+    d = [torch.tensor(a, device="cuda") for a in (x, y, v)]
+    ctx = T.Context()
+    for m in (1, 4096, 16385, 4097, 16384, 32769, 33):
+        tx, ty, _ = inputs(m, m + 1)
+        t = [torch.tensor(1.5 * a - 0.25, device="cuda") for a in (tx, ty)]
+        out, ref = (torch.full((m,), float("nan"), device="cuda", dtype=torch.float64)
+                    for _ in range(2))
+        torch.cuda.synchronize()
+        ctx.potential_device(0.5, *d, *t, out)
+        T.Context().direct_potential_device(*d, *t, ref)
+        assert float((out - ref).norm()) < 1e-5 * float(ref.norm()), m
