@@ -1182,24 +1182,41 @@ __global__ void k_task_map_groups(int ngroups, const int *__restrict__ counts,
             put_task(tt, t - tbase, t - toff[g], g, counts[g]);
 }
 
-// Sum of the parts of every multi-task group, in task order (deterministic).
-__global__ void k_potential_gather_parts(int ngroups, int m, const int *__restrict__ tperm,
-                                         const int *__restrict__ offs,
-                                         const double *__restrict__ partial,
-                                         double *__restrict__ out) {
-    pdl_begin();
+// Sum of the parts of every multi-task group, in task order (deterministic).  Bound by latency:
+// what is older than the evaluation (offsets, order) is read before the wait for it, and the parts
+// GP_BATCH at a time (24 parts a group at 4096 sources: 142.0 -> 139.9 us a solve).
+constexpr int GP_BATCH = 8;
+
+__global__ __launch_bounds__(256) void k_potential_gather_parts(int ngroups, int m,
+                                                                const int *__restrict__ tperm,
+                                                                const int *__restrict__ offs,
+                                                                const double *__restrict__ partial,
+                                                                double *__restrict__ out) {
     const int lane = lane_id();
     const int *toff = offs + 2 * ngroups;
-    const int tbase = toff[0];
-    for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < ngroups;
-         g += (gridDim.x * blockDim.x) >> 5) {
-        const int t0 = toff[g] - tbase, np = toff[g + 1] - toff[g];
+    const int stride = (gridDim.x * blockDim.x) >> 5;
+    bool waited = false;
+    for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < ngroups; g += stride) {
+        const int t0 = toff[g] - toff[0], np = toff[g + 1] - toff[g];
         if (np <= 1) continue;
-        double s = 0;
-        for (int p = 0; p < np; ++p) s += partial[(size_t)(t0 + p) * 32 + lane];
         const int t = g * 32 + lane;
-        if (t < m) out[tperm[t]] = s;
+        const int to = t < m ? tperm[t] : 0;
+        if (!waited) pdl_begin();   // the offsets and the order are older than the evaluation
+        waited = true;
+        const double *p = partial + (size_t)t0 * 32 + lane;
+        double s = 0;
+        int k = 0;
+        for (; k + GP_BATCH <= np; k += GP_BATCH) {
+            double v[GP_BATCH];
+#pragma unroll
+            for (int u = 0; u < GP_BATCH; ++u) v[u] = p[(size_t)(k + u) * 32];
+#pragma unroll
+            for (int u = 0; u < GP_BATCH; ++u) s += v[u];
+        }
+        for (; k < np; ++k) s += p[(size_t)k * 32];
+        if (t < m) out[to] = s;
     }
+    if (!waited) pdl_begin();
 }
 
 // Mixed form: a_k / R^(k+1) in FP32, R = the cell's power-of-two radius (see force.cu).
