@@ -52,6 +52,32 @@ __device__ __forceinline__ int gallop_lower_bound(const int *__restrict__ keys, 
     return lower_bound_dev(keys, a + 1, min(a + step, hi), val);
 }
 
+// The same bound, found by a group of SB_LANES lanes that read SB_LANES keys per step: first at
+// distances 8, 64, 512 ... from lo, then evenly inside the bracket.  A cell of 1000 sources takes 4
+// dependent reads, where one lane's doubling and halving take 20.  `gmask` names the group's lanes, `g` this one.
+constexpr int SB_LANES = 8;
+
+__device__ __forceinline__ int group_lower_bound(const int *__restrict__ keys, int lo, int hi,
+                                                 int val, unsigned gmask, int g) {
+    if (lo >= hi) return lo;
+    // how many of the group's probes, at rising positions, are below val
+    auto below = [&](int p, bool in) {
+        return __popc(__ballot_sync(gmask, in && keys[in ? p : lo] < val) & gmask);
+    };
+    const int reach = 1 << (3 * (g + 1));   // 8 .. 2^24 (sources are fewer than 2^30)
+    int c = below(lo + reach, reach < hi - lo);
+    int a = c ? lo + (1 << (3 * c)) + 1 : lo;                    // the answer is in [a, b]
+    int b = c < SB_LANES ? min(hi, lo + (1 << (3 * (c + 1)))) : hi;
+    while (a < b) {
+        const int step = (b - a + SB_LANES) / (SB_LANES + 1);
+        const int p = a + (g + 1) * step - 1;
+        c = below(p, p < b);
+        if (c < SB_LANES) b = min(b, a + (c + 1) * step - 1);
+        a += c * step;
+    }
+    return a;
+}
+
 // The split list: per tile of TL_TILE sources, each source's level mask (bit l: it starts an
 // inner cell of level l), a block scan
 // of the flags and the tile's global offset by a decoupled look-back over the tiles before it
@@ -326,11 +352,18 @@ __global__ void k_tree_root(int n, TNode *tnode, int2 *range, int4 *cell) {
     tnode[0].child = -1;
 }
 
-// Four threads per inner cell: the r-th inner cell of level l is started by list entry
-// inv[l][r] (source s = lpos[j]); its own id comes from its parent's rank.  Thread q of the four
-// finds the end of child q (the key boundary of child q + 1, or of the cell's end for q = 3) by
-// a search from s; the four searches run at once instead of one after another (each boundary
-// lies inside [s, e), since the keys are sorted), and thread q writes child q.
+// A warp (WIDE) or four threads per inner cell: the r-th inner cell of level l is started by list
+// entry inv[l][r] (source s = lpos[j]); its own id comes from its parent's rank.  The lanes q of
+// the cell (eight each, or one) find the end of child q (the key boundary of child q + 1, or of the
+// cell's end for q = 3) by a search from s; the four searches run at once instead of one after
+// another (each boundary lies inside [s, e), since the keys are sorted), and the first lane of q
+// writes child q.  Bound by the latency of dependent reads: with WIDE the tree phase takes 38 -> 32
+// us for the potential of 64K sources, 56 -> 46 for the force of 1M (4,080 cells).  With more
+// cells than resident warps the wide search's extra reads count: 15,000 cells 76 -> 72 us, 30,000
+// 97 -> 105, 59,000 150 -> 174 us.
+constexpr int TC_WIDE_CELLS = 16384;   // up to here WIDE
+
+template <bool WIDE>
 __global__ void k_tree_children(const int *__restrict__ keys, int n, int leafcap,
                                 const int *__restrict__ lpos,
                                 const unsigned short *__restrict__ lmask,
@@ -339,11 +372,15 @@ __global__ void k_tree_children(const int *__restrict__ keys, int n, int leafcap
                                 TNode *__restrict__ tnode, int2 *__restrict__ range,
                                 int4 *__restrict__ cell, unsigned *err) {
     pdl_begin();
-    const int q = threadIdx.x & 3;
-    const unsigned gmask = 0xFu << (lane_id() & ~3);   // the cell's four lanes
-    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; t < ninner;
-         t += (gridDim.x * blockDim.x) >> 2) {
-        // level of inner cell t: the inner cells are numbered level by level (the four threads
+    constexpr int W = WIDE ? SB_LANES : 1;   // lanes per child
+    static_assert(4 * SB_LANES == 32, "a warp per cell");
+    const int lane = threadIdx.x % (4 * W), q = lane / W, g = lane % W;
+    const int first = lane_id() - lane;                             // the cell's lanes in the warp
+    const unsigned cmask = (unsigned)(((1ull << (4 * W)) - 1) << first);
+    const unsigned gmask = ((1u << W) - 1) << (first + q * W);      // the child's
+    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) / (4 * W); t < ninner;
+         t += (gridDim.x * blockDim.x) / (4 * W)) {
+        // level of inner cell t: the inner cells are numbered level by level (the cell's lanes
         // compute the same values, so they branch together)
         int l = 0, r = t;
         while (l < LMAX - 1 && r >= (lo.off[l + 2] - lo.off[l + 1]) / 4) {
@@ -354,7 +391,7 @@ __global__ void k_tree_children(const int *__restrict__ keys, int n, int leafcap
         const int s = lpos[j];
         const unsigned mj = lmask[j];
         if (!((mj >> l) & 1u)) {
-            if (q == 0) atomicOr(err, DEVERR_TREE);
+            if (lane == 0) atomicOr(err, DEVERR_TREE);
             continue;
         }
         const int key = keys[s];
@@ -367,31 +404,32 @@ __global__ void k_tree_children(const int *__restrict__ keys, int n, int leafcap
             // before s).  Its rank is the count of such entries up to j, minus one.
             const int prank = rank[(size_t)(l - 1) * stride + j] + (int)((mj >> (l - 1)) & 1u) - 1;
             if (prank < 0) {
-                if (q == 0) atomicOr(err, DEVERR_TREE);
+                if (lane == 0) atomicOr(err, DEVERR_TREE);
                 continue;
             }
             id = lo.off[l] + 4 * prank + (P & 3);
         }
         const int base = lo.off[l + 1] + 4 * r;
         if (id < 0 || id >= nnodes || base < 0 || base + 4 > nnodes) {
-            if (q == 0) atomicOr(err, DEVERR_BOUNDS);
+            if (lane == 0) atomicOr(err, DEVERR_BOUNDS);
             continue;
         }
-        if (q == 0) tnode[id].child = base;
-        if (l == 0 && q == 0) {   // the root's record (k_tree_root, when nothing is split)
+        if (lane == 0) tnode[id].child = base;
+        if (l == 0 && lane == 0) {   // the root's record (k_tree_root, when nothing is split)
             range[0] = make_int2(0, n);
             cell[0] = make_int4(0, 0, 0, -1);
             tnode[0].count = n;
         }
         const int cshift = shift - 2;
         // the end of child q: the first key of child q + 1, or past the cell for q = 3
-        int end_q;
-        if (q < 3)
-            end_q = gallop_lower_bound(keys, s, n, ((P << 2) | (q + 1)) << cshift);
-        else
-            end_q = l == 0 ? n : gallop_lower_bound(keys, s, n, (P + 1) << shift);
-        int beg_q = __shfl_up_sync(gmask, end_q, 1, 4);
+        const int bound = q < 3 ? ((P << 2) | (q + 1)) << cshift : (P + 1) << shift;
+        int end_q = n;
+        if (q < 3 || l > 0)
+            end_q = WIDE ? group_lower_bound(keys, s, n, bound, gmask, g)
+                         : gallop_lower_bound(keys, s, n, bound);
+        int beg_q = __shfl_up_sync(cmask, end_q, W, 4 * W);
         if (q == 0) beg_q = s;
+        if (g != 0) continue;
         const int cx = compact_bits(P), cy = compact_bits(P >> 1);
         const int cid = base + q;
         const int cnt = end_q - beg_q;
@@ -403,8 +441,8 @@ __global__ void k_tree_children(const int *__restrict__ keys, int n, int leafcap
     }
 }
 
-static int grid_for_tree(int n, int threads) {
-    long long g = ((long long)n + threads - 1) / threads;
+static int grid_for_tree(long long n, int threads) {
+    long long g = (n + threads - 1) / threads;
     if (g > 148 * 8) g = 148 * 8;
     if (g < 1) g = 1;
     return (int)g;
@@ -496,10 +534,13 @@ int build_topology(Context &c, int leafcap) {
         return rc;
     if (ninner == 0)
         k_tree_root<<<1, 1, 0, c.stream>>>(n, tnode, range, cell);
-    else
-        k_tree_children<<<grid_for_tree(4 * (int)ninner, 128), 128, 0, c.stream>>>(
+    else {
+        const bool wide = ninner <= TC_WIDE_CELLS;
+        auto children = wide ? k_tree_children<true> : k_tree_children<false>;
+        children<<<grid_for_tree((wide ? 4 * SB_LANES : 4) * ninner, 128), 128, 0, c.stream>>>(
             keys, n, leafcap, lpos, lmask, rank, rinv, cap, (int)ninner, lo, c.nnodes, tnode, range,
             cell, err);
+    }
     TC_KERNEL_CHECK();
     return TC_OK;
 }
@@ -508,7 +549,8 @@ void kernels_tree(KernelList &v) {
     v.insert(v.end(), {(const void *)k_tree_list, (const void *)k_rank_count,
                        (const void *)k_rank_scan, (const void *)k_rank_apply,
                        (const void *)k_rank_small,
-                       (const void *)k_tree_root, (const void *)k_tree_children});
+                       (const void *)k_tree_root, (const void *)k_tree_children<true>,
+                       (const void *)k_tree_children<false>});
 }
 
 }  // namespace tc
