@@ -241,11 +241,19 @@ __global__ __launch_bounds__(LS_WARPS * 32) void k_leaf_setup_warp(
 
 // k_leaf_p2e: a_n = -1/(n+1) sum_i v_i (z_i - c)^(n+1), one warp per leaf, lanes over sources
 // with the P coefficients in registers; the 32 partial sums of each coefficient meet in shared
-// memory, transposed so that lane n adds up coefficient n.
+// memory, transposed, and are added there in parts by all lanes (LEAF_PARTS).
 template <int P, class T = double>
-struct LeafShared {
+struct alignas(16) LeafShared {
     T v[32][2 * P + 1];
 };
+
+// The 2 P columns of 32 rows are cut in PARTS each, so that all lanes take the same number of cut
+// columns (P = 24: 96, three of 16 rows each; P = 12: 96, three of 8 rows).  The mixed form is
+// bound by the conversions of these sums: with one lane per coefficient, both its columns and
+// lanes from P on idle, 64 a lane instead of 48.  16M sheet: upward phase mixed 592 -> 580 us, FP64
+// 675 -> 664.
+template <int P>
+constexpr int LEAF_PARTS = P % 16 == 0 ? 1 : P % 8 == 0 ? 2 : P % 4 == 0 ? 4 : P % 2 == 0 ? 8 : 16;
 
 
 // MIXED: the mixed-precision form accumulates in FP32 on offsets scaled by R, the power of two
@@ -259,6 +267,8 @@ __global__ __launch_bounds__(UP_WARPS * 32, MIXED ? 4 : 3) void k_leaf_p2e(
     const TNode *__restrict__ tnode, double *exps, const Frame *__restrict__ frame) {
     pdl_begin();
     using acc_t = typename std::conditional<MIXED, float, double>::type;
+    constexpr int PARTS = LEAF_PARTS<P>, TASKS = 2 * P * PARTS / 32, ROWS = 32 / PARTS;
+    static_assert(ROWS % 2 == 0 && sizeof(LeafShared<P, acc_t>) >= 32 * TASKS * sizeof(double));
     constexpr int U = MIXED ? 4 : (P > 16 ? 6 : 4);   // sources per lane in flight
     extern __shared__ __align__(16) unsigned char leaf_smem[];
     LeafShared<P, acc_t> &sh = reinterpret_cast<LeafShared<P, acc_t> *>(leaf_smem)[threadIdx.x >> 5];
@@ -369,20 +379,36 @@ __global__ __launch_bounds__(UP_WARPS * 32, MIXED ? 4 : 3) void k_leaf_p2e(
             sh.v[lane][P + n] = ai[n];
         }
         __syncwarp();
-        if (lane < P) {
-            double sr0 = 0, sr1 = 0, si0 = 0, si1 = 0;
+        double part[TASKS];
+#pragma unroll
+        for (int k = 0; k < TASKS; ++k) {
+            const int t = 32 * k + lane;
+            const acc_t *col = &sh.v[t / (2 * P) * ROWS][t % (2 * P)];
+            double s0 = 0, s1 = 0;
 #pragma unroll 8
-            for (int i = 0; i < 32; i += 2) {
-                sr0 += (double)sh.v[i][lane];
-                sr1 += (double)sh.v[i + 1][lane];
-                si0 += (double)sh.v[i][P + lane];
-                si1 += (double)sh.v[i + 1][P + lane];
+            for (int i = 0; i < ROWS; i += 2) {
+                s0 += (double)col[i * (2 * P + 1)];
+                s1 += (double)col[(i + 1) * (2 * P + 1)];
+            }
+            part[k] = s0 + s1;
+        }
+        __syncwarp();
+        double *parts = reinterpret_cast<double *>(&sh);
+#pragma unroll
+        for (int k = 0; k < TASKS; ++k) parts[32 * k + lane] = part[k];
+        __syncwarp();
+        if (lane < P) {
+            double sr = parts[lane], si = parts[P + lane];
+#pragma unroll
+            for (int h = 1; h < PARTS; ++h) {
+                sr += parts[h * 2 * P + lane];
+                si += parts[h * 2 * P + P + lane];
             }
             double fac = -1.0 / (lane + 1);
             if (MIXED) fac = ldexp(fac, e * (lane + 1));
             double *ex = exps + (size_t)node * 2 * P;
-            ex[lane] = (sr0 + sr1) * fac;
-            ex[P + lane] = (si0 + si1) * fac;
+            ex[lane] = sr * fac;
+            ex[P + lane] = si * fac;
         }
         __syncwarp();
     }
