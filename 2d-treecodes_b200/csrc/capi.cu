@@ -405,7 +405,10 @@ static int potential_device(Context &c, double theta, const double *xs, const do
     int rc;
     phase_mark(c, 0);
     c.single = single_stream(n, (m + 31) / 32) && !values_ready;
-    if ((rc = build_tree_moments(c, 0, xs, ys, vs, n, m, values_ready, xt, yt))) return rc;
+    if ((rc = build_tree_moments(c, 0, xs, ys, vs, n, m, values_ready, xt, yt))) {
+        if (c.targets_sorted) wait_stream(c, c.aux);   // it may still read the targets
+        return rc;
+    }
     if ((rc = potential(c, theta, xt, yt, m, out, expansions_then_mark))) return rc;
     phase_mark(c, 5);
     if ((rc = check_device_errors(c, "treecode_potential"))) return rc;

@@ -1239,8 +1239,9 @@ __global__ void k_scale_coeffs_pot(int nnodes, const TNode *__restrict__ tnode,
 
 static int sm_count_p() { return device_sm_count(); }
 
-// Target sort and lists run on the auxiliary stream; `between` (the expansion work) runs on the
-// main stream meanwhile, and the evaluation waits for both.
+// The lists are built on the auxiliary stream, where the target sort went before (sort_sources);
+// `between` (the expansion work) runs on the main stream meanwhile, and the evaluation waits for
+// both.
 int potential(Context &c, double theta, const double *xt, const double *yt, int m, double *out,
               OverlapFn between) {
     if (m == 0) return between ? between(c) : TC_OK;
@@ -1277,7 +1278,9 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
     TC_CUDA_TRY(stream_after(c, c.aux, c.stream, c.ev_fork));
     {
         AuxScope on_aux(c);
-        if ((rc = sort_targets(c, xt, yt, m, &vo))) return rc;
+        if (!c.targets_sorted && (rc = sort_targets(c, xt, yt, m, &c.tperm))) return rc;
+        vo = c.tperm;
+        c.targets_sorted = false;
         if ((rc = list_scratch(c, 2, nwarps, ngroups, sizeof(int2), sl, ls)) ||
             (rc = ensure(c, S_LSTART, (size_t)3 * ngroups, &sstart)))
             return rc;

@@ -1208,6 +1208,19 @@ int ctrl_prepare(Context &c, int n, int m) {
     return TC_OK;
 }
 
+// The order of a solve's targets, on the auxiliary stream from where the sources' frame is on the
+// main one (all that it needs): beside the rest of the source sort and the tree build.  After the
+// tree it delayed the lists and with them the evaluation: FP64 solves of 64K sources and targets
+// 386 -> 356 us, 131K 852 -> 819, 4M 13.19 -> 13.11 ms; mixed, 700,001 1470 -> 1430 us.
+static int targets_beside(Context &c, const double *xt, const double *yt, int m) {
+    if (!xt || m <= 0) return TC_OK;
+    TC_CUDA_TRY(stream_after(c, c.aux, c.stream, c.ev_fork));
+    AuxScope on_aux(c);
+    const int rc = sort_targets(c, xt, yt, m, &c.tperm);
+    if (rc == TC_OK) c.targets_sorted = true;
+    return rc;
+}
+
 int sort_sources(Context &c, const double *x, const double *y, const double *v, int n,
                  cudaEvent_t values_ready, const double *xt, const double *yt, int m) {
     const bool ovl = c.launch_overlap;   // launch_pdl chains (tc_set_launch_overlap)
@@ -1236,12 +1249,13 @@ int sort_sources(Context &c, const double *x, const double *y, const double *v, 
         int *tperm = nullptr;
         if (xt && c.single && m > 0 && m <= SMALL_SORT) {
             if ((rc = ensure(c, S_TPERM, m, &tperm))) return rc;
+            c.tperm = tperm;
             c.targets_sorted = true;
         }
         rc = std::max(n, tperm ? m : 0) <= 4 * SMALL_THREADS
                  ? sort_small<4>(c, x, y, v_now, n, frame, keys, perm, xs, ys, vs, xt, yt, m, tperm)
                  : sort_small<16>(c, x, y, v_now, n, frame, keys, perm, xs, ys, vs, xt, yt, m, tperm);
-        if (rc) return rc;
+        if (rc || (!c.single && (rc = targets_beside(c, xt, yt, m)))) return rc;
         c.nsrc = n;
         if (values_ready) {
             c.late_x = c.late_y = nullptr;   // x and y are sorted; v in finish_sources
@@ -1270,6 +1284,7 @@ int sort_sources(Context &c, const double *x, const double *y, const double *v, 
     unsigned *status = c.ctrl.status, *sink = c.ctrl.sink;
     k_bbox<<<gb, BBOX_THREADS, 0, c.stream>>>(x, y, n, partials, done, frame);
     TC_KERNEL_CHECK();
+    if ((rc = targets_beside(c, xt, yt, m))) return rc;
     // resident values: the records are written by the first pass, in buckets (see FirstPass);
     // values that arrive later: items in input order; x, y, v gathered by the permutation
     // in finish_sources
@@ -1356,10 +1371,6 @@ int sort_targets(Context &c, const double *xt, const double *yt, int m, int **pe
     if ((rc = ensure(c, S_TPERM, m, &tperm))) return rc;
     if (m <= SMALL_SORT) {
         *perm = tperm;
-        if (c.targets_sorted) {   // with the sources (sort_sources of this solve)
-            c.targets_sorted = false;
-            return TC_OK;
-        }
         return m <= 4 * SMALL_THREADS ? sort_small_targets<4>(c, xt, yt, m, tperm)
                                       : sort_small_targets<16>(c, xt, yt, m, tperm);
     }

@@ -154,7 +154,9 @@ struct Context {
     // a small solve: everything on `stream`, in order (single_stream); AuxScope and stream_after
     // then do nothing
     bool single = false;
-    bool targets_sorted = false;   // the solve's target order was formed with the sources'
+    // the solve's target order, formed with the sources' or beside the tree (sort_sources)
+    bool targets_sorted = false;
+    int *tperm = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_totals = nullptr, ev_join = nullptr;
     // host entry points: x/y are copied on `stream`, v (and targets) on `aux` after them;
     // ev_inputs marks v's arrival
