@@ -27,6 +27,7 @@
 #include <cfloat>
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 
 #include "tc_internal.h"
 
@@ -417,7 +418,7 @@ __global__ __launch_bounds__(256) void k_keys_pack(const double *__restrict__ x,
 // range of records, L2-resident, instead of from anywhere in HBM:
 //   * k_key_hist reads x and y once and writes the histograms of the four radix digits and of
 //     the top 8 key bits (the buckets);
-//   * k_onesweep_items<true> (the first pass) reads x, y, v, forms the keys, claims each
+//   * k_onesweep_items<.., true> (the first pass) reads x, y, v, forms the keys, claims each
 //     source a record slot in its bucket (tile counts in shared memory, one global atomic per
 //     tile and bucket) and writes the record (x, y, v, index); its items carry the record's
 //     position, key << 32 | slot;
@@ -491,28 +492,35 @@ struct FirstPass {
     int *bucket_fill;           // slots claimed per bucket so far (zeroed per sort)
 };
 
-// One onesweep pass over 8-byte items, digit (item >> shift) & 0xFF: tiles of 3072 items
-// (256 threads x 12, four CTAs per SM); the tile's digit counts, then the global digit offsets
-// by decoupled look-back, then the stable rank within each warp from digit ballots; items are
-// placed in sorted order in shared memory and written out in runs of equal digits.
+// One onesweep pass over 8-byte items, digit (item >> shift) & 0xFF: tiles of 256 threads x ITEMS;
+// the tile's digit counts, then the global digit offsets by decoupled look-back, then the stable
+// rank within each warp from digit ballots; items are placed in sorted order in shared memory and
+// written out in runs of equal digits.  ITEMS is 12 (four CTAs per SM), or 8 where that is few tiles
+// per SM and a pass lasts as long as one tile's phases (sort_tile): potential of 64K sources 359 ->
+// 352 us, force 64K 234 -> 226, 256K 392 -> 374, 1M 1014 -> 1007, potential 700,001 1437 -> 1417;
+// at 16M it is the slower one (sort 1057 -> 1128).
 // `stall_tile` (a test setting, -1 otherwise) names a tile that publishes into `sink` instead
 // of its status words, so that the tiles after it wait until `spin_limit` and report
 // DEVERR_SPIN_LIMIT.
 constexpr int PS_THREADS = 256;
 constexpr int PS_WARPS = PS_THREADS / 32;
-constexpr int PS_ITEMS = 12;
-constexpr int PS_TILE = PS_THREADS * PS_ITEMS;
+constexpr int PS_TILE = PS_THREADS * 12;         // a tile of the general form
+constexpr int PS_SMALL_TILE = PS_THREADS * 8;
+constexpr int PS_SMALL_MAX = 3 << 19;             // sources up to which tiles are the small ones
+inline int sort_tile(int n) { return n <= PS_SMALL_MAX ? PS_SMALL_TILE : PS_TILE; }
+inline int sort_tiles(int n) { return (n + sort_tile(n) - 1) / sort_tile(n); }
 
 // FIRST: the first pass of resident values (the tile's items formed from x, y, v, records
 // written to their buckets, see FirstPass); otherwise the items are read from `in`.  STALL:
 // the instance that honours stall_tile (the test setting; the others ignore it).
-template <bool FIRST, bool STALL = false>
+template <int ITEMS, bool FIRST, bool STALL = false>
 __global__ __launch_bounds__(PS_THREADS, FIRST ? 3 : 4) void k_onesweep_items(
     const unsigned long long *__restrict__ in, unsigned long long *__restrict__ out, int n,
     int shift, const int *__restrict__ digit_offsets, unsigned *status, int *tile_counter,
     unsigned *err, int spin_limit, int stall_tile, unsigned *sink, FirstPass fp) {
+    constexpr int TILE = PS_THREADS * ITEMS;
     pdl_begin();
-    __shared__ unsigned long long s_items[PS_TILE];
+    __shared__ unsigned long long s_items[TILE];
     __shared__ int s_whist[PS_WARPS][RS_RADIX];
     __shared__ int s_count[RS_RADIX];
     __shared__ int s_tile_start[RS_RADIX];
@@ -520,26 +528,31 @@ __global__ __launch_bounds__(PS_THREADS, FIRST ? 3 : 4) void k_onesweep_items(
     __shared__ int s_tile;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // the pass's digit is a whole byte of the key half: one byte permutation
+    const unsigned digit_sel = 0x4440u | (unsigned)(shift - 32) >> 3;
+    auto digit_of = [&](unsigned long long it) {
+        return (int)__byte_perm((unsigned)(it >> 32), 0u, digit_sel);
+    };
     if (tid == 0) s_tile = atomicAdd(tile_counter, 1);
     for (int i = tid; i < PS_WARPS * RS_RADIX; i += PS_THREADS) (&s_whist[0][0])[i] = 0;
     s_count[tid] = 0;
     if (FIRST) s_global[tid] = 0;   // the tile's count per bucket, first
     __syncthreads();
     const int tile = s_tile;
-    const int tile_base = tile * PS_TILE;
-    const int tile_n = min(PS_TILE, n - tile_base);
-    const int warp_base = tile_base + warp * (PS_ITEMS * 32);
+    const int tile_base = tile * TILE;
+    const int tile_n = min(TILE, n - tile_base);
+    const int warp_base = tile_base + warp * (ITEMS * 32);
 
-    unsigned long long item[PS_ITEMS];
-    int rank[PS_ITEMS];
+    unsigned long long item[ITEMS];
+    int rank[ITEMS];
     constexpr int FB = 4;   // the first pass's loads in flight
-    static_assert(PS_ITEMS % FB == 0, "whole batches");
+    static_assert(ITEMS % FB == 0, "whole batches");
     if constexpr (FIRST) {
         // keys, digit counts and each source's slot among the tile's sources of its bucket; the
         // loads are issued in batches of FB before the shared atomics that consume them
         const Frame f = *fp.frame;
 #pragma unroll
-        for (int k0 = 0; k0 < PS_ITEMS; k0 += FB) {
+        for (int k0 = 0; k0 < ITEMS; k0 += FB) {
             double xv[FB], yv[FB];
 #pragma unroll
             for (int k = 0; k < FB; ++k) {
@@ -554,21 +567,21 @@ __global__ __launch_bounds__(PS_THREADS, FIRST ? 3 : 4) void k_onesweep_items(
                 if (idx < n) {
                     key = morton_key(xv[k], yv[k], f);
                     slot = atomicAdd(&s_global[(unsigned)key >> BUCKET_SHIFT], 1);
-                    atomicAdd(&s_count[(key >> (shift - 32)) & 0xFF], 1);
+                    atomicAdd(&s_count[__byte_perm((unsigned)key, 0u, digit_sel)], 1);
                 }
                 item[k0 + k] = ((unsigned long long)(unsigned)key << 32) | (unsigned)slot;
             }
         }
     } else {
 #pragma unroll
-        for (int k = 0; k < PS_ITEMS; ++k) {
+        for (int k = 0; k < ITEMS; ++k) {
             const int idx = warp_base + k * 32 + lane;
             item[k] = idx < n ? in[idx] : 0ull;
         }
 #pragma unroll
-        for (int k = 0; k < PS_ITEMS; ++k)
+        for (int k = 0; k < ITEMS; ++k)
             if (warp_base + k * 32 + lane < n)
-                atomicAdd(&s_count[(int)(item[k] >> shift) & 0xFF], 1);
+                atomicAdd(&s_count[digit_of(item[k])], 1);
     }
     // Early counts: the tile's digit totals first (shared atomics), so that its aggregate is
     // published and the look-back done before the ranking (and the first pass's records), not
@@ -599,7 +612,7 @@ __global__ __launch_bounds__(PS_THREADS, FIRST ? 3 : 4) void k_onesweep_items(
         __syncthreads();
         // each record with one 32-byte store (one whole DRAM sector), batches of FB loads first
 #pragma unroll
-        for (int k0 = 0; k0 < PS_ITEMS; k0 += FB) {
+        for (int k0 = 0; k0 < ITEMS; k0 += FB) {
             double xv[FB], yv[FB], vv[FB];
 #pragma unroll
             for (int k = 0; k < FB; ++k) {
@@ -627,39 +640,43 @@ __global__ __launch_bounds__(PS_THREADS, FIRST ? 3 : 4) void k_onesweep_items(
 
     const unsigned lt = lanemask_lt();
     int *hist = s_whist[warp];
+    auto ranks = [&](auto full) {
 #pragma unroll
-    for (int k = 0; k < PS_ITEMS; ++k) {
-        const int idx = warp_base + k * 32 + lane;
-        const bool valid = idx < n;
-        const unsigned vmask = __ballot_sync(FULL_MASK, valid);
-        const int dk = (int)(item[k] >> shift) & 0xFF;
-        unsigned peers = digit_peers(vmask, dk);
-        if (!valid) peers = 0;
-        const int old = valid ? hist[dk] : 0;
-        __syncwarp();
-        if (valid && (peers & lt) == 0) hist[dk] = old + __popc(peers);
-        __syncwarp();
-        rank[k] = old + __popc(peers & lt);
-    }
+        for (int k = 0; k < ITEMS; ++k) {
+            const bool valid = decltype(full)::value || warp_base + k * 32 + lane < n;
+            const unsigned vmask = decltype(full)::value ? FULL_MASK : __ballot_sync(FULL_MASK, valid);
+            const int dk = digit_of(item[k]);
+            unsigned peers = digit_peers(vmask, dk);
+            if (!valid) peers = 0;
+            const int old = valid ? hist[dk] : 0;
+            __syncwarp();
+            if (valid && (peers & lt) == 0) hist[dk] = old + __popc(peers);
+            __syncwarp();
+            rank[k] = old + __popc(peers & lt);
+        }
+    };
+    const bool full_tile = tile_n == TILE;
+    if (full_tile)
+        ranks(std::true_type{});
+    else
+        ranks(std::false_type{});
     __syncthreads();
-    int run = 0;
+    const int start = block_exclusive_scan(total, nullptr);
+    int run = start;
 #pragma unroll
     for (int w = 0; w < PS_WARPS; ++w) {
         const int c = s_whist[w][d];
         s_whist[w][d] = run;
         run += c;
     }
-    const int start = block_exclusive_scan(total, nullptr);
-    s_tile_start[d] = start;
     s_global[d] = digit_offsets[d] + excl - start;
     __syncthreads();
 
 #pragma unroll
-    for (int k = 0; k < PS_ITEMS; ++k) {
-        const int idx = warp_base + k * 32 + lane;
-        if (idx < n) {
-            const int dk = (int)(item[k] >> shift) & 0xFF;
-            const int p = s_tile_start[dk] + s_whist[warp][dk] + rank[k];
+    for (int k = 0; k < ITEMS; ++k) {
+        if (full_tile || warp_base + k * 32 + lane < n) {
+            const int dk = digit_of(item[k]);
+            const int p = s_whist[warp][dk] + rank[k];
             if ((unsigned)p >= (unsigned)tile_n) {
                 atomicOr(err, DEVERR_BOUNDS);
                 continue;
@@ -669,15 +686,19 @@ __global__ __launch_bounds__(PS_THREADS, FIRST ? 3 : 4) void k_onesweep_items(
     }
     __syncthreads();
 
-#pragma unroll 4
-    for (int j = tid; j < tile_n; j += PS_THREADS) {
+    auto write = [&](int j) {
         const unsigned long long it = s_items[j];
-        const int g = s_global[(int)(it >> shift) & 0xFF] + j;
-        if ((unsigned)g >= (unsigned)n) {
+        const int g = s_global[digit_of(it)] + j;
+        if ((unsigned)g >= (unsigned)n)
             atomicOr(err, DEVERR_BOUNDS);
-            continue;
-        }
-        out[g] = it;
+        else
+            out[g] = it;
+    };
+    if (full_tile) {
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) write(tid + k * PS_THREADS);
+    } else {
+        for (int j = tid; j < tile_n; j += PS_THREADS) write(j);
     }
 }
 
@@ -1164,7 +1185,7 @@ int exclusive_scan(Context &c, const int *d_in, int *d_out, int n, int part, uns
 constexpr int NHIST = RS_MAX_PASSES + 1;
 
 int ctrl_prepare(Context &c, int n, int m) {
-    const size_t words_s = (size_t)RS_MAX_PASSES * ((n + PS_TILE - 1) / PS_TILE) * RS_RADIX;
+    const size_t words_s = (size_t)RS_MAX_PASSES * sort_tiles(n) * RS_RADIX;
     const size_t words_t = (size_t)RS_MAX_PASSES * ((m + RS_TILE - 1) / RS_TILE) * RS_RADIX;
     const size_t words_l = tree_list_tiles(n);
     unsigned *base = nullptr;
@@ -1273,7 +1294,7 @@ int sort_sources(Context &c, const double *x, const double *y, const double *v, 
     unsigned long long *items_a, *items_b;
     double2 *rec;
     const int npasses = (2 * LMAX + 7) / 8;
-    const int ntiles = (n + PS_TILE - 1) / PS_TILE;
+    const int ntiles = sort_tiles(n);
     if ((rc = ensure(c, S_ITEMS_A, n, &items_a)) || (rc = ensure(c, S_ITEMS_B, n, &items_b)) ||
         (rc = ensure(c, S_REC, 2 * (size_t)n, &rec)))
         return rc;
@@ -1305,11 +1326,16 @@ int sort_sources(Context &c, const double *x, const double *y, const double *v, 
     for (int p = 0; p < npasses; ++p) {
         const bool odd = p & 1;
         const int stall = p == 0 && c.test_stall == TC_STALL_SORT ? 0 : -1;
-        auto pass = p == 0 ? (bucketed ? (stall >= 0 ? k_onesweep_items<true, true>
-                                                   : k_onesweep_items<true, false>)
-                                       : (stall >= 0 ? k_onesweep_items<false, true>
-                                                     : k_onesweep_items<false, false>))
-                           : k_onesweep_items<false, false>;
+        auto pass_of = [&](auto tile) {
+            constexpr int ITEMS = decltype(tile)::value / PS_THREADS;
+            if (p > 0) return k_onesweep_items<ITEMS, false>;
+            if (stall >= 0)
+                return bucketed ? k_onesweep_items<ITEMS, true, true>
+                                : k_onesweep_items<ITEMS, false, true>;
+            return bucketed ? k_onesweep_items<ITEMS, true> : k_onesweep_items<ITEMS, false>;
+        };
+        auto pass = sort_tile(n) == PS_TILE ? pass_of(std::integral_constant<int, PS_TILE>{})
+                                            : pass_of(std::integral_constant<int, PS_SMALL_TILE>{});
         TC_CUDA_TRY(launch_pdl(ovl, pass, ntiles, PS_THREADS, 0, c.stream,
                                (const unsigned long long *)(odd ? items_b : items_a),
                                odd ? items_a : items_b, n, 32 + 8 * p,
@@ -1432,10 +1458,14 @@ void kernels_sort(KernelList &v) {
                        (const void *)k_gather_items_inplace, (const void *)k_hist,
                        (const void *)k_hist_scan,
                        (const void *)k_onesweep, (const void *)k_keys_pack,
-                       (const void *)k_onesweep_items<true>,
-                       (const void *)k_onesweep_items<false>, (const void *)k_key_hist,
-                       (const void *)k_onesweep_items<true, true>,
-                       (const void *)k_onesweep_items<false, true>,
+                       (const void *)k_onesweep_items<12, true>,
+                       (const void *)k_onesweep_items<12, false>, (const void *)k_key_hist,
+                       (const void *)k_onesweep_items<12, true, true>,
+                       (const void *)k_onesweep_items<12, false, true>,
+                       (const void *)k_onesweep_items<8, true>,
+                       (const void *)k_onesweep_items<8, false>,
+                       (const void *)k_onesweep_items<8, true, true>,
+                       (const void *)k_onesweep_items<8, false, true>,
                        (const void *)k_gather_sources, (const void *)k_gather_xy,
                        (const void *)k_gather_v, (const void *)k_items_split,
                        (const void *)k_scan_reduce, (const void *)k_scan_blocks,
@@ -1508,7 +1538,7 @@ extern "C" TC_API int tc_sort_sources_noalloc(const double *xsources, const doub
     static_assert((2 * LMAX + 7) / 8 % 2 == 0, "an even number of passes ends in items_a");
     for (int p = 0; p < npasses; ++p) {
         const bool odd = p & 1;
-        k_onesweep_items<false><<<ntiles, PS_THREADS, 0, s>>>(
+        k_onesweep_items<12, false><<<ntiles, PS_THREADS, 0, s>>>(
             odd ? items_b : items_a, odd ? items_a : items_b, n, 32 + 8 * p,
             offsets + p * RS_RADIX, status + (size_t)p * ntiles * RS_RADIX, counter + p, err,
             RS_SPIN_LIMIT, -1, nullptr, FirstPass{});

@@ -85,3 +85,22 @@ def test_sources_and_targets_sorted_side_by_side(n):
         ctx.potential_device(0.5, *d, *t, out)
         T.Context().direct_potential_device(*d, *t, ref)
         assert float((out - ref).norm()) < 1e-5 * float(ref.norm()), m
+
+
+@pytest.mark.parametrize("n", [16385, 18431, 18432, 18433, 1048577, 1572863, 1572864, 1572865,
+                               1575936, 1575937])
+def test_general_sort_is_stable_at_the_tiles_edges(n):
+    """Both tile sizes of the radix passes, around whole tiles and the size where they change."""
+    import torch
+    import treecodes as T
+
+    x, y, v = inputs(n, n)
+    d = [torch.tensor(a, device="cuda") for a in (x, y, v)]
+    torch.cuda.synchronize()
+    t = T.Context().tree("potential", *d)
+    assert np.array_equal(np.sort(t["perm"]), np.arange(n))
+    keys = np.empty(n, t["keys"].dtype)
+    keys[t["perm"]] = t["keys"]
+    assert np.array_equal(t["perm"], np.argsort(keys, kind="stable"))
+    for name, a in (("xs", x), ("ys", y), ("vs", v)):
+        assert np.array_equal(t[name], a[t["perm"]]), name
