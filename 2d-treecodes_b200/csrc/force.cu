@@ -5,21 +5,24 @@
 // (P2P, E2P, E2L, L2P).  An MRAG block of 32 x 32 targets is 16 bricks of 8 x 8
 // (treecode-force.cpp:110-111), brick q = (by/8)*4 + bx/8.
 //
-// 1. k_force_lists<false>: one warp per brick walks the tree 32 nodes at a time and classifies
+// 1. k_force_lists<2>: one warp per brick walks the tree 32 nodes at a time and classifies
 //    every node with the reference's two criteria (treecode-force.cpp:136-151):
 //      E2L  iff  dist(brick centre, com)/r - 1 > 1/theta  and  r_brick <= r
 //      E2P  iff  r^2 < theta^2 |clamp(com to brick) - com|^2
 //      else P2P for a leaf, descend for an inner node.
-//    Counts per brick and kind are compacted with warp ballots.  The arithmetic is the one
+//    Entries are compacted with warp ballots into per-warp scratch runs.  The arithmetic is the one
 //    the compiled reference executes (fma(dx, dx, dy*dy), brick centre fma(bx + 3.5, h, x0),
 //    r_brick = 4.949747468305833 h), so every decision is the reference's.
 // 2. exclusive scan of the 3 x nbricks counts -> list offsets (E2L | E2P | P2P lists).
-// 3. k_force_lists<true>: same walk, writes node ids into the lists.
-// 4. k_force_far: persistent warps over bricks, 2 targets per lane; local expansion from the
+// 3. k_force_lists_copy puts the runs in CSR order (k_force_lists<1>, a second walk, where a run
+//    outgrew its region).
+// 4. k_force_far: persistent warps over bricks (few bricks: a block per brick, its E2L done before
+//    by k_force_e2l), the ones with most work first, 2 targets per lane; local expansion from the
 //    E2L list (lane l owns coefficient l), L2P, E2P from the E2P list, written into the
 //    ix + 32*(iy + 32*ib) layout (treecode-force.cpp:191-197).
 // 5. k_force_near: persistent warps over tasks, a task being a segment of at most P2P_SEG
-//    sources of a brick's P2P list; P2P over the listed leaves with source tiles staged in
+//    sources of a brick's P2P list (fewer where bricks are few), the longest first where they
+//    are many; P2P over the listed leaves with source tiles staged in
 //    shared memory.  Single-task bricks add their sums to the outputs; the parts of multi-task
 //    bricks are added in task order by k_force_gather_parts, so results are deterministic.
 #include <cfloat>

@@ -10,8 +10,9 @@
 // Targets are first sorted by Morton key (in the sources' frame) so that the 32 targets of a
 // warp are neighbours and the masks are mostly full.
 //
-// Lists are (node, lane mask) pairs in CSR form per group of 32 targets, built by a counting
-// walk, a scan, and a filling walk.
+// Lists are (node, lane mask) pairs in CSR form per group of 32 targets: one walk writes them into
+// per-warp scratch runs, a scan and a copy put them in order (a second walk fills them where a
+// run outgrew its region).
 #include <cfloat>
 #include <cmath>
 

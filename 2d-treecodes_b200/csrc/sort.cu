@@ -17,6 +17,8 @@
 // (key << 32 | index) and the histograms, four passes sort them, k_items_split writes keys and
 // permutation, k_gather_xy the sorted x and y, and k_gather_v the sorted v once it is in.
 //
+// Up to 16,384 sources (SMALL_SORT) all of it is one block and one launch, k_sort_small.
+//
 // The radix sort is a one-pass-per-digit ("onesweep") LSD sort: every CTA counts the digits of
 // a tile of items, finds its global digit offsets by a decoupled look-back over the tiles
 // before it, ranks the tile in shared memory with warp digit ballots and writes it out in

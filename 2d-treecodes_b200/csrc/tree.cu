@@ -360,7 +360,7 @@ __global__ void k_tree_root(int n, TNode *tnode, int2 *range, int4 *cell) {
 // writes child q.  Bound by the latency of dependent reads: with WIDE the tree phase takes 38 -> 32
 // us for the potential of 64K sources, 56 -> 46 for the force of 1M (4,080 cells).  With more
 // cells than resident warps the wide search's extra reads count: 15,000 cells 76 -> 72 us, 30,000
-// 97 -> 105, 59,000 150 -> 174 us.
+// 88 -> 105, 59,000 143 -> 174 us.
 constexpr int TC_WIDE_CELLS = 16384;   // up to here WIDE
 
 template <bool WIDE>
