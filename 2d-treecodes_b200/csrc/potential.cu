@@ -261,14 +261,16 @@ __global__ __launch_bounds__(PLOC_WARPS * 32) void k_potential_locals(
             const TNode nd = tnode[mine];
             const double zx = nd.xcom - geo.x, zy = nd.ycom - geo.y;
             const double r2 = zx * zx + zy * zy;
-            const double iz = R * rcp_nr(r2);
+            // (where the square nears or passes the top of the number range, R / z0 < 1e-140 counts
+            // for nothing, and the logarithm of an overflow is that of the top)
+            const double iz = r2 < 1e300 ? R * rcp_nr(r2) : 0.0;
             const cplx u = {zx * iz, -zy * iz};
             const cplx u2 = cmul(u, u);
             cplx p = half ? u2 : u;
             __syncwarp();
             if (half) {
                 sh.mass[c] = mass[mine];
-                sh.log[c] = 0.5 * log(r2);
+                sh.log[c] = 0.5 * log(fmin(r2, DBL_MAX));
             }
 #pragma unroll
             for (int q = 0; q < PS_TERMS / 2; ++q) {
@@ -312,19 +314,22 @@ __global__ __launch_bounds__(PLOC_WARPS * 32) void k_potential_locals(
 // warp's entries into its own scratch region (ScratchLayout), recording where each group's run
 // starts, so that a copy into CSR order replaces a second walk.  A region that fills up sets
 // meta[0] (the host then falls back to MODE 1); meta[1 + k] receives the longest run of kind
-// k any warp wrote, and the work counters are added.
+// k any warp wrote, and the work counters are added.  meta[META_WIDE] is set where a group's targets
+// may be NEAR_REACH or more away from a source (every source is in `frame`).
+constexpr int META_WIDE = 3;
 template <int MODE>
 __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
     int ngroups, int m, const double *__restrict__ xt, const double *__restrict__ yt,
     const int *__restrict__ tperm, double theta, const TNode *__restrict__ tnode, int nnodes,
     int *__restrict__ counts, const int *__restrict__ offs, int2 *__restrict__ lists,
     int2 *__restrict__ scratch, ScratchLayout sl, int *__restrict__ sstart, int *meta,
-    unsigned *err, unsigned long long *stats, int seg, SuperSets sets) {
+    unsigned *err, unsigned long long *stats, int seg, SuperSets sets,
+    const Frame *__restrict__ frame) {
     pdl_begin();
     constexpr bool FILL = MODE == 1;
     const int wglob = blockIdx.x * PT_WARPS + (threadIdx.x >> 5);
     int cur[2] = {0, 0};   // MODE 2: entries this warp has written, per kind
-    bool full = false;
+    bool full = false, wide = false;
     __shared__ int2 stack_all[PT_WARPS][PL_STACK];
     const int lane = lane_id(), warp = threadIdx.x >> 5;
     int2 *stack = stack_all[warp];
@@ -350,6 +355,12 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
             bxhi = fmax(bxhi, __shfl_xor_sync(FULL_MASK, bxhi, o));
             bylo = fmin(bylo, __shfl_xor_sync(FULL_MASK, bylo, o));
             byhi = fmax(byhi, __shfl_xor_sync(FULL_MASK, byhi, o));
+        }
+        if (MODE == 2) {
+            const double fx = frame->xmin, fy = frame->ymin, fe = frame->ext;
+            const double reach = fmax(fmax(bxhi - fx, fx + fe - bxlo),
+                                      fmax(byhi - fy, fy + fe - bylo));
+            wide = wide || !(reach < NEAR_REACH);   // (no finite target: also wide)
         }
         int o0 = 0, o1 = 0, l0 = 0, l1 = 0;
         if (FILL) {
@@ -511,6 +522,7 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
         if (lane == 0) {
             atomicMax(&meta[1], cur[0]);
             atomicMax(&meta[2], cur[1]);
+            if (wide) atomicOr(&meta[META_WIDE], 1);
         }
     }
     if (MODE == 2 && stats && lane == 0) {
@@ -933,8 +945,12 @@ constexpr size_t eval_smem() {
     return sizeof(double2) * NLOG_NTAB * NLOG_COPIES + sizeof(EvalShared<P>) * PD_WARPS;
 }
 
-// SETS: the groups' common far field is added from their set's local expansion.
-template <int P, bool SETS>
+// SETS: the groups' common far field is added from their set's local expansion (`local`, null where
+// there are no sets).
+// WIDE: for solves with a target NEAR_REACH or more away from a source, whose squares may pass
+// log_near's range or overflow: log_pos, whose logarithm of infinity is 1024 ln 2, and a true
+// division (the arithmetic of the kernel before log_near).
+template <int P, bool SETS, bool WIDE>
 __global__ __launch_bounds__(PD_WARPS * 32, PD_MIN_BLOCKS) void k_potential_eval(
     int ngroups, int m, const double *__restrict__ xt, const double *__restrict__ yt,
     const int *__restrict__ tperm, const TNode *__restrict__ tnode,
@@ -946,7 +962,11 @@ __global__ __launch_bounds__(PD_WARPS * 32, PD_MIN_BLOCKS) void k_potential_eval
     const double4 *__restrict__ geo, const cplx *__restrict__ local) {
     extern __shared__ __align__(16) unsigned char eval_dyn[];
     double2 *s_tab = reinterpret_cast<double2 *>(eval_dyn);
-    load_near_log_table(s_tab);   // (a constant table: before the kernel before this one is done)
+    double *s_neg_log_c = reinterpret_cast<double *>(eval_dyn);
+    static_assert(sizeof(double) * LOG_NTAB <= sizeof(double2) * NLOG_NTAB * NLOG_COPIES, "");
+    // (constant tables: before the kernel before this one is done)
+    if constexpr (WIDE) load_log_table(s_neg_log_c);
+    else load_near_log_table(s_tab);
     pdl_begin();
     const int lane = lane_id(), warp = threadIdx.x >> 5;
     const unsigned tab = shared_address(s_tab);
@@ -954,6 +974,10 @@ __global__ __launch_bounds__(PD_WARPS * 32, PD_MIN_BLOCKS) void k_potential_eval
     EvalShared<P> &sh =
         reinterpret_cast<EvalShared<P> *>(s_tab + NLOG_NTAB * NLOG_COPIES)[warp];
     const double eps = 10 * DBL_EPSILON;
+    auto log_of = [&](double r2) {
+        if constexpr (WIDE) return log_pos(r2, s_neg_log_c);
+        else return log_near(r2, tab, copy);
+    };
     const int *toff = offs + 2 * ngroups;
     const int tbase = toff[0];
     const int ntasks = toff[ngroups] - tbase;
@@ -987,7 +1011,7 @@ __global__ __launch_bounds__(PD_WARPS * 32, PD_MIN_BLOCKS) void k_potential_eval
         // entry's cell record and coefficients are loaded while the current one is evaluated.
         if (part == 0) {
             const int b0 = offs[g], e0 = offs[g + 1];
-            if constexpr (SETS) {   // the set's common far field: Re sum_l L_l R^l ((t - c) / R)^l
+            if (SETS && (!WIDE || local)) {   // the set's common far field: Re sum_l L_l R^l ((t - c) / R)^l
                 const double4 q4 = geo[g / PS_GROUPS];
                 __syncwarp();
                 sh.coef[lane] = local[(size_t)(g / PS_GROUPS) * PS_TERMS + lane];
@@ -1024,13 +1048,12 @@ __global__ __launch_bounds__(PD_WARPS * 32, PD_MIN_BLOCKS) void k_potential_eval
                 if ((ent.y >> lane) & 1) {
                     const double rz = x - nd.xcom, iz = y - nd.ycom;
                     const double r2 = rz * rz + iz * iz;
-                    // (the bound keeps the reciprocal's Newton steps finite when r2 overflows)
-                    const double inv = rcp_nr(fmin(r2, 1e300));
+                    const double inv = WIDE ? 1.0 / r2 : rcp_nr(r2);
                     const cplx u = {rz * inv, -iz * inv};
                     cplx q = sh.coef[P - 1];
 #pragma unroll
                     for (int k = P - 2; k >= 0; --k) q = cfma(q, u, sh.coef[k]);
-                    far += mm * log_near(r2, tab, copy) * 0.5 + (u.re * q.re - u.im * q.im);
+                    far += mm * log_of(r2) * 0.5 + (u.re * q.re - u.im * q.im);
                 }
             }
         }
@@ -1126,8 +1149,8 @@ __global__ __launch_bounds__(PD_WARPS * 32, PD_MIN_BLOCKS) void k_potential_eval
                             const double2 v = v2[q >> 1];
                             const double xr = x - sp.x, yr = y - sp.y;
                             const double xq = x - sq.x, yq = y - sq.y;
-                            n0 = fma(log_near(fma(xr, xr, fma(yr, yr, eps)), tab, copy), v.x, n0);
-                            n1 = fma(log_near(fma(xq, xq, fma(yq, yq, eps)), tab, copy), v.y, n1);
+                            n0 = fma(log_of(fma(xr, xr, fma(yr, yr, eps))), v.x, n0);
+                            n1 = fma(log_of(fma(xq, xq, fma(yq, yq, eps))), v.y, n1);
                         }
                         near += n0 + n1;
                     }
@@ -1149,8 +1172,7 @@ __global__ __launch_bounds__(PD_WARPS * 32, PD_MIN_BLOCKS) void k_potential_eval
                         for (int q = sq; q < cnt; q += r) {
                             const double2 sp = sh.src.xy[q];
                             const double xr = qx - sp.x, yr = qy - sp.y;
-                            sum = fma(log_near(fma(xr, xr, fma(yr, yr, eps)), tab, copy),
-                                      sh.src.v[q], sum);
+                            sum = fma(log_of(fma(xr, xr, fma(yr, yr, eps))), sh.src.v[q], sum);
                         }
                     sh.part[lane] = sum;
                     __syncwarp();
@@ -1306,7 +1328,8 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
         TC_CUDA_TRY(launch_pdl(c.launch_overlap, k_potential_lists<2>, grid, PT_WARPS * 32, 0,
                                c.stream, ngroups, m, xt, yt, (const int *)vo, theta, tnode, c.nnodes,
                                counts, (const int *)nullptr, (int2 *)nullptr,
-                               static_cast<int2 *>(ls.p), sl, sstart, meta, err, stats, seg, sets));
+                               static_cast<int2 *>(ls.p), sl, sstart, meta, err, stats, seg, sets,
+                               (const Frame *)slot_ptr<Frame>(c, S_FRAME)));
         TC_KERNEL_CHECK();
         // the lists' totals and meta, written to h_pinned by the scan
         if ((rc = exclusive_scan(c, counts, offs, 3 * ngroups, ngroups, c.h_pinned + 32, meta)))
@@ -1321,6 +1344,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
     const int n_e2p = (int)c.h_pinned[32], total = (int)c.h_pinned[33];
     const int ntasks = (int)c.h_pinned[34] - total;
     const bool overflow = c.h_pinned[35] != 0;
+    const bool wide = c.h_pinned[35 + META_WIDE] != 0;
     c.list_walks = overflow ? 2 : 1;
     scratch_learn(c, 2, nwarps, ngroups, c.h_pinned + 36);   // for the next solve
     c.counts.n_e2p = n_e2p;
@@ -1346,7 +1370,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
             // (the second walk does not add to the work counters)
             k_potential_lists<1><<<grid, PT_WARPS * 32, 0, c.stream>>>(
                 ngroups, m, xt, yt, vo, theta, tnode, c.nnodes, nullptr, offs, lists, nullptr,
-                sl, nullptr, nullptr, err, stats, seg, sets);
+                sl, nullptr, nullptr, err, stats, seg, sets, nullptr);
             TC_KERNEL_CHECK();
             k_task_map_groups<<<(int)std::min<long long>((ngroups + 255) / 256,
                                                          (long long)sm_count_p() * 8),
@@ -1393,18 +1417,22 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
                 out, partial, task_ctr, tt, (const float2 *)sexp,
                 (const float *)sscale));
         } else {
-            static const cudaError_t attr_rc[2] = {
-                cudaFuncSetAttribute(k_potential_eval<P, false>,
+            static const cudaError_t attr_rc[3] = {
+                cudaFuncSetAttribute(k_potential_eval<P, false, false>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)eval_smem<P>()),
-                cudaFuncSetAttribute(k_potential_eval<P, true>,
+                cudaFuncSetAttribute(k_potential_eval<P, true, false>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)eval_smem<P>()),
+                cudaFuncSetAttribute(k_potential_eval<P, true, true>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)eval_smem<P>())};
-            TC_CUDA_TRY(attr_rc[0]);
-            TC_CUDA_TRY(attr_rc[1]);
-            auto eval = with_sets ? k_potential_eval<P, true> : k_potential_eval<P, false>;
+            for (const cudaError_t e : attr_rc) TC_CUDA_TRY(e);
+            auto eval = wide        ? k_potential_eval<P, true, true>
+                        : with_sets ? k_potential_eval<P, true, false>
+                                    : k_potential_eval<P, false, false>;
             const int occ =
-                blocks_per_sm<k_potential_eval<P, false>>(PD_WARPS * 32, eval_smem<P>());
+                blocks_per_sm<k_potential_eval<P, false, false>>(PD_WARPS * 32, eval_smem<P>());
             const int egrid = (int)std::min<long long>((ntasks + PD_WARPS - 1) / PD_WARPS,
                                                        (long long)sm_count_p() * occ);
             phase_mark(c, 6);
@@ -1448,8 +1476,9 @@ void kernels_potential(KernelList &v) {
                        (const void *)k_potential_gather_parts, (const void *)k_potential_supers});
 #define TC_POTENTIAL_KERNELS(P)                                                                  \
     v.insert(v.end(), {(const void *)k_potential_eval_mixed<P>,                              \
-                       (const void *)k_potential_eval<P, false>,                                 \
-                       (const void *)k_potential_eval<P, true>,                                  \
+                       (const void *)k_potential_eval<P, false, false>,                          \
+                       (const void *)k_potential_eval<P, true, false>,                           \
+                       (const void *)k_potential_eval<P, true, true>,                            \
                        (const void *)k_potential_locals<P>,                                      \
                        (const void *)k_scale_coeffs_pot<P>});
     TC_FOR_EACH_ORDER(TC_POTENTIAL_KERNELS)

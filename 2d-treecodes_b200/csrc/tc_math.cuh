@@ -73,9 +73,15 @@ __device__ __forceinline__ void load_log_table(double *s_neg_log_c) {
 // FP64 instruction takes two issue slots, so both kinds count.)  The table stands in shared
 // memory NLOG_COPIES times, copy k of entry i at 8 i + k, and a lane reads copy lane % 8: the eight
 // lanes that a 16-byte shared load serves at once then never meet in a bank.
-// fit_near_log_table.py beside this file writes the table; any positive normal x; within 2 ulp
-// of the exact logarithm (tests/test_near_log_table.py).
+// fit_near_log_table.py beside this file writes the table.  Any x from 2^-1022 up to 2^NLOG_TOP: c's
+// exponent field (1022 or 1023) less x's exponent stays that of a normal number, and from 2^1022 on it
+// would not.  Within 2 ulp of the exact logarithm (tests/test_near_log_table.py,
+// tests/test_potential_reach.py).
 constexpr int NLOG_COPIES = 8;
+constexpr int NLOG_TOP = 1020;
+// Squared distances stay below 2^NLOG_TOP where targets and sources differ by less than this in x
+// and in y: 2 (2^509)^2 = 2^1019.
+constexpr double NEAR_REACH = 0x1p509;
 
 // `tab`: the table's 32-bit shared-memory address; `copy`: the lane's copy, 16 (lane % 8).
 __device__ __forceinline__ unsigned shared_address(const void *p) {
