@@ -457,7 +457,7 @@ __device__ __forceinline__ local_t<MIXED> brick_local(
             const int mine = lists[b0 + min(lane & (E2L_BATCH - 1), nb - 1)];
             const TNode nd = tnode[mine];
             const double zx = nd.xcom - b.x0b, zy = nd.ycom - b.y0b;
-            const double iz = rcp_nr(zx * zx + zy * zy);
+            const double iz = rcp_any(zx * zx + zy * zy);
             const cplx u = {zx * iz, -zy * iz};
             const cplx u2 = cmul(u, u);
             cplx p = half ? u2 : u;

@@ -94,6 +94,12 @@ __device__ __forceinline__ double rcp_nr(double d) {
     return fma(y, t, y);
 }
 
+// 1 / d for any d: rcp_nr where the approximation and its correction stay in the number range
+// (rcp_nr turns an infinite square into NaN and flushes 1 / d from d = 2^1022 on).
+__device__ __forceinline__ double rcp_any(double d) {
+    return d > 1e-300 && d < 1e300 ? rcp_nr(d) : 1.0 / d;
+}
+
 __device__ __forceinline__ double shfl_xor_d(double v, int m) {
     return __shfl_xor_sync(FULL_MASK, v, m);
 }

@@ -589,8 +589,7 @@ __device__ __forceinline__ void merge_geom(MergeGeom &g, int r, int lo, int mid,
 #pragma unroll
     for (int c = 0; c < 4; ++c) {   // (unused with three or four negligible children)
         const double x0 = cxc[c] - px, y0 = cyc[c] - py;
-        // (the bound keeps the reciprocal's step finite when the square overflows)
-        const double iz = rcp_nr(fmin(x0 * x0 + y0 * y0, 1e300));
+        const double iz = rcp_any(x0 * x0 + y0 * y0);
         g.zl[c] = cpow_int({x0 * iz, -y0 * iz}, lane < P ? lane + 1 : 1);
     }
 }
