@@ -816,8 +816,8 @@ __global__ __launch_bounds__(EV_WARPS * 32, WPB > 1 ? (MIXED ? 8 : 5) : (MIXED ?
 // P2P (force-kernels.m4:15-55): sum v (xr, yr) / (xr^2 + yr^2 + eps) over the sources of a
 // task's segment.  Both forms take one reciprocal per source for both of the lane's targets,
 // 1/d0 = d1 / (d0 d1).
-//  * MIXED = false: FP64, the reciprocal refined by two Newton steps (the squared separations
-//    are at least eps and, for coordinates below ~1e70, their product stays far from the
+//  * MIXED = false: FP64, the reciprocal refined by one third-order step (the squared separations
+//    are at least eps and, for separations below ~1e70, their product stays far from the
 //    double range's ends).
 //  * MIXED = true: FP32 pairs on offsets from the brick corner (each source's offset to every
 //    target column and row formed once per tile from float hi + lo parts, so the separation
@@ -922,11 +922,18 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
         int t0, tn;
         next_tile(t0, tn);
         double px = 0, py = 0, pv = 0;
-        if (lane < tn) {
-            px = xs[t0 + lane];
-            py = ys[t0 + lane];
-            pv = vs[t0 + lane];
-        }
+        // The lanes past the tile hold its last source, with no value, so that steps may take two
+        // sources at a time: any other place could be so far from the targets that a square
+        // overflows and 0 times infinity enters the sums.
+        auto load = [&] {
+            if (tn > 0) {
+                const int at = t0 + min(lane, tn - 1);
+                px = xs[at];
+                py = ys[at];
+                pv = lane < tn ? vs[at] : 0.0;
+            }
+        };
+        load();
         if constexpr (MIXED) {
             const float epsf = (float)eps;
             const float2 eps2 = make_float2(epsf, epsf);
@@ -938,13 +945,10 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
                 {
                     // offsets of source `lane` from every target column / row: (c h - q) with
                     // q = source - corner, both as float hi + lo, two columns (rows) per f32x2
-                    // instruction; slots past the tile get a zero value (their offsets, of an
-                    // earlier source or of the origin, stay finite and their separations at
-                    // least eps), so steps may take two sources at a time
+                    // instruction
                     float qxh, qxl, qyh, qyl;
                     split_f32(px - b.xlo, qxh, qxl);
                     split_f32(py - b.ylo, qyh, qyl);
-                    const bool live = lane < cnt;
                     const float2 nqxh = make_float2(-qxh, -qxh), nqxl = make_float2(-qxl, -qxl);
                     const float2 nqyh = make_float2(-qyh, -qyh), nqyl = make_float2(-qyl, -qyl);
                     const float2 *ch2 = reinterpret_cast<const float2 *>(sh.ch);
@@ -959,15 +963,11 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
                         sh.dy[c][lane] = dy.x;
                         sh.dy[c + 1][lane] = dy.y;
                     }
-                    sh.v[lane] = live ? (float)pv : 0.f;
+                    sh.v[lane] = (float)pv;
                 }
                 __syncwarp();
                 next_tile(t0, tn);
-                if (lane < tn) {
-                    px = xs[t0 + lane];
-                    py = ys[t0 + lane];
-                    pv = vs[t0 + lane];
-                }
+                load();
                 const float4 *dxr = reinterpret_cast<const float4 *>(sh.dx[tx]);
                 const float4 *dyr0 = reinterpret_cast<const float4 *>(sh.dy[ty]);
                 const float4 *dyr1 = reinterpret_cast<const float4 *>(sh.dy[ty + 4]);
@@ -1010,17 +1010,11 @@ __global__ __launch_bounds__(EV_WARPS * 32, NEAR_MIN_BLOCKS) void k_force_near(
             while (tn > 0) {
                 const int cnt = tn;
                 __syncwarp();
-                // (a zero value at the origin past the tile, for the two-source steps)
-                const bool live = lane < cnt;
-                sh.sxy[lane] = make_double2(live ? px : 0.0, live ? py : 0.0);
-                sh.sv[lane] = live ? pv : 0.0;
+                sh.sxy[lane] = make_double2(px, py);
+                sh.sv[lane] = pv;
                 __syncwarp();
                 next_tile(t0, tn);
-                if (lane < tn) {
-                    px = xs[t0 + lane];
-                    py = ys[t0 + lane];
-                    pv = vs[t0 + lane];
-                }
+                load();
                 auto pair = [&](double2 sp, double v) {
                     const double xr = xt - sp.x;
                     const double xr2e = fma(xr, xr, eps);
