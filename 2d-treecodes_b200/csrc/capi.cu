@@ -235,7 +235,8 @@ static void context_counted(int device, int delta) {
 // (the CUDA default) a kernel is loaded at its first launch, and loading may synchronise the
 // whole device: in the request server, the first solve of a form, order or list-walk mode not
 // seen before stalled every concurrent solve.  Querying each kernel's attributes loads it, so
-// the first context pays that cost at start-up instead.
+// the first context pays that cost at start-up instead.  Attributes are set here too: they hold for
+// the current device alone.
 static int preload_kernels(int device) {
     static std::mutex mu;
     static std::vector<int> loaded;
@@ -252,7 +253,10 @@ static int preload_kernels(int device) {
         cudaFuncAttributes a;
         TC_CUDA_TRY(cudaFuncGetAttributes(&a, k));
     }
-    if (int rc = prefer_force_carveout()) return rc;
+    int rc;
+    if ((rc = prepare_sort()) || (rc = prepare_upward()) || (rc = prepare_force()) ||
+        (rc = prepare_potential()))
+        return rc;
     loaded.push_back(device);
     return TC_OK;
 }

@@ -1438,7 +1438,7 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
 // solve started after the near field instead of beside it.  Preferring half of the SM's memory as
 // shared costs the near field nothing alone: FP64 solves of 64K sources 264 -> 253 us, 1M 1374 ->
 // 1338 us, 16M 3670 -> 3627 us.  (The mixed kernels need less, and gain nothing.)
-int prefer_force_carveout() {
+int prepare_force() {
     for (const void *k :
          {(const void *)k_force_near<false, 5, false>, (const void *)k_force_near<false, 0, false>,
           (const void *)k_force_near<false, 5, true>, (const void *)k_force_near<false, 0, true>})

@@ -1417,17 +1417,6 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
                 out, partial, task_ctr, tt, (const float2 *)sexp,
                 (const float *)sscale));
         } else {
-            static const cudaError_t attr_rc[3] = {
-                cudaFuncSetAttribute(k_potential_eval<P, false, false>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)eval_smem<P>()),
-                cudaFuncSetAttribute(k_potential_eval<P, true, false>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)eval_smem<P>()),
-                cudaFuncSetAttribute(k_potential_eval<P, true, true>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)eval_smem<P>())};
-            for (const cudaError_t e : attr_rc) TC_CUDA_TRY(e);
             auto eval = wide        ? k_potential_eval<P, true, true>
                         : with_sets ? k_potential_eval<P, true, false>
                                     : k_potential_eval<P, false, false>;
@@ -1467,6 +1456,18 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
             c.stream, ngroups, m, (const int *)vo, (const int *)offs, (const double *)partial, out));
         TC_KERNEL_CHECK();
     }
+    return TC_OK;
+}
+
+int prepare_potential() {
+    int rc;
+#define TC_EVAL_SHARED(P)                                                                         \
+    if ((rc = allow_shared((const void *)k_potential_eval<P, false, false>, eval_smem<P>())) ||   \
+        (rc = allow_shared((const void *)k_potential_eval<P, true, false>, eval_smem<P>())) ||    \
+        (rc = allow_shared((const void *)k_potential_eval<P, true, true>, eval_smem<P>())))       \
+        return rc;
+    TC_FOR_EACH_ORDER(TC_EVAL_SHARED)
+#undef TC_EVAL_SHARED
     return TC_OK;
 }
 

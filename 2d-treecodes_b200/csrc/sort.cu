@@ -978,9 +978,6 @@ template <int ITEMS>
 static int sort_small(Context &c, const double *x, const double *y, const double *v, int n,
                       Frame *frame, int *keys, int *perm, double *xs, double *ys, double *vs,
                       const double *xt, const double *yt, int nt, int *tperm) {
-    static const cudaError_t attr_rc = cudaFuncSetAttribute(
-        k_sort_small<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem<ITEMS>());
-    TC_CUDA_TRY(attr_rc);
     k_sort_small<ITEMS><<<tperm ? 2 : 1, SMALL_THREADS, small_smem<ITEMS>(), c.stream>>>(
         x, y, v, n, frame, keys, perm, xs, ys, vs, xt, yt, nt, tperm);
     TC_KERNEL_CHECK();
@@ -989,10 +986,6 @@ static int sort_small(Context &c, const double *x, const double *y, const double
 
 template <int ITEMS>
 static int sort_small_targets(Context &c, const double *x, const double *y, int n, int *perm) {
-    static const cudaError_t attr_rc =
-        cudaFuncSetAttribute(k_sort_small_targets<ITEMS>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem<ITEMS>());
-    TC_CUDA_TRY(attr_rc);
     TC_CUDA_TRY(launch_pdl(c.launch_overlap && c.single, k_sort_small_targets<ITEMS>, 1,
                            SMALL_THREADS, small_smem<ITEMS>(), c.stream, x, y, n,
                            (const Frame *)slot_ptr<Frame>(c, S_FRAME), perm));
@@ -1453,6 +1446,16 @@ static unsigned char *noalloc_scratch_base(int device) {
         addr[device] = p;
     }
     return static_cast<unsigned char *>(addr[device]);
+}
+
+int prepare_sort() {
+    int rc;
+    if ((rc = allow_shared((const void *)k_sort_small<4>, small_smem<4>())) ||
+        (rc = allow_shared((const void *)k_sort_small<16>, small_smem<16>())) ||
+        (rc = allow_shared((const void *)k_sort_small_targets<4>, small_smem<4>())) ||
+        (rc = allow_shared((const void *)k_sort_small_targets<16>, small_smem<16>())))
+        return rc;
+    return TC_OK;
 }
 
 void kernels_sort(KernelList &v) {

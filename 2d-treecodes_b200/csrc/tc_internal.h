@@ -356,8 +356,6 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
                int nblocks, double *xout, double *yout, OverlapFn between,
                double *host_x = nullptr, double *host_y = nullptr);
 
-// Shared-memory preferences of kernels that run beside others (once per device).
-int prefer_force_carveout();
 
 // ---- potential.cu
 int potential(Context &c, double theta, const double *xt, const double *yt, int m, double *out,
@@ -372,6 +370,19 @@ void kernels_upward(KernelList &v);
 void kernels_force(KernelList &v);
 void kernels_potential(KernelList &v);
 void kernels_direct(KernelList &v);
+
+// Attributes of a file's kernels, which belong to the current device: called once per device by
+// preload_kernels.
+int prepare_sort();
+int prepare_upward();
+int prepare_force();
+int prepare_potential();
+
+// Lets a kernel use `bytes` of dynamic shared memory (above 48 KB a launch needs it).
+inline int allow_shared(const void *kernel, size_t bytes) {
+    TC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return TC_OK;
+}
 
 // ---- capi.cu
 int check_device_errors(Context &c, const char *where);

@@ -247,6 +247,11 @@ struct alignas(16) LeafShared {
     T v[32][2 * P + 1];
 };
 
+template <int P, bool MIXED>
+constexpr size_t leaf_bytes() {
+    return UP_WARPS * sizeof(LeafShared<P, typename std::conditional<MIXED, float, double>::type>);
+}
+
 // The 2 P columns of 32 rows are cut in PARTS each, so that all lanes take the same number of cut
 // columns (P = 24: 96, three of 16 rows each; P = 12: 96, three of 8 rows).  The mixed form is
 // bound by the conversions of these sums: with one lane per coefficient, both its columns and
@@ -908,16 +913,9 @@ static int run_expansions(Context &c) {
     const int sms = sm_count_up();
 
     const bool mixed = c.precision == 1;
-    const size_t smem64 = UP_WARPS * sizeof(LeafShared<P, double>);
-    const size_t smem32 = UP_WARPS * sizeof(LeafShared<P, float>);
-    const size_t smem = mixed ? smem32 : smem64;
-    static const cudaError_t attr_rc[2] = {
-        cudaFuncSetAttribute(k_leaf_p2e<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem64),
-        cudaFuncSetAttribute(k_leaf_p2e<P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem32)};
-    TC_CUDA_TRY(attr_rc[0]);
-    TC_CUDA_TRY(attr_rc[1]);
-    const int occ = mixed ? blocks_per_sm<k_leaf_p2e<P, true>>(UP_WARPS * 32, smem32)
-                          : blocks_per_sm<k_leaf_p2e<P, false>>(UP_WARPS * 32, smem64);
+    const size_t smem = mixed ? leaf_bytes<P, true>() : leaf_bytes<P, false>();
+    const int occ = mixed ? blocks_per_sm<k_leaf_p2e<P, true>>(UP_WARPS * 32, smem)
+                          : blocks_per_sm<k_leaf_p2e<P, false>>(UP_WARPS * 32, smem);
     const int grid = (int)std::min<long long>((nn + UP_WARPS - 1) / UP_WARPS, (long long)sms * occ);
     auto p2e = mixed ? k_leaf_p2e<P, true> : k_leaf_p2e<P, false>;
     TC_CUDA_TRY(launch_pdl(ovl, p2e, grid, UP_WARPS * 32, smem, c.stream, nn, c.nsrc, c.leafcap,
@@ -990,6 +988,17 @@ int upward_pass(Context &c, int order) {
     int rc;
     if ((rc = upward_prepare(c, order)) || (rc = upward_moments(c)) || (rc = upward_expansions(c)))
         return rc;
+    return TC_OK;
+}
+
+int prepare_upward() {
+    int rc;
+#define TC_LEAF_SHARED(P)                                                                         \
+    if ((rc = allow_shared((const void *)k_leaf_p2e<P, true>, leaf_bytes<P, true>())) ||          \
+        (rc = allow_shared((const void *)k_leaf_p2e<P, false>, leaf_bytes<P, false>())))          \
+        return rc;
+    TC_FOR_EACH_ORDER(TC_LEAF_SHARED)
+#undef TC_LEAF_SHARED
     return TC_OK;
 }
 
