@@ -418,6 +418,7 @@ static int potential_device(Context &c, double theta, const double *xs, const do
     if ((rc = check_device_errors(c, "treecode_potential"))) return rc;
     c.counts.e2p_pairs = (long long)stat_counter(c, STAT_E2P_PAIRS);
     c.counts.p2p_pairs = (long long)stat_counter(c, STAT_P2P_PAIRS);
+    c.counts.n_e2l = c.counts.e2l_pairs = (long long)stat_counter(c, STAT_SET_CELLS);
     finish_timing(c);
     return TC_OK;
 }

@@ -119,7 +119,7 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_supers(
     int *stack = stack_all[warp];
     const unsigned lt = lanemask_lt();
     const double theta2 = theta * theta, rho2 = rho * rho;
-    unsigned long long pairs = 0;
+    unsigned long long cells = 0;
     for (int g = blockIdx.x * PT_WARPS + warp; g < nsets; g += gridDim.x * PT_WARPS) {
         double bxlo = 1e300, bxhi = -1e300, bylo = 1e300, byhi = -1e300;
         const int t0 = g * PS_GROUPS * 32, cnt = min(PS_GROUPS * 32, m - t0);
@@ -212,10 +212,10 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_supers(
             // has a finite offset)
             geo[g] = expand ? make_double4(cx, cy, half, 0.0) : make_double4(0.0, 0.0, 1.0, 0.0);
         }
-        pairs += (unsigned long long)nc * cnt;
+        cells += nc;
         __syncwarp();
     }
-    if (lane == 0 && pairs) atomicAdd(&stats[STAT_E2P_PAIRS], pairs);
+    if (lane == 0 && cells) atomicAdd(&stats[STAT_SET_CELLS], cells);
 }
 
 // The local expansion of every set from its common far list, about the set's centre c with scale
@@ -1349,9 +1349,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
     scratch_learn(c, 2, nwarps, ngroups, c.h_pinned + 36);   // for the next solve
     c.counts.n_e2p = n_e2p;
     c.counts.n_p2p = total - n_e2p;
-    c.counts.n_e2l = 0;
-    c.counts.e2l_pairs = 0;
-    c.counts.l2p_targets = 0;
+    c.counts.l2p_targets = with_sets ? m : 0;   // (n_e2l and the pairs: read back with the result)
     int2 *lists;
     TaskTable tt = {nullptr, ngroups <= PT_LPT_GROUPS ? ntasks : 0, c.ctrl.task_fill,
                     sstart + 2 * (size_t)ngroups, seg};

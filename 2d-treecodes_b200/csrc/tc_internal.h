@@ -58,13 +58,14 @@ struct Counts {
     long long n_e2l, n_e2p, n_p2p;        // interaction-list entries
     long long p2p_pairs;                  // source-target pairs evaluated directly
     long long e2p_pairs;                  // (target, cell) pairs of far-field evaluation
-    long long e2l_pairs;                  // (brick, cell) pairs of local-expansion builds
+    long long e2l_pairs;                  // (brick or target set, cell) pairs of local-expansion builds
     long long l2p_targets;                // targets evaluated from a local expansion
     long long launches;                   // kernels launched by the last solve
 };
 
 // Device-side work counters (unsigned long long each), Ctrl::stats.
-enum { STAT_P2P_SOURCES = 0, STAT_E2P_PAIRS = 1, STAT_P2P_PAIRS = 2, STAT_SLOTS = 8 };
+// STAT_SET_CELLS: common far-list entries of a potential's target sets.
+enum { STAT_P2P_SOURCES = 0, STAT_E2P_PAIRS = 1, STAT_P2P_PAIRS = 2, STAT_SET_CELLS = 3, STAT_SLOTS = 8 };
 
 // Expansion orders a context can be set to (tc_set_orders).  The reference fixes its orders at
 // build time (Makefile:13-14 of the reference: 12 for the potential, 24 for the force); here

@@ -210,6 +210,13 @@ def algorithmic_flops(stats, kind="force"):
             "k_force_near": 11.0 * stats["p2p_pairs"]}
 
 
+def common_far_flops(stats, p=12):
+    """Flops of a potential solve's common far fields (FP64, many targets): 32 coefficients of a
+    target set from each of its cells, 4p + 8 each (with their share of the powers of 1 / z0), and
+    a 32-term polynomial per target, 8 a term."""
+    return 32.0 * (4 * p + 8) * stats["e2l_pairs"] + 8.0 * 32 * stats["l2p_targets"]
+
+
 def read_profile_traffic(kernel, mixed, workload):
     """DRAM bytes per launch of `kernel` (the form that was timed) from the committed ncu
     summary of the same workload (profiles/<kernel>[.mixed].<workload>.txt), or None."""
@@ -502,6 +509,8 @@ def run_b200(args, ws, rank, local):
     # ---- dominant kernel: the evaluation launches, timed by events on the library's stream
     # (force: the far-field and near-field kernels separately; the longer one is the headline)
     flops = algorithmic_flops(st, kind)
+    if kind == "potential":
+        flops["k_potential_eval"] += common_far_flops(st)
     peak = T.measure_fma_peak(not mixed)
     # each kernel timed alone on the GPU (in a solve the near field shares the SMs with the
     # upward pass and the far field)
