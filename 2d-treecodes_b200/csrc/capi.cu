@@ -732,6 +732,16 @@ TC_API int tc_set_blocksize(tc_context *ctx, int blocksize) {
     return TC_OK;
 }
 
+TC_API int tc_set_whole_blocks(tc_context *ctx, int nblocks) {
+    clear_error();
+    if (!ctx || nblocks < 0) {
+        set_error(TC_ERR_INVALID, "invalid number of blocks %d", nblocks);
+        return TC_ERR_INVALID;
+    }
+    ctx->c.whole_blocks = nblocks;
+    return TC_OK;
+}
+
 TC_API int tc_supported_orders(int *orders, int capacity) {
     static const int list[] = {
 #define TC_ORDER_ITEM(P) P,

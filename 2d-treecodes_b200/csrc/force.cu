@@ -1183,7 +1183,11 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
     // them instead, and the regions are sized up for the next solve.  The runs live in the
     // sort's record buffer when they fit in it, else in a block held only for the build.
     const int nwarps = trgrid * TR_WARPS;
-    const int seg = near_segment(nbricks);
+    // what decides the grouping of a brick's sums goes by the whole solve (tc_set_whole_blocks)
+    const int plan_bricks = (int)std::max<long long>(
+        nbricks, std::min<long long>((long long)c.whole_blocks << (2 * L.lbps), 1 << 30));
+    const int seg = near_segment(plan_bricks);
+    const bool shared_bricks = share_bricks(plan_bricks);
     ScratchLayout sl;
     ListScratch ls;   // released (when transient) after the copy, in stream order
     int *sstart, *meta = c.ctrl.meta;
@@ -1231,7 +1235,7 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
     // many bricks: the near field's longest tasks first too (solves of 1M sources FP64 1337 ->
     // 1316 us, mixed 1041 -> 1038; few bricks have short, cut tasks and gain nothing); a second
     // walk writes no task table, so it takes that way as well
-    const bool by_length = !share_bricks(nbricks) || overflow;
+    const bool by_length = !shared_bricks || overflow;
     {
         AuxScope on_aux(c);
         if ((rc = ensure(c, S_E2L, (size_t)tot[2] + 1, &lists)) ||
@@ -1333,7 +1337,6 @@ int force_mrag(Context &c, double theta, const double *x0s, const double *y0s, c
                             : nt_all >= ((size_t)1 << 21)     ? FORCE_CHUNKS
                             : nt_all >= ((size_t)1 << 19)     ? 2
                                                               : 1;
-        const bool shared_bricks = share_bricks(nbricks);
         // few bricks: their local expansions, unless no brick has an E2L cell
         void *local = nullptr;
         if (shared_bricks && tot[0] > 0) {

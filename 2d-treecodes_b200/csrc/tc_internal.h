@@ -175,6 +175,7 @@ struct Context {
     Ctrl ctrl = {};
     unsigned *h_pinned = nullptr;         // small pinned staging area for readbacks
     int precision = 0;                    // 0 = plain FP64, 1 = mixed
+    int whole_blocks = 0;                 // blocks of the solve that this one is a part of, or 0
     int order_potential = ORDER_POTENTIAL;  // expansion orders of the next solves
     int order_force = ORDER_FORCE;
     int blocksize = BLOCKSIZE;            // MRAG block side of the force entry points

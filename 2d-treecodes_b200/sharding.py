@@ -66,10 +66,17 @@ def target_shard(xt, yt, rank, world):
 
 def solve_shard(ctx, theta, xs, ys, vs, x0s, y0s, hs, rank, world, blocksize=T.BLOCKSIZE):
     """This rank's part of a force_mrag solve on `ctx`: (block indices, xout, yout), the outputs
-    in the reference's layout over the shard's blocks."""
+    in the reference's layout over the shard's blocks.  The shards' outputs equal the unsplit
+    solve's bit for bit (Context.set_whole_blocks)."""
     idx = block_shard(x0s, y0s, rank, world)
+    whole = len(x0s)
     x0s, y0s, hs = (np.asarray(a, dtype=np.float64)[idx] for a in (x0s, y0s, hs))
-    xo, yo = ctx.force_mrag_host(theta, xs, ys, vs, x0s, y0s, hs)
+    set_whole = getattr(ctx, "set_whole_blocks", lambda nblocks: None)   # (a stand-in has no forms)
+    set_whole(whole)
+    try:
+        xo, yo = ctx.force_mrag_host(theta, xs, ys, vs, x0s, y0s, hs)
+    finally:
+        set_whole(0)
     return idx, xo, yo
 
 
@@ -93,7 +100,9 @@ def assemble(parts, nblocks, blocksize=T.BLOCKSIZE):
 
 
 def solve_potential_shard(ctx, theta, xs, ys, vs, xt, yt, rank, world):
-    """This rank's part of a potential solve on `ctx`: (target indices, potentials there)."""
+    """This rank's part of a potential solve on `ctx`: (target indices, potentials there).  A target's
+    sums are grouped by its neighbours among the targets, so that shards differ from the unsplit
+    solve by roundings."""
     idx = target_shard(xt, yt, rank, world)
     xt, yt = (np.asarray(a, dtype=np.float64)[idx] for a in (xt, yt))
     return idx, ctx.potential_host(theta, xs, ys, vs, xt, yt)

@@ -48,6 +48,7 @@ SIGNATURES = {
     "tc_set_orders": (_i, [_vp, _i, _i]),
     "tc_supported_orders": (_i, [ctypes.POINTER(ctypes.c_int), _i]),
     "tc_set_blocksize": (_i, [_vp, _i]),
+    "tc_set_whole_blocks": (_i, [_vp, _i]),
     "tc_log_probe_device": (_i, [_vp, _vp, _i, _vp]),
     "tc_set_timing": (_i, [_vp, _i]),
     "tc_get_stats": (_i, [_vp, _vp]),
@@ -285,6 +286,11 @@ class Context:
         build-time mrag-blocksize): outputs of nblocks * blocksize**2 values."""
         _check(self.lib.tc_set_blocksize(self.h, int(blocksize)))
         self.blocksize = int(blocksize)
+
+    def set_whole_blocks(self, nblocks=0):
+        """The force solves that follow are parts of one of `nblocks` blocks (0: each is a whole
+        one): their outputs equal the whole solve's bit for bit."""
+        _check(self.lib.tc_set_whole_blocks(self.h, int(nblocks)))
 
     def set_timing(self, on=True):
         """True / 1: phase times in stats(); 2: also the force's near- and far-field kernels

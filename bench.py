@@ -363,11 +363,13 @@ def run_b200(args, ws, rank, local):
     kind = w["kind"]
     # targets of the whole job: every rank's own problem (weak) or the one split problem (strong)
     job_m = n_targets(w) * (1 if strong else ws)
+    whole_blocks = 0
     if strong and ws > 1:
         import sharding
         w = dict(w)
         if kind == "force":
             idx = sharding.block_shard(w["x0s"], w["y0s"], rank, ws)
+            whole_blocks = len(w["x0s"])
             for k in ("x0s", "y0s", "hs"):
                 w[k] = np.ascontiguousarray(w[k][idx])
         else:
@@ -376,6 +378,7 @@ def run_b200(args, ws, rank, local):
                 w[k] = np.ascontiguousarray(w[k][idx])
     mixed = args.precision == "mixed"
     ctx = T.Context(device=local, precision=1 if mixed else 0)
+    ctx.set_whole_blocks(whole_blocks)   # a shard's sums grouped as the unsplit solve's
     stream = torch.cuda.ExternalStream(ctx.stream, device=dev)
     d = {k: torch.as_tensor(w[k]).to(dev) for k in w if isinstance(w[k], np.ndarray)}
     m = n_targets(w)

@@ -144,6 +144,11 @@ TC_API int tc_supported_orders(int *orders, int capacity);
  * default and for treecode_force_mrag).  Outputs hold nblocks * blocksize^2 values, target
  * (ix, iy) of block ib at ix + blocksize * (iy + blocksize * ib). */
 TC_API int tc_set_blocksize(tc_context *ctx, int blocksize);
+/* The force solves that follow are parts of one of `nblocks` blocks (0, the default: each is a whole
+ * solve).  How the sums of a block are grouped depends on the number of blocks, few blocks being
+ * shared out among more warps; with this setting a part groups them as the whole solve does, so
+ * that the parts' outputs equal the whole solve's bit for bit. */
+TC_API int tc_set_whole_blocks(tc_context *ctx, int nblocks);
 /* 1: record phase times (tc_get_stats); 2: also run the force evaluation's near- and far-field
  * kernels one after the other, after the upward pass, each alone on the GPU, so that their
  * times measure each kernel by itself (a measurement mode: the solve is slower, results are
