@@ -314,22 +314,19 @@ __global__ __launch_bounds__(PLOC_WARPS * 32) void k_potential_locals(
 // warp's entries into its own scratch region (ScratchLayout), recording where each group's run
 // starts, so that a copy into CSR order replaces a second walk.  A region that fills up sets
 // meta[0] (the host then falls back to MODE 1); meta[1 + k] receives the longest run of kind
-// k any warp wrote, and the work counters are added.  meta[META_WIDE] is set where a group's targets
-// may be NEAR_REACH or more away from a source (every source is in `frame`).
-constexpr int META_WIDE = 3;
+// k any warp wrote, and the work counters are added.  (meta[META_WIDE] is the target sort's.)
 template <int MODE>
 __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
     int ngroups, int m, const double *__restrict__ xt, const double *__restrict__ yt,
     const int *__restrict__ tperm, double theta, const TNode *__restrict__ tnode, int nnodes,
     int *__restrict__ counts, const int *__restrict__ offs, int2 *__restrict__ lists,
     int2 *__restrict__ scratch, ScratchLayout sl, int *__restrict__ sstart, int *meta,
-    unsigned *err, unsigned long long *stats, int seg, SuperSets sets,
-    const Frame *__restrict__ frame) {
+    unsigned *err, unsigned long long *stats, int seg, SuperSets sets) {
     pdl_begin();
     constexpr bool FILL = MODE == 1;
     const int wglob = blockIdx.x * PT_WARPS + (threadIdx.x >> 5);
     int cur[2] = {0, 0};   // MODE 2: entries this warp has written, per kind
-    bool full = false, wide = false;
+    bool full = false;
     __shared__ int2 stack_all[PT_WARPS][PL_STACK];
     const int lane = lane_id(), warp = threadIdx.x >> 5;
     int2 *stack = stack_all[warp];
@@ -355,12 +352,6 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
             bxhi = fmax(bxhi, __shfl_xor_sync(FULL_MASK, bxhi, o));
             bylo = fmin(bylo, __shfl_xor_sync(FULL_MASK, bylo, o));
             byhi = fmax(byhi, __shfl_xor_sync(FULL_MASK, byhi, o));
-        }
-        if (MODE == 2) {
-            const double fx = frame->xmin, fy = frame->ymin, fe = frame->ext;
-            const double reach = fmax(fmax(bxhi - fx, fx + fe - bxlo),
-                                      fmax(byhi - fy, fy + fe - bylo));
-            wide = wide || !(reach < NEAR_REACH);   // (no finite target: also wide)
         }
         int o0 = 0, o1 = 0, l0 = 0, l1 = 0;
         if (FILL) {
@@ -522,7 +513,6 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
         if (lane == 0) {
             atomicMax(&meta[1], cur[0]);
             atomicMax(&meta[2], cur[1]);
-            if (wide) atomicOr(&meta[META_WIDE], 1);
         }
     }
     if (MODE == 2 && stats && lane == 0) {
@@ -1328,8 +1318,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
         TC_CUDA_TRY(launch_pdl(c.launch_overlap, k_potential_lists<2>, grid, PT_WARPS * 32, 0,
                                c.stream, ngroups, m, xt, yt, (const int *)vo, theta, tnode, c.nnodes,
                                counts, (const int *)nullptr, (int2 *)nullptr,
-                               static_cast<int2 *>(ls.p), sl, sstart, meta, err, stats, seg, sets,
-                               (const Frame *)slot_ptr<Frame>(c, S_FRAME)));
+                               static_cast<int2 *>(ls.p), sl, sstart, meta, err, stats, seg, sets));
         TC_KERNEL_CHECK();
         // the lists' totals and meta, written to h_pinned by the scan
         if ((rc = exclusive_scan(c, counts, offs, 3 * ngroups, ngroups, c.h_pinned + 32, meta)))
@@ -1368,7 +1357,7 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
             // (the second walk does not add to the work counters)
             k_potential_lists<1><<<grid, PT_WARPS * 32, 0, c.stream>>>(
                 ngroups, m, xt, yt, vo, theta, tnode, c.nnodes, nullptr, offs, lists, nullptr,
-                sl, nullptr, nullptr, err, stats, seg, sets, nullptr);
+                sl, nullptr, nullptr, err, stats, seg, sets);
             TC_KERNEL_CHECK();
             k_task_map_groups<<<(int)std::min<long long>((ngroups + 255) / 256,
                                                          (long long)sm_count_p() * 8),

@@ -160,12 +160,21 @@ __device__ __forceinline__ int target_key(double x, double y, const Frame &f) {
     return spread_bits((int)qx) | (spread_bits((int)qy) << 1);
 }
 
+// A target may be NEAR_REACH or more away from a source in x or in y (every source is in the frame).
+__device__ __forceinline__ bool target_wide(double x, double y, const Frame &f) {
+    return x <= f.xmin + f.ext - NEAR_REACH || x >= f.xmin + NEAR_REACH ||
+           y <= f.ymin + f.ext - NEAR_REACH || y >= f.ymin + NEAR_REACH;
+}
+
 __global__ void k_target_keys(const double *__restrict__ x, const double *__restrict__ y, int n,
-                              const Frame *__restrict__ frame, int *__restrict__ keys) {
+                              const Frame *__restrict__ frame, int *__restrict__ keys, int *wide) {
     pdl_begin();
     const Frame f = *frame;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        keys[i] = target_key(x[i], y[i], f);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double xi = x[i], yi = y[i];
+        keys[i] = target_key(xi, yi, f);
+        if (target_wide(xi, yi, f)) atomicOr(wide, 1);
+    }
 }
 
 // ---------------------------------------------------------------------------- radix sort
@@ -891,7 +900,7 @@ __global__ __launch_bounds__(SMALL_THREADS) void k_sort_small(
     const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ v, int n,
     Frame *frame, int *__restrict__ keys, int *__restrict__ perm, double *__restrict__ xs,
     double *__restrict__ ys, double *__restrict__ vs, const double *__restrict__ xt,
-    const double *__restrict__ yt, int nt, int *__restrict__ tperm) {
+    const double *__restrict__ yt, int nt, int *__restrict__ tperm, int *wide) {
     extern __shared__ __align__(16) unsigned long long small_dyn[];
     unsigned long long *s_items = small_dyn;
     int *s_hist = reinterpret_cast<int *>(s_items + SMALL_THREADS * ITEMS);
@@ -929,7 +938,11 @@ __global__ __launch_bounds__(SMALL_THREADS) void k_sort_small(
         // past the end: after every key, and after equal ones (they come last in input order)
         unsigned key = 0xffffffffu;
         if (targets) {
-            if (i < nt) key = (unsigned)target_key(xt[i], yt[i], f);
+            if (i < nt) {
+                const double xi = xt[i], yi = yt[i];
+                key = (unsigned)target_key(xi, yi, f);
+                if (target_wide(xi, yi, f)) atomicOr(wide, 1);
+            }
         } else if (i < n) {
             key = (unsigned)morton_key(x[i], y[i], f);
         }
@@ -955,7 +968,7 @@ __global__ __launch_bounds__(SMALL_THREADS) void k_sort_small(
 template <int ITEMS>
 __global__ __launch_bounds__(SMALL_THREADS) void k_sort_small_targets(
     const double *__restrict__ x, const double *__restrict__ y, int n,
-    const Frame *__restrict__ frame, int *__restrict__ perm) {
+    const Frame *__restrict__ frame, int *__restrict__ perm, int *wide) {
     extern __shared__ __align__(16) unsigned long long small_dyn[];
     unsigned long long *s_items = small_dyn;
     int *s_hist = reinterpret_cast<int *>(s_items + SMALL_THREADS * ITEMS);
@@ -967,7 +980,11 @@ __global__ __launch_bounds__(SMALL_THREADS) void k_sort_small_targets(
     for (int k = 0; k < ITEMS; ++k) {
         const int i = warp * 32 * ITEMS + 32 * k + lane;
         unsigned key = 0xffffffffu;
-        if (i < n) key = (unsigned)target_key(x[i], y[i], f);
+        if (i < n) {
+            const double xi = x[i], yi = y[i];
+            key = (unsigned)target_key(xi, yi, f);
+            if (target_wide(xi, yi, f)) atomicOr(wide, 1);
+        }
         item[k] = ((unsigned long long)key << 32) | (unsigned)i;
     }
     block_sort_items<ITEMS>(item, s_items, s_hist);
@@ -979,7 +996,8 @@ static int sort_small(Context &c, const double *x, const double *y, const double
                       Frame *frame, int *keys, int *perm, double *xs, double *ys, double *vs,
                       const double *xt, const double *yt, int nt, int *tperm) {
     k_sort_small<ITEMS><<<tperm ? 2 : 1, SMALL_THREADS, small_smem<ITEMS>(), c.stream>>>(
-        x, y, v, n, frame, keys, perm, xs, ys, vs, xt, yt, nt, tperm);
+        x, y, v, n, frame, keys, perm, xs, ys, vs, xt, yt, nt, tperm,
+        c.ctrl.meta + META_WIDE);
     TC_KERNEL_CHECK();
     return TC_OK;
 }
@@ -988,7 +1006,8 @@ template <int ITEMS>
 static int sort_small_targets(Context &c, const double *x, const double *y, int n, int *perm) {
     TC_CUDA_TRY(launch_pdl(c.launch_overlap && c.single, k_sort_small_targets<ITEMS>, 1,
                            SMALL_THREADS, small_smem<ITEMS>(), c.stream, x, y, n,
-                           (const Frame *)slot_ptr<Frame>(c, S_FRAME), perm));
+                           (const Frame *)slot_ptr<Frame>(c, S_FRAME), perm,
+                           c.ctrl.meta + META_WIDE));
     TC_KERNEL_CHECK();
     return TC_OK;
 }
@@ -1399,7 +1418,7 @@ int sort_targets(Context &c, const double *xt, const double *yt, int m, int **pe
         (rc = ensure(c, S_TPERM2, m, &tperm2)))
         return rc;
     k_target_keys<<<grid_for(m, 256), 256, 0, c.stream>>>(xt, yt, m, slot_ptr<Frame>(c, S_FRAME),
-                                                          tkeys);
+                                                          tkeys, c.ctrl.meta + META_WIDE);
     TC_KERNEL_CHECK();
     return radix_sort_pairs(c, tkeys, nullptr, m, 2 * LMAX, tkeys2, tperm2, tkeys, tperm, &ko, perm);
 }

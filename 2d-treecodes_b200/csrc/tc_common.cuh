@@ -39,6 +39,10 @@ struct Frame {
     double scale;             // (1 / ext) * 2^LMAX, the factor the compiled reference uses
 };
 
+// Targets and sources that differ by less than this in x and in y have squared distances below
+// 2 (2^509)^2 = 2^1019, which the FP64 potential's logarithm and reciprocal are made for (log_near).
+constexpr double NEAR_REACH = 0x1p509;
+
 // A brick's near field is cut into segments of P2P_SEG sources, so that the few bricks on a dense
 // region do not serialise the kernel.  The segments also fix the grid of source tiles (a
 // segment's tiles start at its own start, at a leaf's start, or 32 sources after another), and
@@ -94,10 +98,10 @@ __device__ __forceinline__ double rcp_nr(double d) {
     return fma(y, t, y);
 }
 
-// 1 / d for any d: rcp_nr where the approximation and its correction stay in the number range
-// (rcp_nr turns an infinite square into NaN and flushes 1 / d from d = 2^1022 on).
+// 1 / d for any d: rcp_nr from 2^-1000 to 2^1000 (its approximation flushes 1 / d to 0 from 2^1022
+// on, and its correction makes a NaN of infinity), decided on the high word.
 __device__ __forceinline__ double rcp_any(double d) {
-    return d > 1e-300 && d < 1e300 ? rcp_nr(d) : 1.0 / d;
+    return (unsigned)__double2hiint(d) - 0x01700000u < 0x7e700000u - 0x01700000u ? rcp_nr(d) : 1.0 / d;
 }
 
 __device__ __forceinline__ double shfl_xor_d(double v, int m) {

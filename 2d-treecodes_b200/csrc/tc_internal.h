@@ -101,13 +101,17 @@ constexpr int FORCE_CHUNKS = 4;
 // Everything a solve needs zeroed, in one buffer that one memset at its start clears: on a small
 // solve a memset costs as much as a short kernel, and twelve of them took about a tenth of it.
 // The scanned histograms and the test sink lie behind the cleared part.
+// meta[META_WIDE], set by a potential's target sort: a target may be NEAR_REACH or more away from a
+// source.
+constexpr int META_WIDE = 3;
+
 struct Ctrl {
     unsigned *err;                // device error word
     unsigned long long *stats;    // work counters (STAT_*), read back with err in one copy
     unsigned *bbox_done;
     int *tile_ctr, *bucket_fill;  // source sort: tiles taken per pass, record slots claimed
     int *nlist, *tl_ctr;          // tree: split-list length, tiles taken
-    int *meta;                    // list build: overflow flag, longest runs
+    int *meta;                    // list build: overflow flag, longest runs; potential: META_WIDE
     int *near_ctr, *far_ctr, *e2l_ctr;   // evaluation tasks / far-field bricks taken
     // tasks per bin (TaskBins): far-field bricks (per run) or potential tasks; near-field tasks
     int *task_fill, *near_fill;

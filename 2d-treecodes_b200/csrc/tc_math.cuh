@@ -78,10 +78,7 @@ __device__ __forceinline__ void load_log_table(double *s_neg_log_c) {
 // would not.  Within 2 ulp of the exact logarithm (tests/test_near_log_table.py,
 // tests/test_potential_reach.py).
 constexpr int NLOG_COPIES = 8;
-constexpr int NLOG_TOP = 1020;
-// Squared distances stay below 2^NLOG_TOP where targets and sources differ by less than this in x
-// and in y: 2 (2^509)^2 = 2^1019.
-constexpr double NEAR_REACH = 0x1p509;
+constexpr int NLOG_TOP = 1020;   // (2 NEAR_REACH^2 is below it)
 
 // `tab`: the table's 32-bit shared-memory address; `copy`: the lane's copy, 16 (lane % 8).
 __device__ __forceinline__ unsigned shared_address(const void *p) {
