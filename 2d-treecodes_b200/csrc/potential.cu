@@ -90,7 +90,7 @@ struct SuperSets {
 // bounds that ratio so that what PS_TERMS terms leave out stays below 1e-17 of a cell's weight,
 // under the rounding of the sum: with |a_{k-1} z^-k| <= theta^k / k,
 //   rho^q / q + sum_k theta^k / k C(q + k - 1, k - 1) rho^q / (1 - rho (q + k) / (q + 1)).
-// (theta 0.5, order 12: rho 0.2.)  0: no common entries.
+// (theta 0.5, order 12: rho 0.19.)  0: no common entries.  Some hundred pow calls.
 static double super_rho(double theta, int order) {
     if (!(theta > 0 && theta <= 1)) return 0.0;
     constexpr int q = PS_TERMS;
@@ -1280,8 +1280,8 @@ int potential(Context &c, double theta, const double *xt, const double *yt, int 
     // of cells takes longer than it saves)
     SuperSets sets = {};
     const int nsets = (ngroups + PS_GROUPS - 1) / PS_GROUPS;
-    const double rho = super_rho(theta, c.order);
-    const bool with_sets = c.precision == 0 && ngroups >= PS_MIN_GROUPS && rho > 0;
+    const double rho = c.precision == 0 && ngroups >= PS_MIN_GROUPS ? super_rho(theta, c.order) : 0.0;
+    const bool with_sets = rho > 0;
     cplx *set_local = nullptr;
     ScratchLayout sl;
     ListScratch ls;   // released (when transient) after the copy, in stream order
