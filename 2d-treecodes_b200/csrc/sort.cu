@@ -1279,6 +1279,9 @@ int sort_sources(Context &c, const double *x, const double *y, const double *v, 
     // (the stalled look-back of the test setting is the general sort's)
     if (n <= SMALL_SORT && c.test_stall != TC_STALL_SORT) {
         const double *v_now = values_ready ? nullptr : v;
+        // (not this sort's, but the list builds' scratch: list_scratch)
+        double2 *rec;
+        if ((rc = ensure(c, S_REC, 2 * (size_t)n, &rec))) return rc;
         // the targets beside them, where they are there already and as few (solves on one stream):
         // 4096 sources and targets FP64 162 -> 142 us, mixed 221 -> 201 us
         int *tperm = nullptr;
