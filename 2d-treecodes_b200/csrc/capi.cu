@@ -393,6 +393,14 @@ static int expansions_then_mark(Context &c) {
     return rc;
 }
 
+// Error return after work was queued: it may still read the caller's memory on either stream, so
+// both are waited for before returning.
+static int drain_and_fail(Context &c, int rc) {
+    wait_stream(c, c.aux);
+    wait_stream(c, c.stream);
+    return rc;
+}
+
 static int potential_device(Context &c, double theta, const double *xs, const double *ys,
                             const double *vs, int n, const double *xt, const double *yt, int m,
                             double *out, cudaEvent_t values_ready = nullptr) {
@@ -409,11 +417,9 @@ static int potential_device(Context &c, double theta, const double *xs, const do
     int rc;
     phase_mark(c, 0);
     c.single = single_stream(n, (m + 31) / 32) && !values_ready;
-    if ((rc = build_tree_moments(c, 0, xs, ys, vs, n, m, values_ready, xt, yt))) {
-        if (c.targets_sorted) wait_stream(c, c.aux);   // it may still read the targets
-        return rc;
-    }
-    if ((rc = potential(c, theta, xt, yt, m, out, expansions_then_mark))) return rc;
+    if ((rc = build_tree_moments(c, 0, xs, ys, vs, n, m, values_ready, xt, yt)) ||
+        (rc = potential(c, theta, xt, yt, m, out, expansions_then_mark)))
+        return drain_and_fail(c, rc);
     phase_mark(c, 5);
     if ((rc = check_device_errors(c, "treecode_potential"))) return rc;
     c.counts.e2p_pairs = (long long)stat_counter(c, STAT_E2P_PAIRS);
@@ -448,10 +454,9 @@ static int force_device(Context &c, double theta, const double *xs, const double
     int rc;
     phase_mark(c, 0);
     c.single = false;
-    if ((rc = build_tree_moments(c, 1, xs, ys, vs, n, 0, values_ready))) return rc;
-    if ((rc = force_mrag(c, theta, x0s, y0s, hs, nb, xo, yo, expansions_then_mark, host_x,
-                         host_y)))
-        return rc;
+    if ((rc = build_tree_moments(c, 1, xs, ys, vs, n, 0, values_ready)) ||
+        (rc = force_mrag(c, theta, x0s, y0s, hs, nb, xo, yo, expansions_then_mark, host_x, host_y)))
+        return drain_and_fail(c, rc);
     phase_mark(c, 5);
     if ((rc = check_device_errors(c, "treecode_force_mrag"))) return rc;
     c.counts.p2p_pairs = (long long)stat_counter(c, STAT_P2P_SOURCES) * TILE * TILE;
@@ -504,14 +509,6 @@ static int stage_split(Context &c, std::initializer_list<StagedArray> first,
         values = false;
     }
     return TC_OK;
-}
-
-// Error return of a host entry point after staging began: copies already queued on either
-// stream may still read the caller's memory, so both streams are waited for before returning.
-static int drain_and_fail(Context &c, int rc) {
-    wait_stream(c, c.aux);
-    wait_stream(c, c.stream);
-    return rc;
 }
 
 static int potential_host(Context &c, double theta, const double *xs, const double *ys,
