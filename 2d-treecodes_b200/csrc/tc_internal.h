@@ -342,11 +342,14 @@ inline cudaError_t await_event(Context &c, cudaEvent_t e) {
 
 // Potential solves of at most this many sources and target groups run on one stream, their kernels
 // chained (launch_pdl): the events and cross-stream waits of the two-stream order cost the host
-// and the device ~2 us each, and its second stream has little to overlap.  4096 sources and
-// targets: FP64 186 -> 173 us, mixed 230 -> 219.  (The force's near field does overlap the
+// and the device ~2 us each, and its second stream has little to overlap.  Up to 16,384 of each, where
+// one launch sorts both; more targets have a sort of several launches, which the second stream takes
+// beside the tree.  Sources and targets, two streams -> one, FP64 / mixed: 1000 124 -> 116 / 152 ->
+// 135 us, 4096 145 -> 141 / 247 -> 239, 16,384 302 -> 279 / 392 -> 366; 16,384 and 32,768 299 -> 334 /
+// 368 -> 404, 32,768 of each 285 -> 315 / 341 -> 365.  (The force's near field does overlap the
 // upward pass and the far field: on one stream the 4096-source solve took 184 us instead of 168.)
 constexpr int SINGLE_MAX_SOURCES = 16384;
-constexpr int SINGLE_MAX_GROUPS = 1024;
+constexpr int SINGLE_MAX_GROUPS = 512;
 inline bool single_stream(long long nsources, long long groups) {
     return nsources <= SINGLE_MAX_SOURCES && groups <= SINGLE_MAX_GROUPS;
 }

@@ -1,6 +1,6 @@
 """Host solves whose values arrive while the sources are sorted in one block (up to 16,384): the
 gather of the values by itself, with the targets sorted on the second stream behind their own copy.
-More than 32,768 targets, or blocks, take this route; fewer targets run on one stream."""
+More than 16,384 targets, or blocks, take this route; fewer targets run on one stream."""
 import numpy as np
 import pytest
 
