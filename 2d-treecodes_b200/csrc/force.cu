@@ -304,7 +304,9 @@ struct FarShared<P, true> {
 // warp, so that the solve does not wait for one warp's chain of cells.  The far field alone, a
 // warp per brick and this: 1936 bricks, mixed, 160 -> 121 us; 576 bricks, FP64, 56 -> 42 us.
 // With more bricks the separate E2L launch and the idle lanes cost more than they give (65,536
-// bricks, mixed, 578 -> 670 us).
+// bricks, mixed, 578 -> 670 us).  Solves of a 1M-source sheet, FP64 / mixed: 4096 bricks 511 -> 452 /
+// 482 -> 426 us, 7744 538 -> 500 / 524 -> 463, 10,816 540 -> 539 / 519 -> 486, 16,384 584 -> 612 / 540 ->
+// 527; of 256K sources 7744 bricks 352 -> 350, 10,816 380 -> 392 / 349 -> 359.
 static bool share_bricks(int nbricks) { return nbricks <= 8192; }
 
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {

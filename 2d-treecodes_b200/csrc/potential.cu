@@ -523,8 +523,9 @@ __global__ __launch_bounds__(PT_WARPS * 32) void k_potential_lists(
 
 // Few groups (up to PT_LPT_GROUPS): tasks in bins of falling work, the longest first (TaskBins), so
 // that no long one is left for the end: mixed solves of 700,001 targets 1569 -> 1517 us, FP64 ones
-// of 131,072 905 -> 881 us, 1,048,576 (theta 0.3) 3221 -> 3157 us.  Above it the tail is a small
-// share, and neighbouring groups evaluated together share list sources in cache.
+// of 131,072 905 -> 881 us, 1,048,576 (theta 0.3) 3221 -> 3157 us.  The tail is a smaller share of
+// more groups, while the table takes 64 bytes a task: 32,768 groups FP64 3295 -> 3200 us, mixed 1997 ->
+// 1946; 65,536 groups 5681 -> 5630 (1%) and 3490 -> 3491.
 constexpr int PT_LPT_GROUPS = 32768;
 
 // Where the evaluation's tasks go: entry (task, group) t at t, or (stride > 0) in its bin.
@@ -904,10 +905,11 @@ __global__ __launch_bounds__(PE_WARPS * 32) void k_potential_eval_mixed(
     }
 }
 
-// The FP64 form.  Bound by the FP64 pipe (12 operations per P2P pair, 16 lanes of it per scheduler
-// and cycle, so 24 cycles per 32 pairs) with the issue slots and the shared-memory port close
-// behind.  Blocks of 8 warps share one set of table copies (64 KB); three blocks, 24 warps, fit
-// on an SM.
+// The FP64 form: 12 FP64 operations per P2P pair (16 lanes of the pipe per scheduler, so 24 cycles per
+// 32 pairs) and about 20 others.  On 1M clustered sources and targets 65% of the cycles issue and the
+// FP64 pipe is busy for 56%; an FP64 instruction keeps its scheduler for a second cycle (28%), which
+// leaves 7% of them unused.  Blocks of 8 warps share one set of table copies (64 KB); three blocks, 24
+// warps, fit on an SM.
 // Tasks: group g owns tasks [toff[g], toff[g+1]).  seg == PT_SEG: task 0 evaluates the far field
 // and the first segment of the group's near field, task p > 0 the p-th segment.  seg < PT_SEG:
 // the far field is task 0 (where the group has one), and the p-th near-field task takes the tiles
@@ -939,7 +941,8 @@ constexpr size_t eval_smem() {
 // there are no sets).
 // WIDE: for solves with a target NEAR_REACH or more away from a source, whose squares may pass
 // log_near's range or overflow: log_pos, whose logarithm of infinity is 1024 ln 2, and a true
-// division (the arithmetic of the kernel before log_near).
+// division (the arithmetic of the kernel before log_near).  4096 sources and targets with one such
+// target 159 us a solve instead of 140, 64K 383 and 359, 1M 3394 and 3017.
 template <int P, bool SETS, bool WIDE>
 __global__ __launch_bounds__(PD_WARPS * 32, PD_MIN_BLOCKS) void k_potential_eval(
     int ngroups, int m, const double *__restrict__ xt, const double *__restrict__ yt,

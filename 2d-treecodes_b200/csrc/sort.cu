@@ -509,7 +509,8 @@ struct FirstPass {
 // written out in runs of equal digits.  ITEMS is 12 (four CTAs per SM), or 8 where that is few tiles
 // per SM and a pass lasts as long as one tile's phases (sort_tile): potential of 64K sources 359 ->
 // 352 us, force 64K 234 -> 226, 256K 392 -> 374, 1M 1014 -> 1007, potential 700,001 1437 -> 1417;
-// at 16M it is the slower one (sort 1057 -> 1128).
+// at 16M it is the slower one (sort 1057 -> 1128).  Mixed solves of a sheet on 256 blocks: 512K 357 ->
+// 349, 1.5M 531 -> 528, 2M and 4M the same, 8M 1980 -> 2001 us.
 // `stall_tile` (a test setting, -1 otherwise) names a tile that publishes into `sink` instead
 // of its status words, so that the tiles after it wait until `spin_limit` and report
 // DEVERR_SPIN_LIMIT.

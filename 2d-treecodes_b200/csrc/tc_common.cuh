@@ -79,9 +79,15 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
 // Programmatic dependent launch (launch_pdl): a kernel may be scheduled while the kernel before
-// it on its stream is still draining.  A kernel so launched calls this first: it waits until
-// that kernel has completed and its writes are visible (so stream order holds exactly), then
-// lets the kernel after it be scheduled in turn.  Both are no-ops without the launch attribute.
+// it on its stream is still draining.  A kernel so launched calls this before it reads what that
+// kernel writes, and before it writes anything: it waits until that kernel has completed and its
+// writes are visible, then lets the kernel after it be scheduled in turn.  Both are no-ops without
+// the launch attribute.
+// The order of the two is what early reads rest on.  Every kernel of a chain waits before it releases
+// the next, so when a kernel starts, the one before it has seen its own predecessor complete:
+// whatever is older than the preceding kernel may be read ahead of pdl_begin (merge_geom,
+// k_moments_level, k_potential_gather_parts, the log tables), and nothing else.  A kernel that
+// released the next before its wait would break every chain that it stands in.
 __device__ __forceinline__ void pdl_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -251,8 +251,8 @@ int device_sm_count();
 
 // Launches `kernel` on `s` with programmatic stream serialization when `overlap` is set (the
 // context's launch_overlap): its blocks may be scheduled while the previous kernel of `s`
-// drains, and wait in pdl_begin() (the kernel's first statement) until that kernel has
-// completed.  Otherwise an ordinary launch.  Follow with TC_KERNEL_CHECK().
+// drains, and wait in pdl_begin() until that kernel has completed (what may stand before it:
+// there).  Otherwise an ordinary launch.  Follow with TC_KERNEL_CHECK().
 template <class... P, class... A>
 cudaError_t launch_pdl(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
                        cudaStream_t s, A &&...args) {

@@ -9,7 +9,10 @@ namespace tc {
 
 constexpr int BINOM_N = 2 * MAX_ORDER;
 
-// Pascal's triangle in double (exact: every entry used, up to C(47,23) ~ 1.6e13, is below 2^53).
+// Pascal's triangle in double, exact in every entry used: C(l+k-1, k-1) up to C(47,23) ~ 1.6e13 in
+// translations of order 24, C(55,27) ~ 3.8e15 in those of order 28, and in a potential's common far
+// fields C(l+k-1, k-1), l <= 31, k <= 28; those above 2^53 (up to C(58,27) ~ 2.6e16) have enough factors
+// of two (tests/test_binomials.py).
 // The reference bakes the same integers into its kernels through kernels/binomial.py:1-5.
 struct BinomTable {
     double c[BINOM_N][BINOM_N];

@@ -123,7 +123,7 @@ TC_API int tc_set_launch_overlap(tc_context *ctx, int on);
  *                the tree build's list pass, tile 0 publishes nothing, so the tile after it
  *                waits on it until the spin limit, raises the device error flag and moves on;
  *                the solve then stops after that stage with TC_ERR_TIMEOUT.  Needs more
- *                sources than one tile (3072 for the sort, 4096 for the tree).
+ *                sources than one tile (at most 3072 for the sort, 4096 for the tree).
  *   spin_limit:  reads without progress after which a device wait gives up (<= 0: the default,
  *                4,194,304).
  *   stack_limit: traversal stack entries per warp of the force lists (<= 0: all 2048); a walk
